@@ -46,9 +46,9 @@ struct BTree {
     const float* mats32;
     const double* matsb;    // beta-scaled copies (z-step operators)
     const float* matsb32;
-    const double* matsT;    // transposed, zero-padded copies (GEMM-tiled contraction)
-    const float* matsT32;
-    const double* matsbT;
+    const double* matsD;      // fragment images (FP64 matrix-instruction contraction)
+    const double* matsDbeta;  // the term weight of every matrix
+    const float* matsT32;     // transposed, zero-padded copies (GEMM-tiled FP32 contraction)
     const float* matsbT32;
     const float* matsI;  // split-TF32 operator images (tensor-core contraction)
     const float* matsbI;
@@ -412,7 +412,7 @@ __global__ void k_tchunks(const int* __restrict__ offs, const int* __restrict__ 
     ++nch;
     if (!fill && lane == 0) nchunk[w] = nch;
 }
-// Block images for the line-ordered contraction: image row a (a < 2k) holds X[a][b + P c] of the
+// FP32 block images for the line-ordered contraction: image row a (a < 2k) holds X[a][b + P c] of the
 // node block (P = 2k rounded up to 4; zero where b or c >= 2k), so that a CTA stages a block with
 // 16-byte copies.  One CTA per block: read coalesced into shared memory, write the rows coalesced.
 // Real nodes: entry e (a tree of the pass) contributes input nodes [lb[e], lb[e] + cnt[e]) at slots
@@ -422,12 +422,12 @@ struct ImgSrc {
     long long base;
     int lb, cnt;
 };
-template <int K, typename R>
+template <int K>
 __global__ void __launch_bounds__(256) k_ximage(const ImgSrc* __restrict__ srcs, int nsrc, const double* __restrict__ gblk,
-                                                long long nreal, R* __restrict__ img) {
+                                                long long nreal, float* __restrict__ img) {
     constexpr int K2 = 2 * K, KP = (K2 + 3) / 4 * 4, NN = KP * KP, BS = K2 * K2 * K2, KKK = K * K * K;
     extern __shared__ __align__(16) unsigned char smraw[];
-    R* blk = reinterpret_cast<R*>(smraw);
+    float* blk = reinterpret_cast<float*>(smraw);
     const long long slot = blockIdx.x;
     if (slot < nreal) {
         int lo = 0, hi = nsrc - 1;  // last entry with base <= slot
@@ -438,19 +438,19 @@ __global__ void __launch_bounds__(256) k_ximage(const ImgSrc* __restrict__ srcs,
         }
         const ImgSrc sr = srcs[lo];
         const double* b = sr.coef + (size_t)(sr.lb + (slot - sr.base)) * BS;
-        for (int e = threadIdx.x; e < BS; e += blockDim.x) blk[e] = (R)b[e];
+        for (int e = threadIdx.x; e < BS; e += blockDim.x) blk[e] = (float)b[e];
     } else {
         const double* g = gblk + (size_t)(slot - nreal) * KKK;
         for (int e = threadIdx.x; e < BS; e += blockDim.x) {
             const int a = e % K2, bb = (e / K2) % K2, c = e / (K2 * K2);
-            blk[e] = (a < K && bb < K && c < K) ? (R)g[a + K * (bb + K * c)] : R(0);
+            blk[e] = (a < K && bb < K && c < K) ? (float)g[a + K * (bb + K * c)] : 0.0f;
         }
     }
     __syncthreads();
-    R* out = img + (size_t)slot * K2 * NN;
+    float* out = img + (size_t)slot * K2 * NN;
     for (int e = threadIdx.x; e < K2 * NN; e += blockDim.x) {
         const int a = e / NN, j = e - a * NN, b = j % KP, c = j / KP;
-        out[e] = (b < K2 && c < K2) ? blk[a + K2 * (b + K2 * c)] : R(0);
+        out[e] = (b < K2 && c < K2) ? blk[a + K2 * (b + K2 * c)] : 0.0f;
     }
 }
 
@@ -786,28 +786,25 @@ __host__ __device__ constexpr int gcfg_nc(int k, int nthr) {
 }
 // Row-stride padding of the T1 (x-step output) and T2 (y-step output) buffers, chosen per basis size
 // so that the epilogue stores of a warp fall into few banks (counted wavefronts per step, consecutive
-// column tiles per warp; the FP64 x step with an odd tile width uses strided tiles).  In FP32 the T1
-// stride matches the 16-byte staging rows (T1 replaces a staged block at a line's end), which leaves
-// two-way conflicts on the once-per-line T1 stores at k = 9, 10.
-__host__ __device__ constexpr int gcfg_pad1(int k, bool f32) {
-    return f32 ? ((k == 5 || k == 6 || k == 9 || k == 10 || k == 11 || k == 12) ? 4 : 0) : 0;
+// column tiles per warp).  The T1 stride matches the 16-byte staging rows (T1 replaces a staged block at
+// a line's end), which leaves two-way conflicts on the once-per-line T1 stores at k = 9, 10.
+__host__ __device__ constexpr int gcfg_pad1(int k) {
+    return (k == 5 || k == 6 || k == 9 || k == 10 || k == 11 || k == 12) ? 4 : 0;
 }
 __host__ __device__ constexpr int gcfg_pad2(int k) {
     return (k == 5 || k == 6 || k == 9 || k == 10) ? 0 : (k == 11 || k == 12) ? 8 : 2;
 }
 
-template <int K, typename R>
+template <int K>
 struct GCfg {
-    static constexpr bool F32 = sizeof(R) == 4;
     static constexpr int K2 = 2 * K;
     static constexpr int KP = (K2 + 3) / 4 * 4;
     static constexpr int NN = KP * KP;
     static constexpr int MT = KP / 4;
-    static constexpr int NT = (F32 && MT * (KP / 2) <= 50) ? KP / 2 : KP / 4;
-    static constexpr int LDX = NN + (F32 ? 4 : 2);  // 16-byte rows: staged by cp.async from the block images
-    static constexpr int LD1 = NN + gcfg_pad1(K, F32);
+    static constexpr int NT = MT * (KP / 2) <= 50 ? KP / 2 : KP / 4;
+    static constexpr int LDX = NN + 4;  // 16-byte rows: staged by cp.async from the block images
+    static constexpr int LD1 = NN + gcfg_pad1(K);
     static constexpr int LD2 = NN + gcfg_pad2(K);
-    static constexpr bool XSTRIDED = !F32 && (NT % 2 == 1);
     static constexpr int NTILE = NN / NT;
     static constexpr int NWARP = (NTILE + 7) / 8;
     static constexpr int NTHR = 32 * NWARP;
@@ -816,21 +813,19 @@ struct GCfg {
     static constexpr int NC = gcfg_nc(K, NTHR);  // correction tile columns
     static constexpr int NCT = KK / NC;
     static constexpr int ND = MT * NT;  // accumulators per thread
-    // FP32: accumulators in TMEM, 2 columns per double, warps sharing a lane quarter side by side
+    // accumulators in TMEM, 2 columns per double, warps sharing a lane quarter side by side
     static constexpr int TCOLS_NEED = ((NWARP + 3) / 4) * 2 * ND;
     static constexpr int TCOLS = TCOLS_NEED <= 32 ? 32 : TCOLS_NEED <= 64 ? 64 : TCOLS_NEED <= 128 ? 128
                                  : TCOLS_NEED <= 256 ? 256 : 512;
     static constexpr int XBUF = KP * (LDX > LD1 ? LDX : LD1);  // one staging buffer: X, or T1 at a line's end
     static constexpr int IMG = K2 * NN;                          // block image: rows a < 2k of X, unpadded
     static constexpr size_t SMEM =
-        sizeof(R) * (2 * (size_t)XBUF + (size_t)KP * LD2 + 4 * (size_t)KP * KP + 3 * (size_t)KKK) + 64;
-    static constexpr int MINB = (F32 && 2 * (SMEM + 16 + 1024) <= 233472) ? 2 : 1;
+        sizeof(float) * (2 * (size_t)XBUF + (size_t)KP * LD2 + 4 * (size_t)KP * KP + 3 * (size_t)KKK) + 64;
+    static constexpr int MINB = 2 * (SMEM + 16 + 1024) <= 233472 ? 2 : 1;
     static constexpr bool FITS = SMEM + 16 + 1024 <= 232448 && 2 * NCT <= NTHR && TCOLS_NEED <= 512 &&
-                                 (size_t)KP * LDX * sizeof(R) >= 64 * sizeof(double) && (!F32 || TCOLS * MINB <= 512);
+                                 (size_t)KP * LDX * sizeof(float) >= 64 * sizeof(double) && TCOLS * MINB <= 512;
+    static_assert(NT % 2 == 0, "column pairs");
 };
-
-__device__ __forceinline__ float mfma(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double mfma(double a, double b, double c) { return fma(a, b, c); }
 
 // packed FP32 pairs (sm_100 f32x2 arithmetic): two independent round-to-nearest FMAs per instruction,
 // bit-identical to two fmaf calls
@@ -849,76 +844,8 @@ __device__ __forceinline__ void unpack_f32x2(unsigned long long v, float& lo, fl
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
-// c (+)= At^T B on a thread tile: c[i][j] (+)= sum_{k < kdim} At[k lda + o0 + i] B[k ldb + n0 + j]
-template <int MT, int NT, bool ACC, typename R, typename CT>
-__device__ __forceinline__ void gemm_tile(const R* __restrict__ At, int lda, const R* __restrict__ B, int ldb,
-                                          int o0, int n0, int kdim, CT (&c)[MT][NT]) {
-    if constexpr (sizeof(R) == 4 && sizeof(CT) == 4 && NT % 2 == 0) {
-        // FP32 tile: column pairs in packed registers, one f32x2 FMA per pair and contracted index
-        constexpr int NP = NT / 2;
-        unsigned long long pc[MT][NP];
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NP; ++j) pc[i][j] = ACC ? pack_f32x2(c[i][2 * j], c[i][2 * j + 1]) : 0ull;
-        const R* ap = At + o0;
-        const R* bp = B + n0;
-#pragma unroll 2
-        for (int k = 0; k < kdim; ++k) {
-            unsigned long long a2[MT], b2[NP];
-#pragma unroll
-            for (int i = 0; i < MT; ++i) a2[i] = pack_f32x2(ap[i], ap[i]);
-#pragma unroll
-            for (int j = 0; j < NP; ++j) b2[j] = *reinterpret_cast<const unsigned long long*>(bp + 2 * j);
-#pragma unroll
-            for (int i = 0; i < MT; ++i)
-#pragma unroll
-                for (int j = 0; j < NP; ++j) pc[i][j] = fma_f32x2(a2[i], b2[j], pc[i][j]);
-            ap += lda;
-            bp += ldb;
-        }
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NP; ++j) unpack_f32x2(pc[i][j], c[i][2 * j], c[i][2 * j + 1]);
-        return;
-    }
-    if (!ACC) {
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NT; ++j) c[i][j] = CT(0);
-    }
-    const R* ap = At + o0;
-    const R* bp = B + n0;
-#pragma unroll 2
-    for (int k = 0; k < kdim; ++k) {
-        R a[MT], b[NT];
-#pragma unroll
-        for (int i = 0; i < MT; ++i) a[i] = ap[i];
-        if constexpr (NT % 2 == 0) {
-            using V2 = typename std::conditional<sizeof(R) == 4, float2, double2>::type;
-#pragma unroll
-            for (int j = 0; j < NT; j += 2) {
-                const V2 v = *reinterpret_cast<const V2*>(bp + j);
-                b[j] = v.x;
-                b[j + 1] = v.y;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < NT; ++j) b[j] = bp[j];
-        }
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NT; ++j) c[i][j] = mfma((CT)a[i], (CT)b[j], c[i][j]);
-        ap += lda;
-        bp += ldb;
-    }
-}
-
 // FP32 tile with packed accumulators kept across calls: pc[i][j] (+)= sum_k At[k lda + o0 + i] times the
-// column pair B[k ldb + n0 + 2j], B[k ldb + n0 + 2j + 1] (the same FMAs as gemm_tile's FP32 path)
+// column pair B[k ldb + n0 + 2j], B[k ldb + n0 + 2j + 1], one f32x2 FMA per pair and contracted index
 template <int MT, int NP>
 __device__ __forceinline__ void gemm_tile_packed(const float* __restrict__ At, int lda, const float* __restrict__ B,
                                                  int ldb, int o0, int n0, int kdim, unsigned long long (&pc)[MT][NP]) {
@@ -940,16 +867,32 @@ __device__ __forceinline__ void gemm_tile_packed(const float* __restrict__ At, i
     }
 }
 
-// the same with per-column offsets (correction GEMMs; columns not contiguous)
-template <int MT, int NT, typename R>
-__device__ __forceinline__ void gemm_tile_off(const R* __restrict__ At, int lda, const R* __restrict__ B, int ldb,
-                                              int o0, const int (&off)[NT], int kdim, R (&c)[MT][NT]) {
+// c = At^T B on a thread tile: packed products, unpacked result
+template <int MT, int NT>
+__device__ __forceinline__ void gemm_tile(const float* __restrict__ At, int lda, const float* __restrict__ B, int ldb,
+                                          int o0, int n0, int kdim, float (&c)[MT][NT]) {
+    unsigned long long pc[MT][NT / 2];
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < NT; ++j) c[i][j] = R(0);
+        for (int j = 0; j < NT / 2; ++j) pc[i][j] = 0ull;
+    gemm_tile_packed<MT, NT / 2>(At, lda, B, ldb, o0, n0, kdim, pc);
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT / 2; ++j) unpack_f32x2(pc[i][j], c[i][2 * j], c[i][2 * j + 1]);
+}
+
+// the same with per-column offsets (correction GEMMs; columns not contiguous)
+template <int MT, int NT>
+__device__ __forceinline__ void gemm_tile_off(const float* __restrict__ At, int lda, const float* __restrict__ B, int ldb,
+                                              int o0, const int (&off)[NT], int kdim, float (&c)[MT][NT]) {
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) c[i][j] = 0.0f;
     for (int k = 0; k < kdim; ++k) {
-        R a[MT], b[NT];
+        float a[MT], b[NT];
 #pragma unroll
         for (int i = 0; i < MT; ++i) a[i] = At[k * lda + o0 + i];
 #pragma unroll
@@ -957,7 +900,7 @@ __device__ __forceinline__ void gemm_tile_off(const R* __restrict__ At, int lda,
 #pragma unroll
         for (int i = 0; i < MT; ++i)
 #pragma unroll
-            for (int j = 0; j < NT; ++j) c[i][j] = mfma(a[i], b[j], c[i][j]);
+            for (int j = 0; j < NT; ++j) c[i][j] = fmaf(a[i], b[j], c[i][j]);
     }
 }
 
@@ -969,95 +912,80 @@ __device__ __forceinline__ void gemm_tile_off(const R* __restrict__ At, int lda,
 // product (summed over its plane in T2) and every plane one z mode product (summed into the output
 // block), instead of three mode products per triple.  The s->s correction below the root follows the
 // same grouping on its k^3 blocks.
-// Input blocks are staged from their images (the X layout in `R`, built per pass) into two buffers
+// Input blocks are staged from their images (the X layout in FP32, built per pass) into two buffers
 // by cp.async: the next triple's block and operator load while the current triple computes.  At a
 // line's end its x sums (T1) replace the line's last block in its buffer.
 // tkey (sorted): item << 32 | term << 20 | dz rank << 10 | dy rank; tval: candidate << 32 | term entry.
-template <int K, typename R>
-__global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
+template <int K>
+__global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
     k_gapply(const Chunk* __restrict__ chunks, const Item* __restrict__ items, const BTree* __restrict__ trees,
              const unsigned long long* __restrict__ tkey, const unsigned long long* __restrict__ tval,
-             const int* __restrict__ csrc, const R* __restrict__ ximg, long long gbase, double* partials,
+             const int* __restrict__ csrc, const float* __restrict__ ximg, long long gbase, double* partials,
              unsigned long long* ntrip_out) {
-    using C = GCfg<K, R>;
+    using C = GCfg<K>;
     constexpr int K2 = C::K2, KP = C::KP, MT = C::MT, NT = C::NT, NC = C::NC, ND = C::ND;
     constexpr int LDX = C::LDX, LD1 = C::LD1, LD2 = C::LD2, NN = C::NN, IMG = C::IMG;
     constexpr int KK = C::KK, KKK = C::KKK;
     constexpr int BS = K2 * K2 * K2;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ uint32_t tmem_slot;
-    R* XA = reinterpret_cast<R*>(smraw);  // staging buffers: X [KP][LDX], or T1 [KP][LD1]
-    R* XB = XA + C::XBUF;
-    R* T2 = XB + C::XBUF;                 // [KP][LD2]
-    R* Mx0 = T2 + KP * LD2;               // [KP][KP], At[k][o] = M[o][k]; x operators of the two buffers
-    R* Mx1 = Mx0 + KP * KP;
-    R* My = Mx1 + KP * KP;
-    R* Mz = My + KP * KP;
-    R* U1 = Mz + KP * KP;  // [K][K][K]
-    R* U2 = U1 + KKK;
-    R* Uc = U2 + KKK;
+    float* XA = reinterpret_cast<float*>(smraw);  // staging buffers: X [KP][LDX], or T1 [KP][LD1]
+    float* XB = XA + C::XBUF;
+    float* T2 = XB + C::XBUF;                 // [KP][LD2]
+    float* Mx0 = T2 + KP * LD2;               // [KP][KP], At[k][o] = M[o][k]; x operators of the two buffers
+    float* Mx1 = Mx0 + KP * KP;
+    float* My = Mx1 + KP * KP;
+    float* Mz = My + KP * KP;
+    float* U1 = Mz + KP * KP;  // [K][K][K]
+    float* U2 = U1 + KKK;
+    float* Uc = U2 + KKK;
     const Chunk ch = chunks[blockIdx.x];
     const Item it = items[ch.item];
     const BTree& TR = trees[it.tree];
-    const R* mats = reinterpret_cast<const R*>(C::F32 ? (const void*)TR.matsT32 : (const void*)TR.matsT);
-    const R* matsb = reinterpret_cast<const R*>(C::F32 ? (const void*)TR.matsbT32 : (const void*)TR.matsbT);
+    const float* mats = TR.matsT32;
+    const float* matsb = TR.matsbT32;
     const bool root = TR.root != 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // tiles: 4 row tiles x 8 column tiles per warp; consecutive column tiles (y and z steps, and the
-    // x step unless strided), or column tiles strided by the warp count (x step)
+    // tiles: 4 row tiles x 8 consecutive column tiles per warp
     const int rt = lane & 3;
     const int ct_c = warp * 8 + (lane >> 2);
-    const int ct_x = C::XSTRIDED ? warp + C::NWARP * (lane >> 2) : ct_c;
-    const bool own = ct_c < C::NTILE, own_x = ct_x < C::NTILE;
+    const bool own = ct_c < C::NTILE;
     const int o0 = rt * MT;
-    const int n0 = own ? ct_c * NT : 0, n0x = own_x ? ct_x * NT : 0;
-    const int tb0 = n0 % KP, tc0 = n0 / KP;     // y tile: first a', c;  z tile: first a', b'
-    const int xb0 = n0x % KP, xc0 = n0x / KP;   // x tile: first b, c
+    const int n0 = own ? ct_c * NT : 0;
+    const int tb0 = n0 % KP, tc0 = n0 / KP;     // x tile: first b, c;  y tile: first a', c;  z tile: first a', b'
     // correction tile
     const int crt = tid & 1, cct = tid >> 1;
     const bool cown = !root && cct < C::NCT;
     const int co0 = crt * MT, cn0 = cown ? cct * NC : 0;
 
-    // accumulators: registers (FP64 kernel) or this thread's TMEM lane (FP32 kernel)
-    double acc[C::F32 ? 1 : MT][C::F32 ? 1 : NT];
-    uint32_t tacc = 0;
-    if constexpr (C::F32) {
-        if (warp == 0) {
-            tmem_alloc(&tmem_slot, C::TCOLS);
-            tmem_relinquish();
-        }
-        tmem_fence_before_sync();
-        __syncthreads();
-        tmem_fence_after_sync();
-        tacc = tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * 2 * ND);
-        tmem_visit<ND, true>(tacc, [&](int, int n, auto& r) {
-#pragma unroll
-            for (int q = 0; q < 2 * n; ++q) r[q] = 0u;
-        });
-    } else {
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NT; ++j) acc[i][j] = 0.0;
+    // accumulators: this thread's TMEM lane
+    if (warp == 0) {
+        tmem_alloc(&tmem_slot, C::TCOLS);
+        tmem_relinquish();
     }
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    const uint32_t tacc = tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * 2 * ND);
+    tmem_visit<ND, true>(tacc, [&](int, int n, auto& r) {
+#pragma unroll
+        for (int q = 0; q < 2 * n; ++q) r[q] = 0u;
+    });
     unsigned long long ntrip = 0;
     bool pend2 = false;     // c2 holds a correction block not yet written to Uc
     bool uc_valid = false;  // Uc holds a correction block not yet subtracted
-    R c2[MT][NC];
-    // x sums of the current line (this thread's x tile): FP32 column pairs packed (f32x2), or plain
-    constexpr bool PK = C::F32 && NT % 2 == 0;
-    unsigned long long xp[PK ? MT : 1][PK ? NT / 2 : 1];
-    R xacc[PK ? 1 : MT][PK ? 1 : NT];
+    float c2[MT][NC];
+    unsigned long long xp[MT][NT / 2];  // x sums of the current line (this thread's x tile), column pairs packed
 
     // asynchronous copy of a transposed operator (At[k][o] = M[o][k], P x P) into shared memory, as
     // one commit group
-    auto load_mat = [&](R* dst, const R* tab, int mi) {
-        constexpr int NV = KP * KP * (int)sizeof(R) / 16;
+    auto load_mat = [&](float* dst, const float* tab, int mi) {
+        constexpr int NV = KP * KP * (int)sizeof(float) / 16;
         const char* src = reinterpret_cast<const char*>(tab + (size_t)mi * KP * KP);
         for (int e = tid; e < NV; e += blockDim.x) cp_async16(reinterpret_cast<char*>(dst) + 16 * e, src + 16 * e);
         cp_async_commit();
     };
-    auto image_of = [&](int t) -> const R* {
+    auto image_of = [&](int t) -> const float* {
         const int src = csrc[(int)(tval[t] >> 32)];
         const long long slot = src < 0 ? gbase + (-src - 1) : TR.img_base + (src - TR.img_lb);
         return ximg + (size_t)slot * IMG;
@@ -1065,10 +993,10 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
     // triple t's block image into buffer q (rows a < 2k; the rows of X beyond are never read) and its
     // x operator, one commit group
     auto stage = [&](int t, int q) {
-        const R* img = image_of(t);
-        R* dst = q ? XB : XA;
-        constexpr int RV = NN * (int)sizeof(R) / 16;  // 16-byte vectors per row
-        constexpr int EV = 16 / (int)sizeof(R);
+        const float* img = image_of(t);
+        float* dst = q ? XB : XA;
+        constexpr int RV = NN * (int)sizeof(float) / 16;  // 16-byte vectors per row
+        constexpr int EV = 16 / (int)sizeof(float);
         for (int e = tid; e < K2 * RV; e += blockDim.x) {
             const int a = e / RV, v = e - a * RV;
             cp_async16(dst + a * LDX + v * EV, img + (size_t)a * NN + v * EV);
@@ -1118,37 +1046,25 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
         if (lend) load_mat(My, mats, tr.my);
         if (pend) load_mat(Mz, matsb, tr.mz);
         if (more) stage(t + 1, q ^ 1);
-        if (tid == 0 && t + 2 < ch.c1) prefetch_l2_bulk(image_of(t + 2), (unsigned)(IMG * sizeof(R)));
-        R* Xq = q ? XB : XA;
-        const R* Mxq = q ? Mx1 : Mx0;
-        // ---- x: xacc[a'][b + P c] (+)= sum_a Mx[a'][a] X[a][b + P c]   (a line sums its triples)
-        if (own_x) {
-            const bool live = !gen || (xb0 < K && xc0 < K);  // other tiles of a generated input are zero
-            if constexpr (PK) {
-                if (lstart) {
+        if (tid == 0 && t + 2 < ch.c1) prefetch_l2_bulk(image_of(t + 2), (unsigned)(IMG * sizeof(float)));
+        float* Xq = q ? XB : XA;
+        const float* Mxq = q ? Mx1 : Mx0;
+        // ---- x: xp[a'][b + P c] (+)= sum_a Mx[a'][a] X[a][b + P c]   (a line sums its triples)
+        if (own) {
+            const bool live = !gen || (tb0 < K && tc0 < K);  // other tiles of a generated input are zero
+            if (lstart) {
 #pragma unroll
-                    for (int i = 0; i < MT; ++i)
+                for (int i = 0; i < MT; ++i)
 #pragma unroll
-                        for (int j = 0; j < NT / 2; ++j) xp[i][j] = 0ull;
-                }
-                if (live)
-                    gemm_tile_packed<MT, NT / 2>(reinterpret_cast<const float*>(Mxq), KP,
-                                                 reinterpret_cast<const float*>(Xq), LDX, o0, n0x, gen ? K : K2, xp);
-            } else {
-                if (lstart) {
-#pragma unroll
-                    for (int i = 0; i < MT; ++i)
-#pragma unroll
-                        for (int j = 0; j < NT; ++j) xacc[i][j] = R(0);
-                }
-                if (live) gemm_tile<MT, NT, true>(Mxq, KP, Xq, LDX, o0, n0x, gen ? K : K2, xacc);
+                    for (int j = 0; j < NT / 2; ++j) xp[i][j] = 0ull;
             }
+            if (live) gemm_tile_packed<MT, NT / 2>(Mxq, KP, Xq, LDX, o0, n0, gen ? K : K2, xp);
         }
         if (cown) {  // U1[b][a' + k c] (+)= sum_{a<k} Tx[a'][a] X[a][b + P c]   (summed over the line)
             int off[NC];
 #pragma unroll
             for (int j = 0; j < NC; ++j) off[j] = (cn0 + j) % K + KP * ((cn0 + j) / K);
-            R c[MT][NC];
+            float c[MT][NC];
             gemm_tile_off<MT, NC>(Mxq, KP, Xq, LDX, co0, off, K, c);
 #pragma unroll
             for (int i = 0; i < MT; ++i)
@@ -1156,7 +1072,7 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
                 for (int j = 0; j < NC; ++j) {
                     const int n = cn0 + j;
                     if (co0 + i < K) {
-                        R& d = U1[(n % K) * KK + co0 + i + K * (n / K)];
+                        float& d = U1[(n % K) * KK + co0 + i + K * (n / K)];
                         d = lstart ? c[i][j] : d + c[i][j];
                     }
                 }
@@ -1164,24 +1080,17 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
         ++ntrip;
         if (!lend) continue;
         __syncthreads();  // every reader of Xq is done: the line's x sums replace its last block
-        R* T1 = Xq;       // [KP][LD1]
-        if (own_x) {
-            if constexpr (PK) {
+        float* T1 = Xq;       // [KP][LD1]
+        if (own) {
 #pragma unroll
-                for (int j = 0; j < NT / 2; ++j)
+            for (int j = 0; j < NT / 2; ++j)
 #pragma unroll
-                    for (int i = 0; i < MT; ++i) {
-                        float lo, hi;
-                        unpack_f32x2(xp[i][j], lo, hi);
-                        T1[(xb0 + 2 * j) * LD1 + o0 + i + KP * xc0] = lo;
-                        T1[(xb0 + 2 * j + 1) * LD1 + o0 + i + KP * xc0] = hi;
-                    }
-            } else {
-#pragma unroll
-                for (int j = 0; j < NT; ++j)
-#pragma unroll
-                    for (int i = 0; i < MT; ++i) T1[(xb0 + j) * LD1 + o0 + i + KP * xc0] = xacc[i][j];
-            }
+                for (int i = 0; i < MT; ++i) {
+                    float lo, hi;
+                    unpack_f32x2(xp[i][j], lo, hi);
+                    T1[(tb0 + 2 * j) * LD1 + o0 + i + KP * tc0] = lo;
+                    T1[(tb0 + 2 * j + 1) * LD1 + o0 + i + KP * tc0] = hi;
+                }
         }
         // My (and Mz) were committed before the next triple's staging group
         if (more) cp_async_wait_group<1>();
@@ -1196,36 +1105,30 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
         if (own) {
             const bool zero = line_gen && !(tc0 < K);  // this tile is zero for generated inputs
             if (!zero || first_line) {
-                R c[MT][NT];
+                float c[MT][NT];
                 if (zero) {
 #pragma unroll
                     for (int i = 0; i < MT; ++i)
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) c[i][j] = R(0);
+                        for (int j = 0; j < NT; ++j) c[i][j] = float(0);
                 } else {
-                    gemm_tile<MT, NT, false>(My, KP, T1, LD1, o0, n0, line_gen ? K : K2, c);
+                    gemm_tile<MT, NT>(My, KP, T1, LD1, o0, n0, line_gen ? K : K2, c);
                 }
 #pragma unroll
                 for (int i = 0; i < MT; ++i) {
-                    R* row = T2 + tc0 * LD2 + tb0 + KP * (o0 + i);
-                    if constexpr (NT % 2 == 0) {
-                        using V2 = typename std::conditional<sizeof(R) == 4, float2, double2>::type;
+                    float* row = T2 + tc0 * LD2 + tb0 + KP * (o0 + i);
 #pragma unroll
-                        for (int j = 0; j < NT; j += 2) {
-                            V2 v;
-                            if (first_line) {
-                                v.x = c[i][j];
-                                v.y = c[i][j + 1];
-                            } else {
-                                v = *reinterpret_cast<const V2*>(row + j);
-                                v.x += c[i][j];
-                                v.y += c[i][j + 1];
-                            }
-                            *reinterpret_cast<V2*>(row + j) = v;
+                    for (int j = 0; j < NT; j += 2) {
+                        float2 v;
+                        if (first_line) {
+                            v.x = c[i][j];
+                            v.y = c[i][j + 1];
+                        } else {
+                            v = *reinterpret_cast<const float2*>(row + j);
+                            v.x += c[i][j];
+                            v.y += c[i][j + 1];
                         }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < NT; ++j) row[j] = first_line ? c[i][j] : row[j] + c[i][j];
+                        *reinterpret_cast<float2*>(row + j) = v;
                     }
                 }
             }
@@ -1234,7 +1137,7 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
             int off[NC];
 #pragma unroll
             for (int j = 0; j < NC; ++j) off[j] = cn0 + j;
-            R c[MT][NC];
+            float c[MT][NC];
             gemm_tile_off<MT, NC>(My, KP, U1, KK, co0, off, K, c);
 #pragma unroll
             for (int i = 0; i < MT; ++i)
@@ -1242,7 +1145,7 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
                 for (int j = 0; j < NC; ++j) {
                     const int n = cn0 + j;
                     if (co0 + i < K) {
-                        R& d = U2[(n / K) * KK + (n % K) + K * (co0 + i)];
+                        float& d = U2[(n / K) * KK + (n % K) + K * (co0 + i)];
                         d = first_line ? c[i][j] : d + c[i][j];
                     }
                 }
@@ -1252,10 +1155,10 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
         __syncthreads();  // T2, U2 and Uc of the plane are complete
         // ---- z: acc[c'][a' + P b'] += sum_c (beta Mz)[c'][c] T2[c][a' + P b']  (- previous correction)
         const int kdz = plane_gen ? K : K2;
-        if constexpr (C::F32) {
+        {
             float c[MT][NT];
             if (own) {
-                gemm_tile<MT, NT, false>(Mz, KP, T2, LD2, o0, n0, kdz, c);
+                gemm_tile<MT, NT>(Mz, KP, T2, LD2, o0, n0, kdz, c);
             } else {
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
@@ -1272,16 +1175,6 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
                     double_to_words(v, r[2 * q2], r[2 * q2 + 1]);
                 }
             });
-        } else {
-            if (own) {
-                gemm_tile<MT, NT, true>(Mz, KP, T2, LD2, o0, n0, kdz, acc);
-                if (uc_valid) {
-#pragma unroll
-                    for (int i = 0; i < MT; ++i)
-#pragma unroll
-                        for (int j = 0; j < NT; ++j) acc[i][j] -= uc_at(i, j);
-                }
-            }
         }
         uc_valid = false;
         if (cown) {  // c2[c'][a' + k b'] = sum_{c<k} (beta Tz)[c'][c] U2[c][a' + k b']
@@ -1308,26 +1201,17 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
             if (!(ax < K && by < K && cz < K)) w2 += v * v;
         }
     };
-    if constexpr (C::F32) {
-        tmem_visit<ND, false>(tacc, [&](int d0, int n, auto& r) {
+    tmem_visit<ND, false>(tacc, [&](int d0, int n, auto& r) {
 #pragma unroll
-            for (int q = 0; q < n; ++q) {
-                const int d = d0 + q;
-                if (own) emit(d / NT, d % NT, words_to_double(r[2 * q], r[2 * q + 1]));
-            }
-        });
-        tmem_fence_before_sync();
-        __syncthreads();
-        tmem_fence_after_sync();
-        if (warp == 0) tmem_dealloc(tmem_slot, C::TCOLS);
-    } else {
-        if (own) {
-#pragma unroll
-            for (int i = 0; i < MT; ++i)
-#pragma unroll
-                for (int j = 0; j < NT; ++j) emit(i, j, acc[i][j]);
+        for (int q = 0; q < n; ++q) {
+            const int d = d0 + q;
+            if (own) emit(d / NT, d % NT, words_to_double(r[2 * q], r[2 * q + 1]));
         }
-    }
+    });
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    if (warp == 0) tmem_dealloc(tmem_slot, C::TCOLS);
     double* red = reinterpret_cast<double*>(XA);  // the staging buffers are no longer read
     __syncthreads();
     block_sum2(n2, w2, red);
@@ -1343,6 +1227,7 @@ __global__ void __launch_bounds__(GCfg<K, R>::NTHR, GCfg<K, R>::MINB)
 }  // namespace mwb
 #include "mw_tapply.cuh"
 #include "mw_happly.cuh"
+#include "mw_dapply.cuh"
 namespace mwb {
 
 // triples of every chunk (the sort key of the longest-first launch order); chunks never exceed 2^16 triples
@@ -1521,9 +1406,9 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
         d.mats32 = b.tab->d_mats32;
         d.matsb = b.tab->d_matsb;
         d.matsb32 = b.tab->d_matsb32;
-        d.matsT = b.tab->d_matsT;
+        d.matsD = b.tab->d_matsD;
+        d.matsDbeta = b.tab->d_mbeta;
         d.matsT32 = b.tab->d_matsT32;
-        d.matsbT = b.tab->d_matsbT;
         d.matsbT32 = b.tab->d_matsbT32;
         d.matsI = b.tab->d_matsI;
         d.matsbI = b.tab->d_matsbI;
@@ -1635,11 +1520,12 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     // the GEMM-tiled engine runs the line-ordered contraction (chunks of sorted triples); the
     // tensor-core and pencil engines take chunks of whole candidates
     bool lined = false, lined32 = false, hyb = false;
+    const bool fp64 = !pencil && bp.precision == 0;
 #define L_ENG(KK)                                                                                    \
     hyb = !pencil && bp.precision == 3 && HCfg<KK>::FITS;                                            \
-    lined = hyb || (!pencil && !(bp.precision == 2 && TCfg<KK>::FITS && tc_prec_ok) &&               \
-            ((bp.precision >= 1 && GCfg<KK, float>::FITS) || (bp.precision != 1 && GCfg<KK, double>::FITS))); \
-    lined32 = lined && !hyb && bp.precision >= 1 && GCfg<KK, float>::FITS;
+    lined32 = !pencil && !hyb && bp.precision >= 1 && GCfg<KK>::FITS &&                              \
+              !(bp.precision == 2 && TCfg<KK>::FITS && tc_prec_ok);                                  \
+    lined = fp64 || hyb || lined32;
     MWB_DISPATCH_K(K, L_ENG)
 #undef L_ENG
     int* d_cand_item = (int*)dalloc(ctx, sizeof(int) * ncap);
@@ -1717,15 +1603,13 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
         if (hyb) {                                                                                              \
             d_ximg = launch_simage<KK>(ctx, nimg, d_srcs, nt, d_gblk, nreal, s);                                \
         } else if (lined32) {                                                                                   \
-            d_ximg = dalloc(ctx, sizeof(float) * (size_t)nimg * GCfg<KK, float>::IMG);                          \
+            d_ximg = dalloc(ctx, sizeof(float) * (size_t)nimg * GCfg<KK>::IMG);                                 \
             const int smem = (int)(sizeof(float) * 8 * KK * KK * KK);                                          \
-            MWB_CUDA(cudaFuncSetAttribute(k_ximage<KK, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-            k_ximage<KK, float><<<(unsigned)nimg, 256, smem, s>>>(d_srcs, nt, d_gblk, nreal, (float*)d_ximg);    \
+            MWB_CUDA(cudaFuncSetAttribute(k_ximage<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));    \
+            k_ximage<KK><<<(unsigned)nimg, 256, smem, s>>>(d_srcs, nt, d_gblk, nreal, (float*)d_ximg);           \
         } else {                                                                                                \
-            d_ximg = dalloc(ctx, sizeof(double) * (size_t)nimg * GCfg<KK, double>::IMG);                        \
-            const int smem = (int)(sizeof(double) * 8 * KK * KK * KK);                                         \
-            MWB_CUDA(cudaFuncSetAttribute(k_ximage<KK, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-            k_ximage<KK, double><<<(unsigned)nimg, 256, smem, s>>>(d_srcs, nt, d_gblk, nreal, (double*)d_ximg);  \
+            d_ximg = dalloc(ctx, sizeof(double) * (size_t)nimg * DCfg<KK>::IMG);                                \
+            k_dimage<KK><<<(unsigned)nimg, 256, 0, s>>>(d_srcs, nt, d_gblk, nreal, (double*)d_ximg);             \
         }                                                                                                       \
     }
             MWB_DISPATCH_K(K, L_IMG)
@@ -1786,18 +1670,18 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
             MWB_CUDA(cudaFuncSetAttribute(k_tapply<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
             k_tapply<KK><<<nchunks, TCfg<KK>::NTHR, smem, s>>>(d_chunks, d_items, d_trees, d_cdelta, d_csrc,     \
                                                                d_gblk, d_gnorm2, d_partials, d_ntrip_tot, d_kerr); \
-        } else if (bp.precision >= 1 && GCfg<KK, float>::FITS && !pencil) {                                  \
-            size_t smem = GCfg<KK, float>::SMEM;                                                             \
-            MWB_CUDA(cudaFuncSetAttribute(k_gapply<KK, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-            k_gapply<KK, float><<<nchunks, GCfg<KK, float>::NTHR, smem, s>>>(d_run, d_items, d_trees, d_tkey,    \
-                                                                              d_tval, d_csrc, (const float*)d_ximg, \
-                                                                              nreal, d_partials, d_ntrip_tot);     \
-        } else if (bp.precision != 1 && GCfg<KK, double>::FITS && !pencil) {                                  \
-            size_t smem = GCfg<KK, double>::SMEM;                                                            \
-            MWB_CUDA(cudaFuncSetAttribute(k_gapply<KK, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-            k_gapply<KK, double><<<nchunks, GCfg<KK, double>::NTHR, smem, s>>>(d_run, d_items, d_trees, d_tkey,   \
-                                                                                d_tval, d_csrc, (const double*)d_ximg, \
-                                                                                nreal, d_partials, d_ntrip_tot);    \
+        } else if (fp64) {                                                                                   \
+            size_t smem = DCfg<KK>::SMEM;                                                                    \
+            MWB_CUDA(cudaFuncSetAttribute(k_dapply<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+            k_dapply<KK><<<nchunks, DCfg<KK>::NTHR, smem, s>>>(d_run, d_items, d_trees, d_tkey, d_tval, d_csrc,  \
+                                                               (const double*)d_ximg, nreal, d_partials,         \
+                                                               d_ntrip_tot);                                     \
+        } else if (lined32) {                                                                                \
+            size_t smem = GCfg<KK>::SMEM;                                                                    \
+            MWB_CUDA(cudaFuncSetAttribute(k_gapply<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+            k_gapply<KK><<<nchunks, GCfg<KK>::NTHR, smem, s>>>(d_run, d_items, d_trees, d_tkey, d_tval, d_csrc,  \
+                                                               (const float*)d_ximg, nreal, d_partials,          \
+                                                               d_ntrip_tot);                                     \
         } else if (bp.precision >= 1) {                                                                      \
             size_t smem = ACfg<KK, float>::SMEM;                                                             \
             MWB_CUDA(cudaFuncSetAttribute(k_bapply<KK, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \

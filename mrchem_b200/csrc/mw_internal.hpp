@@ -108,11 +108,13 @@ struct OpDepth {
     float* d_mats32 = nullptr;  // FP32 copy of d_mats (mixed-precision apply)
     double* d_matsb = nullptr;  // each matrix scaled by its term's beta (z-step operators)
     float* d_matsb32 = nullptr;
-    // the same four tables transposed and zero-padded to P x P (P = 2k rounded up to a multiple of
-    // 4), entry [k][o] = M[o][k]: the layout the GEMM-tiled contraction copies into shared memory
-    double* d_matsT = nullptr;
+    // FP64 matrix-instruction contraction (k_dapply): every matrix as A fragments, [step s][row tile r]
+    // [lane], lane 4 n + i holding M[8 r + n][4 s + i] (zero outside), and its term's beta
+    double* d_matsD = nullptr;
+    double* d_mbeta = nullptr;
+    // the FP32 tables transposed and zero-padded to P x P (P = 2k rounded up to a multiple of 4), entry
+    // [k][o] = M[o][k]: the layout the GEMM-tiled contraction copies into shared memory
     float* d_matsT32 = nullptr;
-    double* d_matsbT = nullptr;
     float* d_matsbT32 = nullptr;
     // split-TF32 operator images for the tensor-core contraction: per matrix one K-major FP32 image of
     // 3 KP8 rows and KP8 columns (KP8 = 2k rounded up to a multiple of 8, zero padding): rows o,
