@@ -331,7 +331,7 @@ Op::~Op() {
         dfree(c, kv.second->d_matsb32);
         dfree(c, kv.second->d_matsD);
         dfree(c, kv.second->d_matsT32);
-        dfree(c, kv.second->d_mbeta);
+        dfree(c, kv.second->d_matsE);
         dfree(c, kv.second->d_matsbT32);
         dfree(c, kv.second->d_matsI);
         dfree(c, kv.second->d_matsbI);
@@ -625,18 +625,22 @@ static const OpDepth& op_depth(Op& op, int depth, int dir = 0) {
     std::vector<float> mT32(mT.begin(), mT.end()), mbT32(mbT.begin(), mbT.end());
     od->d_matsT32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mT.size()));
     od->d_matsbT32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mT.size()));
-    // A fragments of the FP64 matrix instruction
+    // A and B fragments of the FP64 matrix instruction
     const int dRT = (K2 + 7) / 8, dS = (K2 + 3) / 4;
-    std::vector<double> mD(nmat * dRT * dS * 32, 0.0);
+    std::vector<double> mD(nmat * dRT * dS * 32, 0.0), mE(nmat * dRT * dS * 32, 0.0);
     for (size_t mi = 0; mi < nmat; ++mi)
         for (int o = 0; o < K2; ++o)
-            for (int k = 0; k < K2; ++k)
+            for (int k = 0; k < K2; ++k) {
+                const int n = 2 * (o % 4) + (o % 8) / 4;  // B fragment column of row o
                 mD[((mi * dS + k / 4) * dRT + o / 8) * 32 + 4 * (o % 8) + k % 4] = od->mats[mi * K2 * K2 + (size_t)o * K2 + k];
+                mE[((mi * dRT + o / 8) * dS + k / 4) * 32 + 4 * n + k % 4] = mb[mi * K2 * K2 + (size_t)o * K2 + k];
+            }
     od->d_matsD = (double*)dalloc(ctx, sizeof(double) * std::max<size_t>(1, mD.size()));
-    od->d_mbeta = (double*)dalloc(ctx, sizeof(double) * std::max<size_t>(1, mbeta.size()));
-    if (!mD.empty()) MWB_CUDA(cudaMemcpyAsync(od->d_matsD, mD.data(), sizeof(double) * mD.size(), cudaMemcpyHostToDevice, s));
-    if (!mbeta.empty())
-        MWB_CUDA(cudaMemcpyAsync(od->d_mbeta, mbeta.data(), sizeof(double) * mbeta.size(), cudaMemcpyHostToDevice, s));
+    od->d_matsE = (double*)dalloc(ctx, sizeof(double) * std::max<size_t>(1, mE.size()));
+    if (!mD.empty()) {
+        MWB_CUDA(cudaMemcpyAsync(od->d_matsD, mD.data(), sizeof(double) * mD.size(), cudaMemcpyHostToDevice, s));
+        MWB_CUDA(cudaMemcpyAsync(od->d_matsE, mE.data(), sizeof(double) * mE.size(), cudaMemcpyHostToDevice, s));
+    }
     // split-TF32 images: three TF32 pieces per entry (hi, mid, lo: each the TF32 rounding of what the
     // previous pieces leave of the FP64 value)
     const int KP8 = (K2 + 7) / 8 * 8;

@@ -47,7 +47,7 @@ struct BTree {
     const double* matsb;    // beta-scaled copies (z-step operators)
     const float* matsb32;
     const double* matsD;      // fragment images (FP64 matrix-instruction contraction)
-    const double* matsDbeta;  // the term weight of every matrix
+    const double* matsE;
     const float* matsT32;     // transposed, zero-padded copies (GEMM-tiled FP32 contraction)
     const float* matsbT32;
     const float* matsI;  // split-TF32 operator images (tensor-core contraction)
@@ -1407,7 +1407,7 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
         d.matsb = b.tab->d_matsb;
         d.matsb32 = b.tab->d_matsb32;
         d.matsD = b.tab->d_matsD;
-        d.matsDbeta = b.tab->d_mbeta;
+        d.matsE = b.tab->d_matsE;
         d.matsT32 = b.tab->d_matsT32;
         d.matsbT32 = b.tab->d_matsbT32;
         d.matsI = b.tab->d_matsI;
@@ -1737,7 +1737,7 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     readback(ctx, {{ntot, d_ntrip_tot, sizeof(ntot)}, {sflags.data(), d_sflags, sizeof(int) * ni},
                    {g.data(), d_g, any_root ? sizeof(double) * nt : 0}});
     if ((ntot[1] & 0xffffffffull) != 0)
-        throw Error(-2, "tensor-core contraction: an MMA or copy completion wait exceeded its time limit");
+        throw Error(-2, "contraction: an MMA or copy completion wait exceeded its time limit");
     if (ctx->prof) {
         float ms = 0.0f;
         MWB_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));

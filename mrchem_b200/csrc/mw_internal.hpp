@@ -108,10 +108,11 @@ struct OpDepth {
     float* d_mats32 = nullptr;  // FP32 copy of d_mats (mixed-precision apply)
     double* d_matsb = nullptr;  // each matrix scaled by its term's beta (z-step operators)
     float* d_matsb32 = nullptr;
-    // FP64 matrix-instruction contraction (k_dapply): every matrix as A fragments, [step s][row tile r]
-    // [lane], lane 4 n + i holding M[8 r + n][4 s + i] (zero outside), and its term's beta
+    // FP64 matrix-instruction contraction (k_dapply), RT = row tiles of 8, S = steps of 4, zero outside 2k:
+    // every matrix as A fragments [s][r][lane 4 n + i] = M[8 r + n][4 s + i], and beta-scaled as B fragments
+    // [j][s][lane 4 n + i] = beta M[8 j + 4 (n mod 2) + n / 2][4 s + i]
     double* d_matsD = nullptr;
-    double* d_mbeta = nullptr;
+    double* d_matsE = nullptr;
     // the FP32 tables transposed and zero-padded to P x P (P = 2k rounded up to a multiple of 4), entry
     // [k][o] = M[o][k]: the layout the GEMM-tiled contraction copies into shared memory
     float* d_matsT32 = nullptr;
