@@ -6,12 +6,9 @@
 #include <map>
 #include <numeric>
 #include <string>
-#include <tuple>
-#include <unordered_map>
 
 #include "../../include/mwb200.h"
 #include "mw_kernels.cuh"
-#include "mw_slice.hpp"
 #include "mw_learned.cuh"
 
 namespace mwb {
@@ -344,76 +341,6 @@ Op::~Op() {
     cudaStreamSynchronize(c->stream);
 }
 
-struct BandTmp {
-    bool active = false;
-    int L = -1;
-    std::vector<double> ns;  // l = -L..L
-    std::vector<double> t2, x2;
-};
-
-static std::vector<BandTmp> op_bands(Op& op, int depth) {
-    const Mra& m = *op.mra;
-    const int k = m.k, K2 = 2 * k, n = m.n0 + depth;
-    long extent = 0;
-    for (int d = 0; d < 3; ++d) extent = std::max<long>(extent, (long)m.boxes[d] << depth);
-    const double cut = depth == 0 ? 0.0 : 1e-6 * op.eps * op.B0 * std::pow(4.0, -depth);
-    std::vector<BandTmp> bs(op.terms.size());
-    for (size_t mi = 0; mi < op.terms.size(); ++mi) {
-        BandTmp& b = bs[mi];
-        std::vector<std::pair<long, std::vector<double>>> cache;
-        std::vector<std::vector<double>> mats;
-        std::vector<double> t2, x2;
-        auto compute = [&](long l) {
-            std::vector<double> NS(K2 * K2);
-            op.builder->ns(op.terms[mi].alpha, n, l, NS.data(), cache);
-            double tt = 0.0, xx = 0.0;
-            for (int a = 0; a < K2; ++a)
-                for (int c = 0; c < K2; ++c) {
-                    const double v = NS[a * K2 + c] * NS[a * K2 + c];
-                    if (a < k && c < k) tt += v; else xx += v;
-                }
-            mats.push_back(std::move(NS));
-            t2.push_back(tt);
-            x2.push_back(xx);
-        };
-        compute(0);
-        compute(1);
-        const double beta = op.terms[mi].beta;
-        double S2 = std::max(t2[0] + x2[0], t2[1] + x2[1]);
-        if (depth > 0) {
-            const double xmax = std::sqrt(std::max(x2[0], x2[1]));
-            if (beta * 10.0 * xmax * S2 < cut) continue;
-        }
-        long L = 1;
-        while (L + 1 < extent) {
-            const double last = std::sqrt(t2[L] + x2[L]);
-            if (depth > 0 && beta * last * S2 < cut) break;
-            if (depth == 0 && last <= 1e-300) break;
-            if (depth == 0 && last < 1e-17 * std::sqrt(S2)) break;
-            compute(L + 1);
-            S2 = std::max(S2, t2[L + 1] + x2[L + 1]);
-            ++L;
-        }
-        while (L > 0 && depth > 0 && beta * std::sqrt(t2[L] + x2[L]) * S2 < cut) --L;
-        if (L >= extent) L = extent - 1;
-        b.active = true;
-        b.L = (int)L;
-        b.ns.assign((size_t)(2 * L + 1) * K2 * K2, 0.0);
-        b.t2.assign(2 * L + 1, 0.0);
-        b.x2.assign(2 * L + 1, 0.0);
-        for (long l = -L; l <= L; ++l) {
-            const long al = l < 0 ? -l : l;
-            double* dst = &b.ns[(size_t)(l + L) * K2 * K2];
-            const std::vector<double>& src = mats[al];
-            for (int a = 0; a < K2; ++a)
-                for (int c = 0; c < K2; ++c) dst[a * K2 + c] = (l >= 0) ? src[a * K2 + c] : src[c * K2 + a];
-            b.t2[l + L] = t2[al];
-            b.x2[l + L] = x2[al];
-        }
-    }
-    return bs;
-}
-
 static double bound3(double beta, const double* t, const double* x, bool root) {
     if (root) return beta * std::sqrt((t[0] + x[0]) * (t[1] + x[1]) * (t[2] + x[2]));
     const double v = x[0] * (t[1] + x[1]) * (t[2] + x[2]) + t[0] * x[1] * (t[2] + x[2]) + t[0] * t[1] * x[2];
@@ -424,7 +351,7 @@ static double bound3(double beta, const double* t, const double* x, bool root) {
 // along `dir` is the derivative's NS matrix for the offset and the identity along the other two
 // directions; offsets -1, 0, 1 along `dir`.  The NS matrix of offset l at scale n is
 // F [[T(2l) T(2l-1)]; [T(2l+1) T(2l)]] F^T with T(d) = 2^{n+1} T_unit(d) at the children's scale.
-static void derivative_depth(Op& op, int depth, int dir, OpDepth& od, std::vector<double>& mbeta) {
+static std::unique_ptr<OpDepth> derivative_depth(Op& op, int depth, int dir) {
     const Mra& m = *op.mra;
     const int k = m.k, K2 = 2 * k;
     const double fac = std::ldexp(1.0, m.n0 + depth + 1);
@@ -433,7 +360,7 @@ static void derivative_depth(Op& op, int depth, int dir, OpDepth& od, std::vecto
     };
     std::vector<double> ident((size_t)K2 * K2, 0.0);
     for (int a = 0; a < K2; ++a) ident[(size_t)a * K2 + a] = 1.0;
-    od.mats = ident;  // matrix 0: identity
+    std::vector<double> mats = ident;  // matrix 0: identity
     double tn[3], xn[3];
     const double ti = (double)k, xi = (double)k;  // identity: k ones in the s-s block, k elsewhere
     for (int l = -1; l <= 1; ++l) {
@@ -458,7 +385,7 @@ static void derivative_depth(Op& op, int depth, int dir, OpDepth& od, std::vecto
             }
         tn[l + 1] = t2;
         xn[l + 1] = x2;
-        od.mats.insert(od.mats.end(), NS.begin(), NS.end());  // matrix 2 + l
+        mats.insert(mats.end(), NS.begin(), NS.end());  // matrix 2 + l
     }
     const bool root = depth == 0;
     std::vector<std::pair<DeltaRec, TermRec>> rows;
@@ -483,267 +410,61 @@ static void derivative_depth(Op& op, int depth, int dir, OpDepth& od, std::vecto
         rows.emplace_back(dr, tr);
     }
     std::stable_sort(rows.begin(), rows.end(), [](const auto& a, const auto& b) { return a.first.maxb > b.first.maxb; });
+    auto od = std::make_unique<OpDepth>();
+    std::vector<DeltaRec> deltas;
+    std::vector<TermRec> terms;
     for (auto& r : rows) {
-        r.first.t0 = (int)od.terms.size();
-        od.terms.push_back(r.second);
-        r.first.t1 = (int)od.terms.size();
-        od.deltas.push_back(r.first);
+        r.first.t0 = (int)terms.size();
+        terms.push_back(r.second);
+        r.first.t1 = (int)terms.size();
+        r.first.lrank = ((r.first.d[2] + 1) << 10) | (r.first.d[1] + 1);  // line order: increasing dz, then dy
+        deltas.push_back(r.first);
+        od->maxb.push_back(r.first.maxb);
     }
-    mbeta.assign(4, 1.0);
+    Ctx* ctx = m.ctx;
+    auto up = [&](const auto& v) {
+        using T = typename std::decay<decltype(v[0])>::type;
+        T* d = (T*)dalloc(ctx, sizeof(T) * std::max<size_t>(1, v.size()));
+        upload_bytes(ctx, d, v.data(), sizeof(T) * v.size());
+        return d;
+    };
+    od->d_deltas = up(deltas);
+    od->d_terms = up(terms);
+    std::vector<int2> src;
+    for (int q = 0; q < 4; ++q) src.push_back(int2{q, 0});
+    double* d_blocks = up(mats);
+    int2* d_src = up(src);
+    double* d_beta = up(std::vector<double>(4, 1.0));
+    op_images(ctx, K2, *od, 4, d_src, d_blocks, d_beta);
+    dfree(ctx, d_blocks);
+    dfree(ctx, d_src);
+    dfree(ctx, d_beta);
+    return od;
 }
 
-// build (once) and upload the tables of one depth
+// the tables of one depth, for all operators of a batch that lack them
+static void op_require(Op** op, int n, int depth) {
+    std::vector<Op*> need;
+    for (int i = 0; i < n; ++i) {
+        if (!op[i] || op[i]->kind != 0) continue;
+        std::lock_guard<std::mutex> g(op[i]->mtx);
+        if (op[i]->depths.find(depth) == op[i]->depths.end() && std::find(need.begin(), need.end(), op[i]) == need.end())
+            need.push_back(op[i]);
+    }
+    if (need.empty()) return;
+    if (depth > 0) op_require(need.data(), (int)need.size(), 0);  // the operator scale B0
+    op_build_tables(need, depth);
+}
 static const OpDepth& op_depth(Op& op, int depth, int dir = 0) {
+    if (op.kind == 0) {
+        Op* p = &op;
+        op_require(&p, 1, depth);
+    }
     std::lock_guard<std::mutex> g(op.mtx);
     const int ckey = op.kind == 1 ? 3 * depth + dir : depth;
     auto it = op.depths.find(ckey);
-    if (it != op.depths.end()) return *it->second;
-    const Mra& m = *op.mra;
-    const int K2 = 2 * m.k;
-    auto od = std::make_unique<OpDepth>();
-    std::vector<double> mbeta;  // the term weight of every stored matrix (z-step tables)
-    if (op.kind == 1) {
-        derivative_depth(op, depth, dir, *od, mbeta);
-    } else {
-    std::vector<BandTmp> bs = op_bands(op, depth);
-    std::vector<int> base(bs.size(), -1);
-    for (size_t mi = 0; mi < bs.size(); ++mi) {
-        if (!bs[mi].active) continue;
-        base[mi] = (int)(od->mats.size() / (K2 * K2));
-        od->mats.insert(od->mats.end(), bs[mi].ns.begin(), bs[mi].ns.end());
-    }
-    const bool root = depth == 0;
-    const double cut = root ? 0.0 : 1e-6 * op.eps * op.B0 * std::pow(4.0, -depth);
-    std::map<std::tuple<int, int, int>, std::vector<std::pair<double, int>>> acc;
-    for (size_t mi = 0; mi < bs.size(); ++mi) {
-        const BandTmp& b = bs[mi];
-        if (!b.active) continue;
-        const double beta = op.terms[mi].beta;
-        double S2 = 0.0;
-        for (int i = 0; i < 2 * b.L + 1; ++i) S2 = std::max(S2, b.t2[i] + b.x2[i]);
-        for (int dx = -b.L; dx <= b.L; ++dx) {
-            const double ax = b.t2[dx + b.L] + b.x2[dx + b.L];
-            if (!root && beta * std::sqrt(ax) * S2 < cut) continue;
-            for (int dy = -b.L; dy <= b.L; ++dy) {
-                const double ay = b.t2[dy + b.L] + b.x2[dy + b.L];
-                if (!root && beta * std::sqrt(ax * ay * S2) < cut) continue;
-                for (int dz = -b.L; dz <= b.L; ++dz) {
-                    const double t[3] = {b.t2[dx + b.L], b.t2[dy + b.L], b.t2[dz + b.L]};
-                    const double x[3] = {b.x2[dx + b.L], b.x2[dy + b.L], b.x2[dz + b.L]};
-                    const double bd = bound3(beta, t, x, root);
-                    if (bd <= 0.0 || bd < cut) continue;
-                    acc[std::make_tuple(dx, dy, dz)].push_back({bd, (int)mi});
-                }
-            }
-        }
-    }
-    std::vector<std::pair<DeltaRec, std::vector<TermRec>>> rows;
-    rows.reserve(acc.size());
-    for (auto& kv : acc) {
-        auto& v = kv.second;
-        std::stable_sort(v.begin(), v.end(), [](const std::pair<double, int>& a, const std::pair<double, int>& b) {
-            return a.first > b.first || (a.first == b.first && a.second < b.second);
-        });
-        DeltaRec dr{};
-        dr.d[0] = std::get<0>(kv.first);
-        dr.d[1] = std::get<1>(kv.first);
-        dr.d[2] = std::get<2>(kv.first);
-        dr.maxb = v.front().first;
-        std::vector<TermRec> trs;
-        for (auto& pr : v) {
-            const int mi = pr.second;
-            const BandTmp& b = bs[mi];
-            TermRec tr{};
-            tr.m = mi;
-            tr.mx = base[mi] + dr.d[0] + b.L;
-            tr.my = base[mi] + dr.d[1] + b.L;
-            tr.mz = base[mi] + dr.d[2] + b.L;
-            tr.beta = op.terms[mi].beta;
-            tr.bound = pr.first;
-            trs.push_back(tr);
-        }
-        rows.emplace_back(dr, std::move(trs));
-    }
-    std::stable_sort(rows.begin(), rows.end(),
-                     [](const auto& a, const auto& b) { return a.first.maxb > b.first.maxb; });
-    for (auto& r : rows) {
-        r.first.t0 = (int)od->terms.size();
-        od->terms.insert(od->terms.end(), r.second.begin(), r.second.end());
-        r.first.t1 = (int)od->terms.size();
-        od->deltas.push_back(r.first);
-    }
-    mbeta.assign(od->mats.size() / ((size_t)K2 * K2), 0.0);
-    for (size_t mi = 0; mi < bs.size(); ++mi) {
-        if (!bs[mi].active) continue;
-        for (int q = 0; q < 2 * bs[mi].L + 1; ++q) mbeta[base[mi] + q] = op.terms[mi].beta;
-    }
-    }
-    // line ranks: the contraction groups an output node's triples by (term, dz, dy) (sort key bits:
-    // term << 20 | dz rank << 10 | dy rank), so that the triples of one line share their y and z steps
-    {
-        std::vector<int> zs, ys;
-        for (const DeltaRec& d : od->deltas) {
-            zs.push_back(d.d[2]);
-            ys.push_back(d.d[1]);
-        }
-        for (auto* v : {&zs, &ys}) {
-            std::sort(v->begin(), v->end());
-            v->erase(std::unique(v->begin(), v->end()), v->end());
-        }
-        if (zs.size() > 1024 || ys.size() > 1024)
-            throw Error(MW_ERR_CAPACITY, "operator band wider than 1024 offsets per direction");
-        for (DeltaRec& d : od->deltas) {
-            const int rz = (int)(std::lower_bound(zs.begin(), zs.end(), d.d[2]) - zs.begin());
-            const int ry = (int)(std::lower_bound(ys.begin(), ys.end(), d.d[1]) - ys.begin());
-            d.lrank = (rz << 10) | ry;
-        }
-        for (const TermRec& t : od->terms)
-            if (t.m < 0 || t.m >= 4096) throw Error(MW_ERR_CAPACITY, "more than 4096 operator terms");
-    }
-    Ctx* ctx = m.ctx;
-    cudaStream_t s = ctx->stream;
-    od->d_mats = (double*)dalloc(ctx, sizeof(double) * std::max<size_t>(1, od->mats.size()));
-    od->d_deltas = (DeltaRec*)dalloc(ctx, sizeof(DeltaRec) * std::max<size_t>(1, od->deltas.size()));
-    od->d_terms = (TermRec*)dalloc(ctx, sizeof(TermRec) * std::max<size_t>(1, od->terms.size()));
-    od->d_mats32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, od->mats.size()));
-    od->d_matsb = (double*)dalloc(ctx, sizeof(double) * std::max<size_t>(1, od->mats.size()));
-    od->d_matsb32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, od->mats.size()));
-    std::vector<float> m32(od->mats.begin(), od->mats.end());
-    std::vector<double> mb(od->mats.size());
-    for (size_t q = 0; q < od->mats.size(); ++q) mb[q] = mbeta[q / ((size_t)K2 * K2)] * od->mats[q];
-    std::vector<float> mb32(mb.begin(), mb.end());
-    // transposed, zero-padded copies for the GEMM-tiled contraction
-    const int KP = (K2 + 3) / 4 * 4;
-    const size_t nmat = od->mats.size() / ((size_t)K2 * K2);
-    std::vector<double> mT(nmat * KP * KP, 0.0), mbT(nmat * KP * KP, 0.0);
-    for (size_t mi = 0; mi < nmat; ++mi)
-        for (int o = 0; o < K2; ++o)
-            for (int k = 0; k < K2; ++k) {
-                mT[mi * KP * KP + (size_t)k * KP + o] = od->mats[mi * K2 * K2 + (size_t)o * K2 + k];
-                mbT[mi * KP * KP + (size_t)k * KP + o] = mb[mi * K2 * K2 + (size_t)o * K2 + k];
-            }
-    std::vector<float> mT32(mT.begin(), mT.end()), mbT32(mbT.begin(), mbT.end());
-    od->d_matsT32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mT.size()));
-    od->d_matsbT32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mT.size()));
-    // A and B fragments of the FP64 matrix instruction
-    const int dRT = (K2 + 7) / 8, dS = (K2 + 3) / 4;
-    std::vector<double> mD(nmat * dRT * dS * 32, 0.0), mE(nmat * dRT * dS * 32, 0.0);
-    for (size_t mi = 0; mi < nmat; ++mi)
-        for (int o = 0; o < K2; ++o)
-            for (int k = 0; k < K2; ++k) {
-                const int n = 2 * (o % 4) + (o % 8) / 4;  // B fragment column of row o
-                mD[((mi * dS + k / 4) * dRT + o / 8) * 32 + 4 * (o % 8) + k % 4] = od->mats[mi * K2 * K2 + (size_t)o * K2 + k];
-                mE[((mi * dRT + o / 8) * dS + k / 4) * 32 + 4 * n + k % 4] = mb[mi * K2 * K2 + (size_t)o * K2 + k];
-            }
-    od->d_matsD = (double*)dalloc(ctx, sizeof(double) * std::max<size_t>(1, mD.size()));
-    od->d_matsE = (double*)dalloc(ctx, sizeof(double) * std::max<size_t>(1, mE.size()));
-    if (!mD.empty()) {
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsD, mD.data(), sizeof(double) * mD.size(), cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsE, mE.data(), sizeof(double) * mE.size(), cudaMemcpyHostToDevice, s));
-    }
-    // split-TF32 images: three TF32 pieces per entry (hi, mid, lo: each the TF32 rounding of what the
-    // previous pieces leave of the FP64 value)
-    const int KP8 = (K2 + 7) / 8 * 8;
-    const size_t isz = (size_t)3 * KP8 * KP8;
-    std::vector<float> mI(nmat * isz, 0.0f), mbI(nmat * isz, 0.0f);
-    auto put3 = [&](std::vector<float>& img, size_t mi, int o, int k, double v) {
-        const size_t w = mi * isz + (size_t)(o + 3 * KP8 * (k / 4)) * 4 + k % 4;  // row o of the hi block
-        const float h = tf32_round((float)v);
-        const float md = tf32_round((float)(v - (double)h));
-        const float l = tf32_round((float)(v - (double)h - (double)md));
-        img[w] = h;
-        img[w + 4 * (size_t)KP8] = md;  // row KP8 + o
-        img[w + 8 * (size_t)KP8] = l;   // row 2 KP8 + o
-    };
-    for (size_t mi = 0; mi < nmat; ++mi)
-        for (int o = 0; o < K2; ++o)
-            for (int k = 0; k < K2; ++k) {
-                put3(mI, mi, o, k, od->mats[mi * K2 * K2 + (size_t)o * K2 + k]);
-                put3(mbI, mi, o, k, mb[mi * K2 * K2 + (size_t)o * K2 + k]);
-            }
-    od->d_matsI = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mI.size()));
-    od->d_matsbI = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mI.size()));
-    if (!mI.empty()) {
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsI, mI.data(), sizeof(float) * mI.size(), cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsbI, mbI.data(), sizeof(float) * mbI.size(), cudaMemcpyHostToDevice, s));
-    }
-    // tensor-core x step (k_happly, 2k <= 20): split-layout FP32 operators of the y/z tiles and the BF16
-    // slice images of every matrix as an x operator
-    if (K2 >= 13 && K2 <= 20) {
-        const int MT = KP / 4;
-        std::vector<float> mS(nmat * KP * KP, 0.0f), mbS(nmat * KP * KP, 0.0f);
-        for (size_t mi = 0; mi < nmat; ++mi)
-            for (int o = 0; o < K2; ++o)
-                for (int k = 0; k < K2; ++k) {
-                    const size_t w = mi * KP * KP + (size_t)k * KP + split_pos(o, MT, 4);
-                    mS[w] = (float)od->mats[mi * K2 * K2 + (size_t)o * K2 + k];
-                    mbS[w] = (float)mb[mi * K2 * K2 + (size_t)o * K2 + k];
-                }
-        const XGeo xg(K2);
-        std::vector<uint16_t> mX(nmat * (size_t)xg.OPB / 2, 0);
-        std::vector<float> sl0(K2), sl1(K2), sl2(K2), t0(K2), t1(K2), t2(K2);
-        for (size_t mi = 0; mi < nmat; ++mi) {
-            uint16_t* img = mX.data() + mi * (size_t)xg.OPB / 2;
-            for (int o = 0; o < K2; ++o) {
-                slice3_row(&od->mats[mi * K2 * K2 + (size_t)o * K2], K2, 1, sl0.data(), sl1.data(), sl2.data());
-                const float* sl[3] = {sl0.data(), sl1.data(), sl2.data()};
-                if (o < xg.W2)  // the s->s block row M[o][0 .. k)
-                    slice3_row(&od->mats[mi * K2 * K2 + (size_t)o * K2], xg.W2, 1, t0.data(), t1.data(), t2.data());
-                const float* tl[3] = {t0.data(), t1.data(), t2.data()};
-                for (int q = 0; q < 3; ++q) {  // (a) the operand of data slice q
-                    uint16_t* op = img + (size_t)q * xg.OPB_Q / 2;
-                    for (int b = q; b < 3; ++b) {
-                        const int row = b * xg.W + o;
-                        for (int k = 0; k < std::min(K2, 8 * xg.NCHM); ++k)
-                            op[((size_t)(k / 8) * xg.NBQ + row) * 8 + k % 8] = bf16_bits_exact(sl[b - q][k]);
-                        if (o < xg.W2) {
-                            const int row2 = xg.NCOL + b * xg.W2 + o;
-                            for (int k = 0; k < xg.W2; ++k)
-                                op[((size_t)(k / 8) * xg.NBQ + row2) * 8 + k % 8] = bf16_bits_exact(tl[b - q][k]);
-                        }
-                    }
-                }
-                if (xg.PACK) {  // (b) the packed step over x = 16 .. K2-1
-                    uint16_t* pk = img + (size_t)xg.OPB_A / 2;
-                    for (int b = 0; b < 3; ++b)
-                        for (int q = 0; q <= b; ++q)
-                            for (int l = 0; l < xg.LO; ++l) {
-                                const int kk = 4 * q + l, row = b * xg.W + o;
-                                pk[((size_t)(kk / 8) * xg.NCOL + row) * 8 + kk % 8] = bf16_bits_exact(sl[b - q][16 + l]);
-                            }
-                    for (int l = 0; l < xg.LO; ++l) {  // data slice 3 against operator slice 0, into block 2
-                        const int kk = 12 + l, row = 2 * xg.W + o;
-                        pk[((size_t)(kk / 8) * xg.NCOL + row) * 8 + kk % 8] = bf16_bits_exact(sl[0][16 + l]);
-                    }
-                }
-            }
-        }
-        od->d_matsS32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mS.size()));
-        od->d_matsbS32 = (float*)dalloc(ctx, sizeof(float) * std::max<size_t>(1, mS.size()));
-        od->d_matsX = (unsigned char*)dalloc(ctx, std::max<size_t>(16, mX.size() * 2));
-        if (!mS.empty()) {
-            MWB_CUDA(cudaMemcpyAsync(od->d_matsS32, mS.data(), sizeof(float) * mS.size(), cudaMemcpyHostToDevice, s));
-            MWB_CUDA(cudaMemcpyAsync(od->d_matsbS32, mbS.data(), sizeof(float) * mS.size(), cudaMemcpyHostToDevice, s));
-            MWB_CUDA(cudaMemcpyAsync(od->d_matsX, mX.data(), mX.size() * 2, cudaMemcpyHostToDevice, s));
-        }
-        MWB_CUDA(cudaStreamSynchronize(s));  // host vectors leave scope
-    }
-    if (!mT.empty()) {
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsT32, mT32.data(), sizeof(float) * mT.size(), cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsbT32, mbT32.data(), sizeof(float) * mT.size(), cudaMemcpyHostToDevice, s));
-    }
-    if (!od->mats.empty()) {
-        MWB_CUDA(cudaMemcpyAsync(od->d_mats, od->mats.data(), sizeof(double) * od->mats.size(), cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(od->d_mats32, m32.data(), sizeof(float) * m32.size(), cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsb, mb.data(), sizeof(double) * mb.size(), cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(od->d_matsb32, mb32.data(), sizeof(float) * mb32.size(), cudaMemcpyHostToDevice, s));
-    }
-    if (!od->deltas.empty())
-        MWB_CUDA(cudaMemcpyAsync(od->d_deltas, od->deltas.data(), sizeof(DeltaRec) * od->deltas.size(), cudaMemcpyHostToDevice, s));
-    if (!od->terms.empty())
-        MWB_CUDA(cudaMemcpyAsync(od->d_terms, od->terms.data(), sizeof(TermRec) * od->terms.size(), cudaMemcpyHostToDevice, s));
-    MWB_CUDA(cudaStreamSynchronize(s));
-    return *op.depths.emplace(ckey, std::move(od)).first->second;
+    if (it == op.depths.end()) it = op.depths.emplace(ckey, derivative_depth(op, depth, dir)).first;
+    return *it->second;
 }
 
 static void op_init(Op& op, Mra* m, double mu, double prec) {
@@ -759,14 +480,16 @@ static void op_init(Op& op, Mra* m, double mu, double prec) {
     r_max = std::sqrt(r_max);
     const double r_min = 0.01 * std::ldexp(root_edge, -m->max_depth);
     op.terms = kernel_expansion(mu, op.eps, r_min, r_max);
-    op.builder = std::make_unique<GaussianOperatorBuilder>(m->basis, m->F);
-    // operator scale from the root-depth bands
-    std::vector<BandTmp> b0 = op_bands(op, 0);
-    op.B0 = 0.0;
-    for (size_t mi = 0; mi < op.terms.size(); ++mi) {
-        if (!b0[mi].active) continue;
-        const int L = b0[mi].L;
-        op.B0 = std::max(op.B0, op.terms[mi].beta * std::pow(b0[mi].t2[L] + b0[mi].x2[L], 1.5));
+    if (!m->builder) {  // the construction's basis tables, with the world's first operator
+        m->builder = std::make_unique<GaussianOperatorBuilder>(m->basis, m->F);
+        auto up = [&](const std::vector<double>& v) {
+            double* d = (double*)dalloc(m->ctx, sizeof(double) * v.size());
+            upload_bytes(m->ctx, d, v.data(), sizeof(double) * v.size());
+            return d;
+        };
+        m->d_cc = up(m->builder->device_coefficients());
+        m->d_px = up(m->builder->rule_x());
+        m->d_pw = up(m->builder->rule_w());
     }
 }
 
@@ -818,6 +541,10 @@ static void apply_batched(double prec, int n, Tree** out, Op** op, Tree** inp, i
         BatchPass bp;
         bp.precision = precision;
         std::vector<int> idx;
+        std::vector<Op*> need;
+        for (int i = 0; i < n; ++i)
+            if (active[i] && out[i]->levels() > depth) need.push_back(op[i]);
+        op_require(need.data(), (int)need.size(), depth);
         for (int i = 0; i < n; ++i) {
             if (!active[i] || out[i]->levels() <= depth) continue;
             const int b = out[i]->level_begin[depth], e = out[i]->level_begin[depth + 1];
@@ -832,13 +559,13 @@ static void apply_batched(double prec, int n, Tree** out, Op** op, Tree** inp, i
             bt.g0 = g0[i];
             bt.depth = depth;
             if (depth == 0) {
-                const double nu0 = bt.tab->deltas.empty() ? 0.0 : bt.tab->deltas.front().maxb;
+                const double nu0 = bt.tab->maxb.empty() ? 0.0 : bt.tab->maxb.front();
                 bt.theta = kScreen * prec * fnorm[i] * nu0;
             } else {
                 bt.theta = kScreen * split_threshold(prec, g0[i], depth);
             }
             int np = 0;
-            while (nu_max[i] > 0.0 && np < (int)bt.tab->deltas.size() && !(bt.tab->deltas[np].maxb * nu_max[i] < bt.theta))
+            while (nu_max[i] > 0.0 && np < (int)bt.tab->maxb.size() && !(bt.tab->maxb[np] * nu_max[i] < bt.theta))
                 ++np;
             bt.nprefix = np;
             bp.trees.push_back(bt);
@@ -883,6 +610,9 @@ static long long run_entries(double prec, int precision, const std::vector<Entry
                              const std::vector<double>& g0, int dir = 0) {
     long long trip = 0;
     cudaStream_t s = out[0]->mra->ctx->stream;
+    std::map<int, std::vector<Op*>> need;
+    for (const Entry& en : ents) need[en.depth].push_back(op[en.tree]);
+    for (auto& kv : need) op_require(kv.second.data(), (int)kv.second.size(), kv.first);
     for (size_t e0 = 0; e0 < ents.size(); e0 += 128) {
         BatchPass bp;
         bp.precision = precision;
@@ -899,13 +629,13 @@ static long long run_entries(double prec, int precision, const std::vector<Entry
             bt.g0 = g0[i];
             bt.depth = en.depth;
             if (en.depth == 0) {
-                const double nu0 = bt.tab->deltas.empty() ? 0.0 : bt.tab->deltas.front().maxb;
+                const double nu0 = bt.tab->maxb.empty() ? 0.0 : bt.tab->maxb.front();
                 bt.theta = kScreen * prec * fnorm[i] * nu0;
             } else {
                 bt.theta = kScreen * split_threshold(prec, g0[i], en.depth);
             }
             int np = 0;
-            while (nu_max[i] > 0.0 && np < (int)bt.tab->deltas.size() && !(bt.tab->deltas[np].maxb * nu_max[i] < bt.theta))
+            while (nu_max[i] > 0.0 && np < (int)bt.tab->maxb.size() && !(bt.tab->maxb[np] * nu_max[i] < bt.theta))
                 ++np;
             bt.nprefix = np;
             bp.trees.push_back(bt);
@@ -958,6 +688,7 @@ static void apply_learned(double prec, int n, Tree** out, Op** op, Tree** inp, i
     {
         BatchPass bp;
         bp.precision = precision;
+        op_require(op, n, 0);
         for (const Entry& en : ents) {
             const int i = en.tree;
             BatchTree bt;
@@ -968,10 +699,10 @@ static void apply_learned(double prec, int n, Tree** out, Op** op, Tree** inp, i
             bt.oend = en.end;
             bt.prec = prec;
             bt.depth = 0;
-            const double nu0 = bt.tab->deltas.empty() ? 0.0 : bt.tab->deltas.front().maxb;
+            const double nu0 = bt.tab->maxb.empty() ? 0.0 : bt.tab->maxb.front();
             bt.theta = kScreen * prec * fnorm[i] * nu0;
             int np = 0;
-            while (nu_max[i] > 0.0 && np < (int)bt.tab->deltas.size() && !(bt.tab->deltas[np].maxb * nu_max[i] < bt.theta))
+            while (nu_max[i] > 0.0 && np < (int)bt.tab->maxb.size() && !(bt.tab->maxb[np] * nu_max[i] < bt.theta))
                 ++np;
             bt.nprefix = np;
             bp.trees.push_back(bt);
@@ -1193,6 +924,9 @@ static void mra_free(mwb::Mra* m) {
     mwb::dfree(c, m->d_FT);
     mwb::dfree(c, m->d_PF);
     mwb::dfree(c, m->d_MV);
+    mwb::dfree(c, m->d_cc);
+    mwb::dfree(c, m->d_px);
+    mwb::dfree(c, m->d_pw);
     cudaStreamSynchronize(c->stream);
     delete static_cast<mw_mra_s*>(m);
     ctx_release(c);
@@ -1855,19 +1589,19 @@ int mw_op_terms(mw_op op, double* alpha, double* beta) {
 int mw_op_scaling_matrix(mw_op op, double alpha, int n, long long l, double* T) {
     MW_TRY({
         MW_ARG(op && T, "null pointer");
-        MW_ARG(op->kind == 0 && op->builder, "not a separated-Gaussian convolution operator");
+        MW_ARG(op->kind == 0, "not a separated-Gaussian convolution operator");
         MW_ARG(alpha > 0.0, "alpha must be positive");
-        op->builder->scaling(alpha, n, (long)l, T);
+        op->mra->builder->scaling(alpha, n, (long)l, T);
     })
 }
 
 int mw_op_ns_matrix(mw_op op, int term, int n, long long l, double* NS) {
     MW_TRY({
         MW_ARG(op && NS, "null pointer");
-        MW_ARG(op->kind == 0 && op->builder, "not a separated-Gaussian convolution operator");
+        MW_ARG(op->kind == 0, "not a separated-Gaussian convolution operator");
         MW_ARG(term >= 0 && term < (int)op->terms.size(), "term index out of range");
         std::vector<std::pair<long, std::vector<double>>> cache;
-        op->builder->ns(op->terms[term].alpha, n, (long)l, NS, cache);
+        op->mra->builder->ns(op->terms[term].alpha, n, (long)l, NS, cache);
     })
 }
 

@@ -80,6 +80,12 @@ struct Mra {
     double* d_F = nullptr;   // F
     double* d_FT = nullptr;  // F^T
     double* d_PF = nullptr;  // projection matrix F * blkdiag(W, W)
+    // operator construction (GaussianOperatorBuilder): cross-correlation coefficients [c+ | c-][p][i k + j], and
+    // the Gauss-Legendre rule of the moments
+    std::unique_ptr<GaussianOperatorBuilder> builder;
+    double* d_cc = nullptr;
+    double* d_px = nullptr;
+    double* d_pw = nullptr;
     double* d_MV = nullptr;  // evaluation matrix blkdiag(E, E) * F^T (pointwise product)
     // trees and operators that point here; a destroyed world is freed with the last of them
     int refs = 0;
@@ -101,10 +107,8 @@ struct TermRec {
 };
 
 struct OpDepth {
-    std::vector<double> mats;          // NS matrices, (2k)^2 each
-    std::vector<DeltaRec> deltas;      // sorted by maxb, descending
-    std::vector<TermRec> terms;
-    double* d_mats = nullptr;
+    std::vector<double> maxb;   // the offsets' largest bounds, descending (the order of d_deltas)
+    double* d_mats = nullptr;   // NS matrices, (2k)^2 each
     float* d_mats32 = nullptr;  // FP32 copy of d_mats (mixed-precision apply)
     double* d_matsb = nullptr;  // each matrix scaled by its term's beta (z-step operators)
     float* d_matsb32 = nullptr;
@@ -141,8 +145,7 @@ struct Op {
     std::vector<double> dT[3];     // derivative unit-scale blocks T(-1), T(0), T(1), k x k
     double mu = 0.0, prec = 0.0, eps = 0.0;
     std::vector<GaussTerm> terms;
-    std::unique_ptr<GaussianOperatorBuilder> builder;
-    double B0 = 0.0;
+    double B0 = 0.0;  // operator scale, from the root depth's tables
     std::map<int, std::unique_ptr<OpDepth>> depths;
     std::mutex mtx;
     ~Op();

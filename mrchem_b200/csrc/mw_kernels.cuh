@@ -72,6 +72,10 @@ void tree_compress_bottom_up(Tree& t);
 // split the nodes of the last level whose wavelet norm exceeds thr; returns the number of new nodes
 int tree_refine_last_level(Tree& t, double thr);
 
+// operator tables (mw_optab.cu): one depth of several convolution operators, and the images of given matrices
+void op_build_tables(const std::vector<Op*>& ops, int depth);
+void op_images(Ctx* ctx, int K2, OpDepth& od, int nmat, const int2* d_src, const double* d_blocks, const double* d_beta);
+
 // one refinement pass of a batched apply (mw_apply.cu)
 struct BatchTree {
     Tree* out = nullptr;

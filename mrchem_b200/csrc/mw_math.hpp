@@ -16,18 +16,6 @@
 
 namespace mwb {
 
-// FP32 -> TF32 (10 explicit mantissa bits) rounded to nearest with ties away from zero, the rounding
-// of the device's TF32 split; infinities and NaNs pass unchanged
-inline float tf32_round(float x) {
-    uint32_t u;
-    std::memcpy(&u, &x, 4);
-    if ((u & 0x7f800000u) != 0x7f800000u) u = (u + 0x1000u) & 0xffffe000u;
-    float r;
-    std::memcpy(&r, &u, 4);
-    return r;
-}
-
-
 constexpr double kPi = 3.14159265358979323846;
 
 // Gauss-Legendre rule on [0,1], ascending nodes.
@@ -359,6 +347,19 @@ public:
             }
     }
     int k() const { return k_; }
+    // the tables of the device form: c+ and c- as [p][i k + j], one after the other, and the moments' rule
+    std::vector<double> device_coefficients() const {
+        const int K2 = 2 * k_, kk = k_ * k_;
+        std::vector<double> c((size_t)2 * K2 * kk);
+        for (int e = 0; e < kk; ++e)
+            for (int p = 0; p < K2; ++p) {
+                c[(size_t)p * kk + e] = cpos_[(size_t)e * K2 + p];
+                c[(size_t)(K2 + p) * kk + e] = cneg_[(size_t)e * K2 + p];
+            }
+        return c;
+    }
+    const std::vector<double>& rule_x() const { return px_; }
+    const std::vector<double>& rule_w() const { return pw_; }
 
 private:
     const ScalingBasis& B_;
