@@ -922,7 +922,10 @@ static void mra_free(mwb::Mra* m) {
     cudaSetDevice(c->device);
     mwb::dfree(c, m->d_F);
     mwb::dfree(c, m->d_FT);
-    mwb::dfree(c, m->d_PF);
+    mwb::dfree(c, m->d_frF);
+    mwb::dfree(c, m->d_frFT);
+    mwb::dfree(c, m->d_frPF);
+    mwb::dfree(c, m->d_frMV);
     mwb::dfree(c, m->d_MV);
     mwb::dfree(c, m->d_cc);
     mwb::dfree(c, m->d_px);
@@ -1228,10 +1231,9 @@ int mw_mra_create(mw_ctx ctx, int min_scale, const int* corner, const int* boxes
         MWB_CUDA(cudaMemcpyAsync(m->d_MV, MV.data(), sizeof(double) * K2 * K2, cudaMemcpyHostToDevice, s));
         m->d_F = (double*)dalloc(ctx, sizeof(double) * K2 * K2);
         m->d_FT = (double*)dalloc(ctx, sizeof(double) * K2 * K2);
-        m->d_PF = (double*)dalloc(ctx, sizeof(double) * K2 * K2);
         MWB_CUDA(cudaMemcpyAsync(m->d_F, m->F.data(), sizeof(double) * K2 * K2, cudaMemcpyHostToDevice, s));
         MWB_CUDA(cudaMemcpyAsync(m->d_FT, FT.data(), sizeof(double) * K2 * K2, cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(m->d_PF, PF.data(), sizeof(double) * K2 * K2, cudaMemcpyHostToDevice, s));
+        world_fragments(*m, PF, MV, FT);
         MWB_CUDA(cudaStreamSynchronize(s));
         ctx->refs++;
         *out = m;

@@ -24,6 +24,7 @@
 #include <string>
 #include <type_traits>
 
+#include "mw_block.cuh"
 #include "mw_device.cuh"
 #include "mw_kernels.cuh"
 #include "mw_tmem.cuh"
@@ -184,107 +185,45 @@ __global__ void k_bresolve_gen(int* csrc, int ncand, const uint64_t* __restrict_
 // 2. generated input nodes: reconstruct the leaf ancestor, take the child on the path, descend
 //    with zero wavelets (s_c = H_c^T s per dimension)
 // ---------------------------------------------------------------------------------------------
-// One direction of the two-scale reconstruction of a padded (2k)^3 shared block (out[o] = sum_i M[o][i]
-// in[i], as pencil_transform) restricted to what child cc needs: outputs o in [cc[DIM] k, cc[DIM] k + k)
-// only, on the pencils whose earlier directions' indices lie in the child's halves.
-template <int K, int DIM>
-__device__ static inline void child_transform(const double* __restrict__ M, double* A, const int (&cc)[3]) {
-    using G = Geo<K>;
-    constexpr int NPC = DIM == 0 ? G::K2 * G::K2 : DIM == 1 ? K * G::K2 : K * K;
-    for (int p = threadIdx.x; p < NPC; p += blockDim.x) {
-        int base, stride;
-        if (DIM == 0) {  // all (y, z)
-            base = G::P * ((p % G::K2) + G::K2 * (p / G::K2));
-            stride = 1;
-        } else if (DIM == 1) {  // x in the child's half, all z
-            base = (cc[0] * K + p % K) + G::P * G::K2 * (p / K);
-            stride = G::P;
-        } else {  // x and y in the child's halves
-            base = (cc[0] * K + p % K) + G::P * (cc[1] * K + p / K);
-            stride = G::P * G::K2;
-        }
-        double x[G::K2];
-#pragma unroll
-        for (int i = 0; i < G::K2; ++i) x[i] = A[base + i * stride];
-#pragma unroll 1
-        for (int o = cc[DIM] * K; o < cc[DIM] * K + K; ++o) {
-            double s = 0.0;
-#pragma unroll
-            for (int i = 0; i < G::K2; ++i) s = fma(M[o * G::K2 + i], x[i], s);
-            A[base + o * stride] = s;
-        }
-    }
-}
-
+// One block per node: the three directions' matrices from the leaf's block straight to the node (bx_path_operators), then
+// one separable transform on the FP64 matrix instruction, whatever the number of levels.
 template <int K>
-__global__ void __launch_bounds__(256) k_bgenerate(const uint64_t* __restrict__ ukey, const int* __restrict__ uleaf,
-                                                   const BTree* __restrict__ trees,
-                                                   const double* __restrict__ FT, double* gblk, double* gnorm2) {
-    using G = Geo<K>;
-    extern __shared__ double sm[];
-    double* A = sm;
-    double* M = A + G::VOL;
-    double* S = M + G::K2 * G::K2;
-    double* red = S + K * K * K;
+struct GenCfg {
+    using B = BX<K, K>;
+    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 3 * B::FRAG);
+    static constexpr int MINB = K <= 6 ? 4 : K <= 10 ? 2 : 1;
+};
+template <int K>
+__global__ void __launch_bounds__(BX<K, K>::NTHR, GenCfg<K>::MINB)
+    k_bgenerate(const uint64_t* __restrict__ ukey, const int* __restrict__ uleaf, const BTree* __restrict__ trees,
+                const double* __restrict__ FT, double* gblk, double* gnorm2) {
+    using B = BX<K, K>;
+    extern __shared__ __align__(16) double sm[];
+    __shared__ double red[64];
+    double* X = sm;
+    double* f = X + B::VOL;
     const int g = blockIdx.x;
     const uint64_t gkey = ukey[g];
     const BTree& T = trees[(int)(gkey >> 57)];
-    const int depth = T.depth;
     const int leaf = uleaf[g];
-    for (int i = threadIdx.x; i < G::K2 * G::K2; i += blockDim.x) M[i] = FT[i];
-    for (int e = threadIdx.x; e < G::BS; e += blockDim.x) {
-        const int a = e % G::K2, b = (e / G::K2) % G::K2, c = e / (G::K2 * G::K2);
-        A[G::at(a, b, c)] = T.in.coef[(size_t)leaf * G::BS + e];
-    }
-    long long t[3], tl[3];
+    long long t[3];
     key_trans(gkey & ((1ull << 57) - 1), t);
-    key_trans(T.inkey[leaf], tl);
-    const int dl = depth - key_depth(T.inkey[leaf]);
-    int cc[3];  // the leaf's child on the way down
-    for (int q = 0; q < 3; ++q) cc[q] = (int)((t[q] >> (dl - 1)) - 2 * tl[q]);
+    bx_path_operators<K, false>(FT, nullptr, t, T.depth - key_depth(T.inkey[leaf]), X, f);
+    bx_load<K>(X, T.in.coef + (size_t)leaf * Geo<K>::BS);
+    cp_async_wait_all();
     __syncthreads();
-    // the leaf's reconstruction restricted to child cc: each direction computes only the outputs of the
-    // child's half, over the inputs the next direction reads (same sums as the full transform)
-    child_transform<K, 0>(M, A, cc);
+    bx_slices<K, K>(X, f, f + B::FRAG);
     __syncthreads();
-    child_transform<K, 1>(M, A, cc);
-    __syncthreads();
-    child_transform<K, 2>(M, A, cc);
-    __syncthreads();
-    for (int e = threadIdx.x; e < K * K * K; e += blockDim.x) {
-        const int a = e % K, b = (e / K) % K, c = e / (K * K);
-        S[e] = A[G::at(cc[0] * K + a, cc[1] * K + b, cc[2] * K + c)];
-    }
-    __syncthreads();
-    for (int lev = dl - 2; lev >= 0; --lev) {
-        for (int dim = 0; dim < 3; ++dim) {
-            const int c = (int)((t[dim] >> lev) & 1);
-            for (int p = threadIdx.x; p < K * K; p += blockDim.x) {
-                const int u = p % K, v = p / K;
-                int bs, st;
-                if (dim == 0) { bs = K * (u + K * v); st = 1; }
-                else if (dim == 1) { bs = u + K * K * v; st = K; }
-                else { bs = u + K * v; st = K * K; }
-                double x[K];
-#pragma unroll
-                for (int i = 0; i < K; ++i) x[i] = S[bs + i * st];
-#pragma unroll 1
-                for (int o = 0; o < K; ++o) {
-                    double s = 0.0;
-#pragma unroll
-                    for (int i = 0; i < K; ++i) s = fma(M[(c * K + o) * G::K2 + i], x[i], s);
-                    S[bs + o * st] = s;
-                }
-            }
-            __syncthreads();
-        }
-    }
     double n2 = 0.0, dmy = 0.0;
-    for (int e = threadIdx.x; e < K * K * K; e += blockDim.x) {
-        const double v = S[e];
-        gblk[(size_t)g * K * K * K + e] = v;
-        n2 += v * v;
-    }
+    double* out = gblk + (size_t)g * K * K * K;
+    bx_columns<K, K>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {
+        out[n + K * K * c] = v0;
+        n2 += v0 * v0;
+        if (n + 1 < K * K) {
+            out[n + 1 + K * K * c] = v1;
+            n2 += v1 * v1;
+        }
+    });
     block_sum2(n2, dmy, red);
     if (threadIdx.x == 0) gnorm2[g] = n2;
 }
@@ -1495,11 +1434,10 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
         MWB_CUDA(cudaGetLastError());
         d_gblk = (double*)dalloc(ctx, sizeof(double) * (size_t)nu * K * K * K);
         d_gnorm2 = (double*)dalloc(ctx, sizeof(double) * nu);
-#define L_GEN(KK)                                                                                         \
-    {                                                                                                     \
-        size_t smem = sizeof(double) * (Geo<KK>::VOL + 4 * KK * KK + KK * KK * KK + 64);                 \
-        MWB_CUDA(cudaFuncSetAttribute(k_bgenerate<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        k_bgenerate<KK><<<nu, 256, smem, s>>>(d_ukey, d_uleaf, d_trees, m.d_FT, d_gblk, d_gnorm2);            \
+#define L_GEN(KK)                                                                                                        \
+    {                                                                                                                    \
+        MWB_CUDA(cudaFuncSetAttribute(k_bgenerate<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GenCfg<KK>::SMEM)); \
+        k_bgenerate<KK><<<nu, BX<KK, KK>::NTHR, GenCfg<KK>::SMEM, s>>>(d_ukey, d_uleaf, d_trees, m.d_FT, d_gblk, d_gnorm2); \
     }
         MWB_DISPATCH_K(K, L_GEN)
 #undef L_GEN

@@ -40,18 +40,6 @@
 
 namespace mwb {
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-        : "+d"(c[0]), "+d"(c[1])
-        : "d"(a), "d"(b));
-}
-
-// smallest n >= v with n mod 16 in {4, 12}: rows of doubles on four distinct groups of four banks
-__host__ __device__ constexpr int dcfg_ld(int v) {
-    while (v % 16 != 4 && v % 16 != 12) ++v;
-    return v;
-}
-
 template <int K>
 struct DCfg {
     static constexpr int K2 = 2 * K;

@@ -1,5 +1,5 @@
 // mw_device.cuh -- device helpers shared by the kernels: Morton node keys, the open-addressing hash
-// index, block geometry of a node, block reductions and the in-place pencil transform.
+// index, block geometry of a node, asynchronous copies, block reductions and the FP64 matrix instruction.
 #pragma once
 #include <cstdint>
 
@@ -68,11 +68,7 @@ __device__ static inline int hlookup(const uint64_t* hk, const int* hv, uint32_t
 template <int K>
 struct Geo {
     static constexpr int K2 = 2 * K;
-    static constexpr int P = K2 + 1;
-    static constexpr int VOL = P * K2 * K2;
-    static constexpr int NP = K2 * K2;
     static constexpr int BS = K2 * K2 * K2;
-    __device__ static inline int at(int a, int b, int c) { return a + P * (b + K2 * c); }
 };
 
 // 16-byte asynchronous global -> shared copies (cp.async, L2 only), their commit and completion
@@ -121,28 +117,18 @@ __device__ static inline void block_sum2(double& a, double& b, double* red) {
     }
 }
 
-// in-place 1-D transform of all pencils along DIM of a padded (2k)^3 shared tensor by the
-// K2 x K2 shared matrix M (out[o] = sum_i M[o][i] in[i])
-template <int K, int DIM>
-__device__ static inline void pencil_transform(const double* __restrict__ M, double* A) {
-    using G = Geo<K>;
-    for (int p = threadIdx.x; p < G::NP; p += blockDim.x) {
-        const int u = p % G::K2, v = p / G::K2;
-        int base, stride;
-        if (DIM == 0) { base = G::P * (u + G::K2 * v); stride = 1; }
-        else if (DIM == 1) { base = u + G::P * G::K2 * v; stride = G::P; }
-        else { base = u + G::P * v; stride = G::P * G::K2; }
-        double x[G::K2];
-#pragma unroll
-        for (int i = 0; i < G::K2; ++i) x[i] = A[base + i * stride];
-#pragma unroll 1
-        for (int o = 0; o < G::K2; ++o) {
-            double s = 0.0;
-#pragma unroll
-            for (int i = 0; i < G::K2; ++i) s = fma(M[o * G::K2 + i], x[i], s);
-            A[base + o * stride] = s;
-        }
-    }
+// FP64 matrix instruction m8n8k4: lane 4 n + i holds A[n][i], B[i][n] and C[n][2 i], C[n][2 i + 1]
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    // volatile: the whole warp executes it together, so it may not be sunk into a branch that uses its result
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+// smallest n >= v with n mod 16 in {4, 12}: rows of doubles on four distinct groups of four banks
+__host__ __device__ constexpr int dcfg_ld(int v) {
+    while (v % 16 != 4 && v % 16 != 12) ++v;
+    return v;
 }
 
 }  // namespace mwb

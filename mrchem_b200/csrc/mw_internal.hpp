@@ -77,9 +77,11 @@ struct Mra {
     ScalingBasis basis;
     std::vector<double> F;  // (2k)^2 two-scale filter
     std::vector<double> W;  // k x k projection quadrature matrix
-    double* d_F = nullptr;   // F
+    double* d_F = nullptr;   // two-scale filter
     double* d_FT = nullptr;  // F^T
-    double* d_PF = nullptr;  // projection matrix F * blkdiag(W, W)
+    // F, F^T, PF and MV as fragments of the block transform (mw_block.cuh), A then B order, each 2 x fr_n doubles
+    double *d_frF = nullptr, *d_frFT = nullptr, *d_frPF = nullptr, *d_frMV = nullptr;
+    int fr_n = 0;
     // operator construction (GaussianOperatorBuilder): cross-correlation coefficients [c+ | c-][p][i k + j], and
     // the Gauss-Legendre rule of the moments
     std::unique_ptr<GaussianOperatorBuilder> builder;

@@ -2,14 +2,14 @@
 // bookkeeping (Morton keys, hash index, splits), candidate screening, generated input nodes and the
 // FP64 non-standard-form contraction.
 //
-// Node blocks are (2k)^3 FP64 tensors, x fastest.  In shared memory a block is stored with the
-// x-pencil stride padded to 2k+1 (odd), so that pencils along every dimension are read without bank
-// conflicts; each thread owns whole pencils, which makes every 1-D transform safe in place.
+// Node blocks are (2k)^3 FP64 tensors, x fastest; a node's transforms run on the FP64 matrix instruction, in place in
+// shared memory (mw_block.cuh).
 #include <cub/cub.cuh>
 
 #include <algorithm>
 #include <cstdio>
 
+#include "mw_block.cuh"
 #include "mw_device.cuh"
 #include "mw_kernels.cuh"
 
@@ -130,19 +130,27 @@ struct WorldGeo {
     double qx[16]; // quadrature nodes on [0,1]
 };
 
-constexpr int kTransformThreads = 256;
-
-// one node of a transform (the whole block); leaves must have been filtered out by the caller in
-// the compress / sum-up modes
 template <int K>
-__device__ __forceinline__ void transform_node(int mode, int node, const TView& t, const double* __restrict__ Mg,
+struct TrCfg {
+    using B = BX<K, 2 * K>;
+    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 2 * B::FRAG);
+    static constexpr int MINB = K <= 6 ? 4 : K <= 10 ? 2 : 1;  // blocks per SM (registers and shared memory)
+};
+
+// One node of a transform (the whole block); leaves must have been filtered out by the caller in the compress /
+// sum-up modes.  fr: the operator's fragments.  HBM- and FP64-bound in like parts (k = 10: 128 KB of traffic and 18,000 cycles
+// of products per node and SM); with a thread per pencil the level of 16 trees took twice as long.
+template <int K>
+__device__ __forceinline__ void transform_node(int mode, int node, const TView& t, const double* __restrict__ fr,
                                                const FuncDesc& f, const WorldGeo& wg) {
-    using G = Geo<K>;
-    extern __shared__ double sm[];
-    double* A = sm;
-    double* M = A + G::VOL;
-    double* red = M + G::K2 * G::K2;
-    for (int i = threadIdx.x; i < G::K2 * G::K2; i += blockDim.x) M[i] = Mg[i];
+    using B = BX<K, 2 * K>;
+    constexpr int K2 = 2 * K, BS = Geo<K>::BS;
+    extern __shared__ __align__(16) double sm[];
+    __shared__ double red[64];
+    double* X = sm;
+    double* fo = X + B::VOL;
+    bx_operator(fo, fr, 2 * B::FRAG, B::NTHR);
+    auto at = [](int a, int b, int c) { return a + B::LDA * b + B::LDP * c; };
     double fac = 1.0;
     if (mode == TM_PROJECT) {
         long long tr[3];
@@ -151,55 +159,55 @@ __device__ __forceinline__ void transform_node(int mode, int node, const TView& 
         const int n1 = wg.n0 + key_depth(key) + 1;
         const double h = ldexp(1.0, -n1);
         fac = pow(2.0, -1.5 * n1);
-        for (int e = threadIdx.x; e < G::BS; e += blockDim.x) {
-            const int a = e % G::K2, b = (e / G::K2) % G::K2, c = e / (G::K2 * G::K2);
+        for (int e = threadIdx.x; e < BS; e += B::NTHR) {
+            const int a = e % K2, b = (e / K2) % K2, c = e / (K2 * K2);
             const double x = wg.lo[0] + (2 * tr[0] + a / K + wg.qx[a % K]) * h;
             const double y = wg.lo[1] + (2 * tr[1] + b / K + wg.qx[b % K]) * h;
             const double z = wg.lo[2] + (2 * tr[2] + c / K + wg.qx[c % K]) * h;
-            A[G::at(a, b, c)] = eval_func(f, x, y, z);
+            X[at(a, b, c)] = eval_func(f, x, y, z);
         }
     } else if (mode == TM_COMPRESS) {
         const int c0 = t.child0[node];
-        for (int e = threadIdx.x; e < G::BS; e += blockDim.x) {
-            const int a = e % G::K2, b = (e / G::K2) % G::K2, c = e / (G::K2 * G::K2);
+        // the children's scaling rows; element pairs by asynchronous copies where a pair never straddles children
+        constexpr int W = K % 2 == 0 ? 2 : 1;
+        for (int e = threadIdx.x; e < BS / W; e += B::NTHR) {
+            const int a = W * (e % (K2 / W)), b = (e / (K2 / W)) % K2, c = e / (K2 / W * K2);
             const int ch = (a / K) + 2 * (b / K) + 4 * (c / K);
-            A[G::at(a, b, c)] =
-                t.coef[(size_t)(c0 + ch) * G::BS + (a % K) + G::K2 * ((b % K) + G::K2 * (c % K))];
+            const double* src = t.coef + (size_t)(c0 + ch) * BS + (a % K) + K2 * ((b % K) + K2 * (c % K));
+            if constexpr (W == 2) cp_async16(X + at(a, b, c), src);
+            else X[at(a, b, c)] = *src;
         }
     } else {
-        for (int e = threadIdx.x; e < G::BS; e += blockDim.x) {
-            const int a = e % G::K2, b = (e / G::K2) % G::K2, c = e / (G::K2 * G::K2);
-            A[G::at(a, b, c)] = t.coef[(size_t)node * G::BS + e];
-        }
+        bx_load<K>(X, t.coef + (size_t)node * BS);
     }
+    cp_async_wait_all();
     __syncthreads();
-    pencil_transform<K, 0>(M, A);
-    __syncthreads();
-    pencil_transform<K, 1>(M, A);
+    bx_slices<K, 2 * K>(X, fo, fo + B::FRAG);
     __syncthreads();
     double n2 = 0.0, w2 = 0.0;
     const int c0 = (mode == TM_SUMUP) ? t.child0[node] : 0;
-    for (int p = threadIdx.x; p < G::NP; p += blockDim.x) {
-        const int a = p % G::K2, b = p / G::K2;
-        double x[G::K2];
-#pragma unroll
-        for (int i = 0; i < G::K2; ++i) x[i] = A[G::at(a, b, i)];
-#pragma unroll 1
-        for (int o = 0; o < G::K2; ++o) {
-            double s = 0.0;
-#pragma unroll
-            for (int i = 0; i < G::K2; ++i) s = fma(M[o * G::K2 + i], x[i], s);
-            if (mode == TM_SUMUP) {
-                const int ch = (a / K) + 2 * (b / K) + 4 * (o / K);
-                t.coef[(size_t)(c0 + ch) * G::BS + (a % K) + G::K2 * ((b % K) + G::K2 * (o % K))] += s;
+    bx_columns<K, 2 * K>(X, fo, [&](int c, int n, double v0, double v1) {
+        const int a = n % K2, b = n / K2;
+        if (mode == TM_SUMUP) {
+            const int ch = 2 * (b / K) + 4 * (c / K), in = K2 * ((b % K) + K2 * (c % K));
+            if constexpr (K % 2 == 0) {
+                double2* p = reinterpret_cast<double2*>(t.coef + (size_t)(c0 + ch + a / K) * BS + a % K + in);
+                const double2 o = *p;
+                *p = make_double2(o.x + v0, o.y + v1);
             } else {
-                s *= fac;
-                t.coef[(size_t)node * G::BS + a + G::K2 * (b + G::K2 * o)] = s;
-                n2 += s * s;
-                if (!(a < K && b < K && o < K)) w2 += s * s;
+                t.coef[(size_t)(c0 + ch + a / K) * BS + a % K + in] += v0;
+                t.coef[(size_t)(c0 + ch + (a + 1) / K) * BS + (a + 1) % K + in] += v1;
             }
+        } else {
+            v0 *= fac;
+            v1 *= fac;
+            *reinterpret_cast<double2*>(t.coef + (size_t)node * BS + n + K2 * K2 * c) = make_double2(v0, v1);
+            n2 += v0 * v0 + v1 * v1;
+            const bool sc = b < K && c < K;
+            if (!(sc && a < K)) w2 += v0 * v0;
+            if (!(sc && a + 1 < K)) w2 += v1 * v1;
         }
-    }
+    });
     if (mode != TM_SUMUP) {
         block_sum2(n2, w2, red);
         if (threadIdx.x == 0) {
@@ -210,25 +218,23 @@ __device__ __forceinline__ void transform_node(int mode, int node, const TView& 
 }
 
 template <int K>
-__global__ void __launch_bounds__(kTransformThreads) k_transform(int mode, const int* __restrict__ nodes, int begin,
-                                                                 TView t, const double* __restrict__ Mg, FuncDesc f,
-                                                                 WorldGeo wg) {
+__global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, TrCfg<K>::MINB)
+    k_transform(int mode, const int* __restrict__ nodes, int begin, TView t, const double* __restrict__ fr, FuncDesc f, WorldGeo wg) {
     // node list, or (nodes == nullptr) the range begin + blockIdx.x, where leaves have nothing to do
     // for the compress / sum-up modes (the whole block leaves together, before any barrier)
     const int node = nodes ? nodes[blockIdx.x] : begin + blockIdx.x;
     if (!nodes && mode != TM_PROJECT && t.child0[node] < 0) return;
-    transform_node<K>(mode, node, t, Mg, f, wg);
+    transform_node<K>(mode, node, t, fr, f, wg);
 }
 
 // compress / sum-up of the internal nodes of one level of several trees: items (tree, node)
 template <int K>
-__global__ void __launch_bounds__(kTransformThreads) k_transform_multi(int mode, const int2* __restrict__ items,
-                                                                       const TView* __restrict__ views,
-                                                                       const double* __restrict__ Mg, WorldGeo wg) {
+__global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, TrCfg<K>::MINB)
+    k_transform_multi(int mode, const int2* __restrict__ items, const TView* __restrict__ views, const double* __restrict__ fr, WorldGeo wg) {
     const int2 it = items[blockIdx.x];
     const TView t = views[it.x];
     if (t.child0[it.y] < 0) return;
-    transform_node<K>(mode, it.y, t, Mg, FuncDesc{0, 0, nullptr}, wg);
+    transform_node<K>(mode, it.y, t, fr, FuncDesc{0, 0, nullptr}, wg);
 }
 
 // one warp per (tree, node) item: squared norm of the block and of its wavelet part
@@ -489,20 +495,46 @@ static WorldGeo world_geo(const Mra& m) {
     return g;
 }
 
+void world_fragments(Mra& m, const std::vector<double>& PF, const std::vector<double>& MV, const std::vector<double>& FT) {
+    auto image = [&](const std::vector<double>& M) {
+        std::vector<double> f;
+#define L_FR(KK)                                                                            \
+    {                                                                                       \
+        constexpr int N = BX<KK, 2 * KK>::FRAG, W = 2 * KK;                                  \
+        f.resize(2 * N);                                                                     \
+        auto entry = [&](int o, int i) { return M[(size_t)o * W + i]; };                     \
+        for (int e = 0; e < N; ++e) {                                                        \
+            f[e] = bx_frag_a<KK, 2 * KK>(e, entry);                                          \
+            f[N + e] = bx_frag_b<KK, 2 * KK>(e, entry);                                      \
+        }                                                                                    \
+    }
+        MWB_DISPATCH_K(m.k, L_FR)
+#undef L_FR
+        m.fr_n = (int)f.size() / 2;
+        double* d = (double*)dalloc(m.ctx, sizeof(double) * f.size());
+        MWB_CUDA(cudaMemcpyAsync(d, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice, m.ctx->stream));
+        MWB_CUDA(cudaStreamSynchronize(m.ctx->stream));  // f leaves scope
+        return d;
+    };
+    m.d_frF = image(m.F);
+    m.d_frFT = image(FT);
+    m.d_frPF = image(PF);
+    m.d_frMV = image(MV);
+}
+
 void launch_transform_nodes(Tree& t, int mode, const int* d_nodes, int nnodes, const FuncDesc* f, cudaStream_t s,
                             int begin) {
     if (nnodes <= 0) return;
     const Mra& m = *t.mra;
-    const double* M = (mode == TM_PROJECT) ? m.d_PF : (mode == TM_COMPRESS ? m.d_F : m.d_FT);
+    const double* fr = (mode == TM_PROJECT) ? m.d_frPF : (mode == TM_COMPRESS ? m.d_frF : m.d_frFT);
     FuncDesc fd = f ? *f : FuncDesc{0, 0, nullptr};
     WorldGeo wg = world_geo(m);
     TView tv = view(t);
-#define L_TR(KK)                                                                                      \
-    {                                                                                                 \
-        size_t smem = sizeof(double) * (Geo<KK>::VOL + 4 * KK * KK + 64);                            \
-        MWB_CUDA(cudaFuncSetAttribute(k_transform<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                      (int)smem));                                                    \
-        k_transform<KK><<<nnodes, kTransformThreads, smem, s>>>(mode, d_nodes, begin, tv, M, fd, wg);   \
+#define L_TR(KK)                                                                                              \
+    {                                                                                                         \
+        MWB_CUDA(cudaFuncSetAttribute(k_transform<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
+                                      (int)TrCfg<KK>::SMEM));                                                 \
+        k_transform<KK><<<nnodes, BX<KK, 2 * KK>::NTHR, TrCfg<KK>::SMEM, s>>>(mode, d_nodes, begin, tv, fr, fd, wg); \
     }
     MWB_DISPATCH_K(m.k, L_TR)
 #undef L_TR
@@ -539,13 +571,12 @@ void trees_finish(const std::vector<Tree*>& ts, bool sumup, bool compress, bool 
     auto level = [&](int mode, int d) {
         const int n = lvl_off[d + 1] - lvl_off[d];
         if (n <= 0) return;
-        const double* M = mode == TM_COMPRESS ? m.d_F : m.d_FT;
+        const double* fr = mode == TM_COMPRESS ? m.d_frF : m.d_frFT;
 #define L_TRM(KK)                                                                                          \
     {                                                                                                      \
-        size_t smem = sizeof(double) * (Geo<KK>::VOL + 4 * KK * KK + 64);                                 \
         MWB_CUDA(cudaFuncSetAttribute(k_transform_multi<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                      (int)smem));                                                         \
-        k_transform_multi<KK><<<n, kTransformThreads, smem, s>>>(mode, d_items + lvl_off[d], d_views, M, wg); \
+                                      (int)TrCfg<KK>::SMEM));                                              \
+        k_transform_multi<KK><<<n, BX<KK, 2 * KK>::NTHR, TrCfg<KK>::SMEM, s>>>(mode, d_items + lvl_off[d], d_views, fr, wg); \
     }
         MWB_DISPATCH_K(m.k, L_TRM)
 #undef L_TRM

@@ -72,6 +72,9 @@ void tree_compress_bottom_up(Tree& t);
 // split the nodes of the last level whose wavelet norm exceeds thr; returns the number of new nodes
 int tree_refine_last_level(Tree& t, double thr);
 
+// fragment images of the world's block transforms (mw_kernels.cu); row-major matrices
+void world_fragments(Mra& m, const std::vector<double>& PF, const std::vector<double>& MV, const std::vector<double>& FT);
+
 // operator tables (mw_optab.cu): one depth of several convolution operators, and the images of given matrices
 void op_build_tables(const std::vector<Op*>& ops, int depth);
 void op_images(Ctx* ctx, int K2, OpDepth& od, int nmat, const int2* d_src, const double* d_blocks, const double* d_beta);

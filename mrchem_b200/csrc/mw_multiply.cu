@@ -24,7 +24,9 @@
 #include <vector>
 
 #include "../../include/mwb200.h"
+#include "mw_block.cuh"
 #include "mw_device.cuh"
+#include "mw_umma.cuh"
 #include "mw_kernels.cuh"
 #include "mw_learned.cuh"
 
@@ -53,149 +55,136 @@ struct MulItem {
     int node;
 };
 
-constexpr int kMulThreads = 416;  // 13 warps: one pencil of a (2k)^3 block per thread at k = 10
-
 template <int K>
 struct MulCfg {
-    using G = Geo<K>;
-    static constexpr int K2 = 2 * K;
-    static constexpr int KKK = K * K * K;
-    static constexpr int PER = (KKK + kMulThreads - 1) / kMulThreads;  // octant values per thread
-    static constexpr size_t SMEM = sizeof(double) * (2 * (size_t)G::VOL + 3 * K2 * K2 + 64) + 16;
-    static constexpr bool FITS = SMEM <= 227 * 1024;
+    using B = BX<K, 2 * K>;
+    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 5 * B::FRAG);
+    static constexpr int MINB = K <= 6 ? 4 : K <= 10 ? 2 : 1;
+    // the first factor's point values wait in tensor memory: 4 RT doubles per lane and couple of column tiles
+    static constexpr int NIT = (B::NZT + 2 * B::NWARP - 1) / (2 * B::NWARP), WORDS = 8 * B::RT;
+    static constexpr int TNEED = (B::NWARP + 3) / 4 * NIT * WORDS;
+    static constexpr int TCOLS = TNEED <= 32 ? 32 : TNEED <= 64 ? 64 : TNEED <= 128 ? 128 : 256;
+    static_assert(TNEED <= 256 && MINB * TCOLS <= 512, "tensor memory");
 };
 
-// Block of a factor at node `key` into the padded tensor T: the node's own compressed block, or the
-// scaling-only block generated below the deepest existing ancestor.  `slot` is a shared int.
+// One output node per block.  Per factor: its block (own, or the deepest ancestor's with the path's operators) to the
+// point values in one separable transform; the product goes back through PF.  FP64-bound: 9 mode products per node on
+// the matrix instruction (16 us per node and SM at k = 10), two blocks per SM so that one's loads and barriers hide behind
+// the other's products.  28 pairs at k = 10: 15.5 ms with a thread per pencil and a reconstruction per level of a
+// missing node.
 template <int K>
-__device__ void mul_fetch(double* T, const double* FT, const uint64_t* hk, const int* hv, uint32_t hcap,
-                          const double* coef, uint64_t key, int* slot) {
-    using G = Geo<K>;
+__global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, MulCfg<K>::MINB)
+    k_mul(const MulItem* __restrict__ items, const MulTree* __restrict__ trees, const double* __restrict__ MVg,
+          const double* __restrict__ frMV, const double* __restrict__ frPF, const double* __restrict__ FTg, int n0) {
+    using B = BX<K, 2 * K>;
     using C = MulCfg<K>;
-    const int depth = key_depth(key);
-    long long tr[3];
-    key_trans(key, tr);
-    if (threadIdx.x == 0) {
-        int idx = hlookup(hk, hv, hcap, key), da = depth;
-        while (idx < 0 && da > 0) {
-            --da;
-            const int sh = depth - da;
-            idx = hlookup(hk, hv, hcap, make_key(da, tr[0] >> sh, tr[1] >> sh, tr[2] >> sh));
-        }
-        slot[0] = idx;
-        slot[1] = da;
-    }
-    __syncthreads();
-    const int idx = slot[0], da = slot[1];
-    if (idx < 0) {  // outside the factor's roots (cannot happen on one world): zero
-        for (int e = threadIdx.x; e < G::VOL; e += blockDim.x) T[e] = 0.0;
-        return;
-    }
-    const double* blk = coef + (size_t)idx * G::BS;
-    for (int e = threadIdx.x; e < G::BS; e += blockDim.x) {
-        const int a = e % G::K2, b = (e / G::K2) % G::K2, c = e / (G::K2 * G::K2);
-        T[G::at(a, b, c)] = blk[e];
-    }
-    for (int lev = da; lev < depth; ++lev) {
-        // reconstruct to the children's scaling parts, keep the child on the path (zero wavelets)
-        __syncthreads();
-        pencil_transform<K, 0>(FT, T);
-        __syncthreads();
-        pencil_transform<K, 1>(FT, T);
-        __syncthreads();
-        pencil_transform<K, 2>(FT, T);
-        __syncthreads();
-        const int sh = depth - lev - 1;
-        const int cx = (int)((tr[0] >> sh) & 1), cy = (int)((tr[1] >> sh) & 1), cz = (int)((tr[2] >> sh) & 1);
-        double v[C::PER];
-#pragma unroll
-        for (int r = 0; r < C::PER; ++r) {
-            const int e = threadIdx.x + r * kMulThreads;
-            v[r] = 0.0;
-            if (e < C::KKK) {
-                const int x = e % K, y = (e / K) % K, z = e / (K * K);
-                v[r] = T[G::at(cx * K + x, cy * K + y, cz * K + z)];
-            }
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < G::VOL; e += blockDim.x) T[e] = 0.0;
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < C::PER; ++r) {
-            const int e = threadIdx.x + r * kMulThreads;
-            if (e < C::KKK) {
-                const int x = e % K, y = (e / K) % K, z = e / (K * K);
-                T[G::at(x, y, z)] = v[r];
-            }
-        }
-    }
-}
-
-template <int K>
-__global__ void __launch_bounds__(kMulThreads) k_mul(const MulItem* __restrict__ items, const MulTree* __restrict__ trees,
-                                                     const double* __restrict__ MVg, const double* __restrict__ PFg,
-                                                     const double* __restrict__ FTg, int n0) {
-    using G = Geo<K>;
-    constexpr int K2 = G::K2;
+    constexpr int K2 = 2 * K, BS = Geo<K>::BS, RT = B::RT;
     extern __shared__ __align__(16) double msm[];
-    double* TA = msm;
-    double* TB = TA + G::VOL;
-    double* MV = TB + G::VOL;
-    double* PF = MV + K2 * K2;
-    double* FT = PF + K2 * K2;
-    double* red = FT + K2 * K2;
-    int* slot = reinterpret_cast<int*>(red + 64);
+    __shared__ double red[64];
+    __shared__ int found[2][2];
+    __shared__ uint32_t tmem_slot;
+    double* X = msm;
+    double* fq = X + B::VOL;         // the factor's operators (A, B, A order)
+    double* fp = fq + 3 * B::FRAG;   // PF (A, B order)
     const MulItem it = items[blockIdx.x];
     const MulTree& T = trees[it.tree];
-    for (int i = threadIdx.x; i < K2 * K2; i += blockDim.x) {
-        MV[i] = MVg[i];
-        PF[i] = PFg[i];
-        FT[i] = FTg[i];
-    }
     const uint64_t key = T.okey[it.node];
-    __syncthreads();
-    mul_fetch<K>(TA, FT, T.ahk, T.ahv, T.ahcap, T.acoef, key, slot);
-    __syncthreads();
-    mul_fetch<K>(TB, FT, T.bhk, T.bhv, T.bhcap, T.bcoef, key, slot);
-    __syncthreads();
-    // values of both factors at the children's quadrature points
-    pencil_transform<K, 0>(MV, TA);
-    pencil_transform<K, 0>(MV, TB);
-    __syncthreads();
-    pencil_transform<K, 1>(MV, TA);
-    pencil_transform<K, 1>(MV, TB);
-    __syncthreads();
-    pencil_transform<K, 2>(MV, TA);
-    pencil_transform<K, 2>(MV, TB);
-    __syncthreads();
-    for (int e = threadIdx.x; e < G::VOL; e += blockDim.x) TA[e] *= TB[e];
-    __syncthreads();
-    pencil_transform<K, 0>(PF, TA);
-    __syncthreads();
-    pencil_transform<K, 1>(PF, TA);
-    __syncthreads();
-    // last dimension in registers, scaled, written with the block norms
-    const double fac = T.c * exp2(1.5 * (double)(n0 + key_depth(key) + 1));
-    double* dst = T.ocoef + (size_t)it.node * G::BS;
-    double n2 = 0.0, w2 = 0.0;
-    for (int p = threadIdx.x; p < G::NP; p += blockDim.x) {
-        const int a = p % K2, b = p / K2;
-        double x[K2];
-#pragma unroll
-        for (int i = 0; i < K2; ++i) x[i] = TA[G::at(a, b, i)];
-#pragma unroll 1
-        for (int o = 0; o < K2; ++o) {
-            double s = 0.0;
-#pragma unroll
-            for (int i = 0; i < K2; ++i) s = fma(PF[o * K2 + i], x[i], s);
-            s *= fac;
-            dst[a + K2 * (b + K2 * o)] = s;
-            n2 += s * s;
-            if (!(a < K && b < K && o < K)) w2 += s * s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, depth = key_depth(key);
+    long long tr[3];
+    key_trans(key, tr);
+    bx_operator(fp, frPF, 2 * B::FRAG, B::NTHR);
+    if (warp < 2) {
+        int idx, da;
+        if (warp == 0) bx_lookup(T.ahk, T.ahv, T.ahcap, key, idx, da);
+        else bx_lookup(T.bhk, T.bhv, T.bhcap, key, idx, da);
+        if (lane == 0) {
+            found[warp][0] = idx;
+            found[warp][1] = da;
         }
     }
+    if (warp == 2) {
+        tmem_alloc(&tmem_slot, C::TCOLS);
+        tmem_relinquish();
+    }
+    tmem_fence_before_sync();
+    __syncthreads();
+    tmem_fence_after_sync();
+    const uint32_t stash = tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((warp >> 2) * C::NIT * C::WORDS);
+    // values of the factors at the children's quadrature points; a square takes its one factor once
+    const bool sq = T.acoef == T.bcoef;
+    for (int q = sq ? 1 : 0; q < 2; ++q) {
+        const int idx = found[q][0], da = found[q][1];
+        const double* coef = q ? T.bcoef : T.acoef;
+        if (idx >= 0) {
+            if (da == depth) {
+                bx_operator(fq, frMV, 2 * B::FRAG, B::NTHR);
+                bx_operator(fq + 2 * B::FRAG, frMV, B::FRAG, B::NTHR);
+            } else {
+                bx_path_operators<K, true>(FTg, MVg, tr, depth - da, X, fq);
+            }
+            bx_load<K>(X, coef + (size_t)idx * BS);
+        } else {  // outside the factor's roots (cannot happen on one world): zero
+            for (int e = tid; e < B::VOL; e += B::NTHR) X[e] = 0.0;
+            for (int e = tid; e < 3 * B::FRAG; e += B::NTHR) fq[e] = 0.0;
+        }
+        cp_async_wait_all();
+        __syncthreads();
+        bx_slices<K, K2>(X, fq, fq + B::FRAG);
+        __syncthreads();
+#pragma unroll 1
+        for (int i = 0; i < C::NIT; ++i) {
+            const int t0 = warp + 2 * B::NWARP * i;
+            double v[2][RT][2];
+            bx_z<K, K2, 2>(X, t0, B::NWARP, fq + 2 * B::FRAG, v);
+            uint32_t w[C::WORDS];
+            if (q == 0) {
+#pragma unroll
+                for (int e = 0; e < 4 * RT; ++e) double_to_words(v[e / (2 * RT)][(e / 2) % RT][e % 2], w[2 * e], w[2 * e + 1]);
+                tmem_span_st<0, C::WORDS>(stash + i * C::WORDS, w);
+                continue;
+            }
+            if (!sq) {
+                tmem_span_ld<0, C::WORDS>(stash + i * C::WORDS, w);
+                tmem_span_wait<0, C::WORDS>(w);
+            }
+            __syncwarp();  // the columns are read
+#pragma unroll
+            for (int e = 0; e < 4 * RT; e += 2) {  // the product, in the place of the second factor's columns
+                const int h = e / (2 * RT), r = (e / 2) % RT;
+                const int c = 8 * r + (lane >> 2), tile = t0 + h * B::NWARP, n = 8 * tile + 2 * (lane & 3);
+                const double a0 = sq ? v[h][r][0] : words_to_double(w[2 * e], w[2 * e + 1]);
+                const double a1 = sq ? v[h][r][1] : words_to_double(w[2 * e + 2], w[2 * e + 3]);
+                if (c < K2 && n < K2 * K2) {
+                    double* p = X + c * B::LDP + B::physo(n);
+                    p[0] = a0 * v[h][r][0];
+                    p[1] = a1 * v[h][r][1];
+                }
+            }
+        }
+        tmem_wait_st();
+        __syncthreads();
+    }
+    bx_slices<K, K2>(X, fp, fp + B::FRAG);
+    __syncthreads();
+    const double fac = T.c * exp2(1.5 * (double)(n0 + depth + 1));
+    double* dst = T.ocoef + (size_t)it.node * BS;
+    double n2 = 0.0, w2 = 0.0;
+    bx_columns<K, K2>(X, fp, [&](int c, int n, double v0, double v1) {
+        const int a = n % K2, b = n / K2;
+        v0 *= fac;
+        v1 *= fac;
+        *reinterpret_cast<double2*>(dst + n + K2 * K2 * c) = make_double2(v0, v1);
+        n2 += v0 * v0 + v1 * v1;
+        const bool sc = b < K && c < K;
+        if (!(sc && a < K)) w2 += v0 * v0;
+        if (!(sc && a + 1 < K)) w2 += v1 * v1;
+    });
+    tmem_fence_before_sync();
     block_sum2(n2, w2, red);
-    if (threadIdx.x == 0) {
+    __syncthreads();
+    tmem_fence_after_sync();
+    if (warp == 2) tmem_dealloc(tmem_slot, C::TCOLS);
+    if (tid == 0) {
         T.onorm2[it.node] = n2;
         T.ownorm2[it.node] = w2;
     }
@@ -217,44 +206,100 @@ struct AddOut {
 };
 constexpr int kAddMaxTerms = 256;
 
-// block of sum_i c_i f_i at one output node: compressed blocks are linear in the function, so the
-// inputs' blocks (own, or generated below the deepest ancestor) are combined as they are
+// Block of sum_i c_i f_i at one output node: compressed blocks are linear in the function, so the
+// inputs' blocks (own, or generated below the deepest ancestor) are combined as they are.  A lane keeps its
+// elements' sums in registers (element pairs in the order of the z product's outputs) and adds an own block
+// straight from global memory; a generated one comes from one separable transform.  HBM-bound when the inputs have the
+// nodes.
 template <int K>
-__global__ void __launch_bounds__(kMulThreads) k_add(const MulItem* __restrict__ items, AddOut out,
-                                                     const AddIn* __restrict__ in, int nin,
-                                                     const double* __restrict__ FTg) {
-    using G = Geo<K>;
-    constexpr int K2 = G::K2;
+struct AddCfg {
+    using B = BX<K, K>;
+    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 3 * B::FRAG);
+    static constexpr int PAIRS = 4 * K * K * K, PER = (PAIRS + B::NTHR - 1) / B::NTHR;  // element pairs per thread
+};
+template <int K>
+__global__ void __launch_bounds__(BX<K, K>::NTHR, 1)
+    k_add(const MulItem* __restrict__ items, AddOut out, const AddIn* __restrict__ in, int nin, const double* __restrict__ FTg) {
+    using B = BX<K, K>;
+    using C = AddCfg<K>;
+    constexpr int K2 = 2 * K, BS = Geo<K>::BS;
     extern __shared__ __align__(16) double asm_[];
-    double* ACC = asm_;
-    double* T = ACC + G::VOL;
-    double* FT = T + G::VOL;
-    double* unused = FT + K2 * K2;
-    double* red = unused + K2 * K2;
-    int* slot = reinterpret_cast<int*>(red + 64);
-    const int node = items[blockIdx.x].node;
-    for (int i = threadIdx.x; i < K2 * K2; i += blockDim.x) FT[i] = FTg[i];
-    for (int e = threadIdx.x; e < G::VOL; e += blockDim.x) ACC[e] = 0.0;
+    __shared__ double red[64];
+    __shared__ int found[kAddMaxTerms][2];
+    double* X = asm_;
+    double* f = X + B::VOL;
+    const int node = items[blockIdx.x].node, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t key = out.key[node];
-    __syncthreads();
-    for (int q = 0; q < nin; ++q) {
-        const AddIn f = in[q];
-        mul_fetch<K>(T, FT, f.hk, f.hv, f.hcap, f.coef, key, slot);
-        __syncthreads();
-        for (int e = threadIdx.x; e < G::VOL; e += blockDim.x) ACC[e] = fma(f.c, T[e], ACC[e]);
-        __syncthreads();
+    const int depth = key_depth(key);
+    long long tr[3];
+    key_trans(key, tr);
+    for (int q = warp; q < nin; q += B::NWARP) {
+        int idx, da;
+        bx_lookup(in[q].hk, in[q].hv, in[q].hcap, key, idx, da);
+        if (lane == 0) {
+            found[q][0] = idx;
+            found[q][1] = da;
+        }
     }
-    double* dst = out.coef + (size_t)node * G::BS;
+    __syncthreads();
+    double acc[C::PER][2];
+#pragma unroll
+    for (int i = 0; i < C::PER; ++i) acc[i][0] = acc[i][1] = 0.0;
+    for (int q = 0; q < nin; ++q) {
+        const int idx = found[q][0], da = found[q][1];
+        const double cf = in[q].c;
+        if (idx < 0) continue;  // outside the function's roots (cannot happen on one world): zero
+        const double* blk = in[q].coef + (size_t)idx * BS;
+        if (da == depth) {
+#pragma unroll
+            for (int i = 0; i < C::PER; ++i) {
+                const int e = tid + i * B::NTHR;
+                if (e < C::PAIRS) {
+                    const double2 v = __ldcs(reinterpret_cast<const double2*>(blk) + e);
+                    acc[i][0] = fma(cf, v.x, acc[i][0]);
+                    acc[i][1] = fma(cf, v.y, acc[i][1]);
+                }
+            }
+            continue;
+        }
+        __syncthreads();  // X is free
+        bx_path_operators<K, false>(FTg, nullptr, tr, depth - da, X, f);
+        bx_load<K>(X, blk);
+        cp_async_wait_all();
+        __syncthreads();
+        bx_slices<K, K>(X, f, f + B::FRAG);
+        __syncthreads();
+        bx_columns<K, K>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {  // in the columns' own place
+            double* p = X + c * B::LDP + B::physo(n);
+            p[0] = v0;
+            if (n + 1 < K * K) X[c * B::LDP + B::physo(n + 1)] = v1;
+        });
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < C::PER; ++i) {
+            const int e = tid + i * B::NTHR, a = 2 * (e % K), b = (e / K) % K2, c = e / (K * K2);
+            if (e < C::PAIRS && b < K && c < K) {
+                const double* p = X + c * B::LDP + B::LDO * b;
+                if (a < K) acc[i][0] = fma(cf, p[a], acc[i][0]);
+                if (a + 1 < K) acc[i][1] = fma(cf, p[a + 1], acc[i][1]);
+            }
+        }
+    }
+    double* dst = out.coef + (size_t)node * BS;
     double n2 = 0.0, w2 = 0.0;
-    for (int e = threadIdx.x; e < G::BS; e += blockDim.x) {
-        const int a = e % K2, b = (e / K2) % K2, c = e / (K2 * K2);
-        const double v = ACC[G::at(a, b, c)];
-        dst[e] = v;
-        n2 += v * v;
-        if (!(a < K && b < K && c < K)) w2 += v * v;
+#pragma unroll
+    for (int i = 0; i < C::PER; ++i) {
+        const int e = tid + i * B::NTHR, a = 2 * (e % K), b = (e / K) % K2, c = e / (K * K2);
+        if (e < C::PAIRS) {
+            reinterpret_cast<double2*>(dst)[e] = make_double2(acc[i][0], acc[i][1]);
+            n2 += acc[i][0] * acc[i][0] + acc[i][1] * acc[i][1];
+            const bool sc = b < K && c < K;
+            if (!(sc && a < K)) w2 += acc[i][0] * acc[i][0];
+            if (!(sc && a + 1 < K)) w2 += acc[i][1] * acc[i][1];
+        }
     }
     block_sum2(n2, w2, red);
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         out.norm2[node] = n2;
         out.wnorm2[node] = w2;
     }
@@ -500,8 +545,8 @@ void multiply_batched(double prec, int n, Tree** out, const double* c, Tree** a,
     {                                                                                                             \
         const size_t smem = MulCfg<KK>::SMEM;                                                                     \
         MWB_CUDA(cudaFuncSetAttribute(k_mul<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));        \
-        k_mul<KK><<<(unsigned)items.size(), kMulThreads, smem, s>>>(d_items, d_trees, m->d_MV, m->d_PF, m->d_FT, \
-                                                                     m->n0);                                      \
+        k_mul<KK><<<(unsigned)items.size(), BX<KK, 2 * KK>::NTHR, smem, s>>>(d_items, d_trees, m->d_MV, m->d_frMV,  \
+                                                                             m->d_frPF, m->d_FT, m->n0);          \
     }
         MWB_MUL_DISPATCH_K(K, L_MUL)
 #undef L_MUL
@@ -533,9 +578,9 @@ void add_trees(double prec, Tree* out, int n, const double* c, Tree** f, int max
         const AddOut ao{out->key, out->coef, out->norm2, out->wnorm2};
 #define L_ADD(KK)                                                                                                   \
     {                                                                                                               \
-        const size_t smem = MulCfg<KK>::SMEM;                                                                       \
+        const size_t smem = AddCfg<KK>::SMEM;                                                                       \
         MWB_CUDA(cudaFuncSetAttribute(k_add<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
-        k_add<KK><<<(unsigned)items.size(), kMulThreads, smem, s>>>(d_items, ao, d_in, n, m->d_FT);               \
+        k_add<KK><<<(unsigned)items.size(), BX<KK, KK>::NTHR, smem, s>>>(d_items, ao, d_in, n, m->d_FT);           \
     }
         MWB_MUL_DISPATCH_K(K, L_ADD)
 #undef L_ADD
