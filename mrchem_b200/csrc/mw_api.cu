@@ -95,13 +95,18 @@ void upload_bytes(Ctx* ctx, void* dst, const void* src, size_t bytes) {
     ctx->pin_off += (bytes + 255) & ~(size_t)255;
 }
 
-void readback(Ctx* ctx, std::initializer_list<ReadReq> reqs) {
+double* mailbox(Ctx* ctx) {
     constexpr size_t kBox = 4u << 20;
     if (!ctx->mbox) {
         MWB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&ctx->mbox), kBox, cudaHostAllocMapped));
         MWB_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&ctx->mbox_dev), ctx->mbox, 0));
         ctx->mbox_cap = kBox;
     }
+    return reinterpret_cast<double*>(ctx->mbox_dev);
+}
+
+void readback(Ctx* ctx, std::initializer_list<ReadReq> reqs) {
+    mailbox(ctx);
     if (reqs.size() > 8) throw Error(MW_ERR_ARG, "readback: at most 8 ranges");
     CopyList L{};
     long long at[8];  // mailbox offset of each request, -1: empty or through the copy engine
@@ -217,59 +222,6 @@ void tree_reserve(Tree& t, int need) {
     }
 }
 
-// root boxes in Morton order
-void tree_make_roots(Tree& t) {
-    const Mra& m = *t.mra;
-    std::vector<uint64_t> keys;
-    for (int z = 0; z < m.boxes[2]; ++z)
-        for (int y = 0; y < m.boxes[1]; ++y)
-            for (int x = 0; x < m.boxes[0]; ++x) keys.push_back(host_make_key(0, x, y, z));
-    std::sort(keys.begin(), keys.end());
-    t.n = 0;
-    t.level_begin.clear();
-    tree_reserve(t, (int)keys.size());
-    cudaStream_t s = m.ctx->stream;
-    launch_hash_reset(t, s);
-    const int n = (int)keys.size();
-    std::vector<int> par(n, -1);
-    upload_bytes(m.ctx, t.key, keys.data(), sizeof(uint64_t) * n);  // staged: the host vectors may go
-    upload_bytes(m.ctx, t.parent, par.data(), sizeof(int) * n);
-    upload_bytes(m.ctx, t.child0, par.data(), sizeof(int) * n);
-    MWB_CUDA(cudaMemsetAsync(t.norm2, 0, sizeof(double) * n, s));
-    MWB_CUDA(cudaMemsetAsync(t.wnorm2, 0, sizeof(double) * n, s));
-    t.n = n;
-    t.level_begin = {0, n};
-    launch_hash_insert(t, 0, n, s);
-}
-
-// split the nodes of the last level whose wavelet norm exceeds thr; returns the number of new nodes
-int tree_refine_last_level(Tree& t, double thr) {
-    Ctx* ctx = t.mra->ctx;
-    cudaStream_t s = ctx->stream;
-    const int b = t.level_begin[t.levels() - 1], e = t.level_begin[t.levels()];
-    const int depth = t.levels() - 1;
-    int* d_list = (int*)dalloc(ctx, sizeof(int) * std::max(1, e - b));
-    int ns = launch_split(t, b, e, depth, thr, t.mra->depth_limit, d_list, s);
-    if (ns > 0) {
-        tree_reserve(t, t.n + 8 * ns);
-        launch_make_children(t, d_list, ns, s);
-        launch_hash_insert(t, t.n, t.n + 8 * ns, s);
-        t.n += 8 * ns;
-        t.level_begin.push_back(t.n);
-    }
-    dfree(ctx, d_list);
-    return 8 * ns;
-}
-
-static int* range_list(Ctx* ctx, int begin, int end) {
-    std::vector<int> v(end - begin);
-    std::iota(v.begin(), v.end(), begin);
-    int* d = (int*)dalloc(ctx, sizeof(int) * std::max<size_t>(1, v.size()));
-    MWB_CUDA(cudaMemcpyAsync(d, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, ctx->stream));
-    MWB_CUDA(cudaStreamSynchronize(ctx->stream));
-    return d;
-}
-
 // bottom-up: every internal node becomes the compression of its children's scaling parts
 void tree_compress_bottom_up(Tree& t) {
     cudaStream_t s = t.mra->ctx->stream;
@@ -292,18 +244,13 @@ static void project(double prec, Tree& t, int type, int np, const double* params
     if (per < 0) throw Error(MW_ERR_ARG, "unknown function type");
     if (np < 1 + per * nterm) throw Error(MW_ERR_ARG, "parameter block too short");
     double* d_p = (double*)dalloc(ctx, sizeof(double) * np);
-    MWB_CUDA(cudaMemcpyAsync(d_p, params, sizeof(double) * np, cudaMemcpyHostToDevice, s));
+    upload_bytes(ctx, d_p, params, sizeof(double) * np);
     FuncDesc f{type, nterm, d_p};
-    tree_make_roots(t);
+    trees_make_roots({&t});
     int b = 0, e = t.n;
     while (e > b) {
-        int* d_list = range_list(ctx, b, e);
-        launch_transform_nodes(t, TM_PROJECT, d_list, e - b, &f, s);
-        dfree(ctx, d_list);
-        if (prec <= 0.0) break;
-        const double ref = std::sqrt(reduce_leaf_norm2(t, s));
-        const int added = tree_refine_last_level(t, split_threshold(prec, ref, t.levels() - 1));
-        if (added == 0) break;
+        launch_transform_nodes(t, TM_PROJECT, nullptr, e - b, &f, s, b);
+        if (prec <= 0.0 || tree_refine_last_level(t, prec) == 0) break;
         b = e;
         e = t.n;
     }
@@ -589,7 +536,7 @@ static void apply_batched(double prec, int n, Tree** out, Op** op, Tree** inp, i
         add_children_many(grow, lists);
         total_trip += bp.triples;
     }
-    trees_finish(std::vector<Tree*>(out, out + n), true, true, true, s);
+    trees_finish(std::vector<Tree*>(out, out + n), true, s);
     MWB_CUDA(cudaStreamSynchronize(s));
     for (int i = 0; i < n; ++i) {
         out[i]->g0 = g0[i];
@@ -803,7 +750,7 @@ static void apply_learned(double prec, int n, Tree** out, Op** op, Tree** inp, i
     // appended refinements in level order)
     pruned += trees_rebuild_device(all, d_keep, s);
     dfree(ctx, d_keep);
-    trees_finish(std::vector<Tree*>(out, out + n), true, true, true, s);
+    trees_finish(std::vector<Tree*>(out, out + n), true, s);
     for (int i = 0; i < n; ++i) {
         out[i]->g0 = g0[i];
         out[i]->prec = prec;
@@ -857,7 +804,7 @@ static void apply_derivative(Tree* out, Op* op, Tree* inp, int dir, int precisio
     Op* p[1] = {op};
     Tree* i1[1] = {inp};
     const long long trip = run_entries(0.0, precision, ents, o, p, i1, fnorm, nu_max, g0, dir);
-    trees_finish(std::vector<Tree*>{out}, true, true, true, s);
+    trees_finish(std::vector<Tree*>{out}, true, s);
     MWB_CUDA(cudaStreamSynchronize(s));
     out->g0 = 0.0;
     out->prec = 0.0;
@@ -911,6 +858,10 @@ static void ctx_free(mwb::Ctx* ctx) {
     if (ctx->pin_ev) cudaEventDestroy(ctx->pin_ev);
     if (ctx->pin) cudaFreeHost(ctx->pin);
     if (ctx->mbox) cudaFreeHost(ctx->mbox);
+    if (ctx->ticket) {
+        mwb::dfree(ctx, ctx->ticket);
+        cudaStreamSynchronize(ctx->stream);
+    }
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete static_cast<mw_ctx_s*>(ctx);
 }
@@ -923,9 +874,6 @@ static void mra_free(mwb::Mra* m) {
     mwb::dfree(c, m->d_F);
     mwb::dfree(c, m->d_FT);
     mwb::dfree(c, m->d_frF);
-    mwb::dfree(c, m->d_frFT);
-    mwb::dfree(c, m->d_frPF);
-    mwb::dfree(c, m->d_frMV);
     mwb::dfree(c, m->d_MV);
     mwb::dfree(c, m->d_cc);
     mwb::dfree(c, m->d_px);

@@ -64,6 +64,7 @@ struct Ctx {
     char* mbox = nullptr;
     char* mbox_dev = nullptr;
     size_t mbox_cap = 0;
+    unsigned* ticket = nullptr;  // blocks done of a reduction whose last block finishes it (zero between calls)
 };
 
 struct Mra {
@@ -193,6 +194,8 @@ struct ReadReq {
     size_t bytes;
 };
 void readback(Ctx* ctx, std::initializer_list<ReadReq> reqs);
+// device address of the mailbox, for a kernel that writes its result there (read ctx->mbox after a synchronisation)
+double* mailbox(Ctx* ctx);
 // the same on stream s: through the mailbox when s is the context's stream, else copy-engine copies on s
 void readback(Ctx* ctx, cudaStream_t s, std::initializer_list<ReadReq> reqs);
 

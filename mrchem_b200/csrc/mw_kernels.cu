@@ -86,19 +86,10 @@ __device__ inline double hydrogen(int n, int l, int m, double Z, double x, doubl
     return radial * ca * ang;
 }
 
+// products of hydrogen orbitals (Gaussian sums are evaluated by their factors, transform_node)
 __device__ inline double eval_func(const FuncDesc& f, double x, double y, double z) {
     double v = 0.0;
-    if (f.type == 1) {
-        for (int g = 0; g < f.nterm; ++g) {
-            const double* q = f.p + 1 + 8 * g;
-            const double dx = x - q[2], dy = y - q[3], dz = z - q[4];
-            double p = 1.0;
-            for (int i = 0; i < (int)q[5]; ++i) p *= dx;
-            for (int i = 0; i < (int)q[6]; ++i) p *= dy;
-            for (int i = 0; i < (int)q[7]; ++i) p *= dz;
-            v += q[0] * p * exp(-q[1] * (dx * dx + dy * dy + dz * dz));
-        }
-    } else if (f.type == 2) {
+    if (f.type == 2) {
         for (int t = 0; t < f.nterm; ++t) {
             const double* q = f.p + 1 + 11 * t;
             const double X = x - q[8], Y = y - q[9], Zc = z - q[10];
@@ -130,6 +121,8 @@ struct WorldGeo {
     double qx[16]; // quadrature nodes on [0,1]
 };
 
+constexpr int kGaussBatch = 8;
+
 template <int K>
 struct TrCfg {
     using B = BX<K, 2 * K>;
@@ -147,6 +140,7 @@ __device__ __forceinline__ void transform_node(int mode, int node, const TView& 
     constexpr int K2 = 2 * K, BS = Geo<K>::BS;
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[64];
+    __shared__ double gf[kGaussBatch][3][K2];
     double* X = sm;
     double* fo = X + B::VOL;
     bx_operator(fo, fr, 2 * B::FRAG, B::NTHR);
@@ -159,12 +153,36 @@ __device__ __forceinline__ void transform_node(int mode, int node, const TView& 
         const int n1 = wg.n0 + key_depth(key) + 1;
         const double h = ldexp(1.0, -n1);
         fac = pow(2.0, -1.5 * n1);
-        for (int e = threadIdx.x; e < BS; e += B::NTHR) {
-            const int a = e % K2, b = (e / K2) % K2, c = e / (K2 * K2);
-            const double x = wg.lo[0] + (2 * tr[0] + a / K + wg.qx[a % K]) * h;
-            const double y = wg.lo[1] + (2 * tr[1] + b / K + wg.qx[b % K]) * h;
-            const double z = wg.lo[2] + (2 * tr[2] + c / K + wg.qx[c % K]) * h;
-            X[at(a, b, c)] = eval_func(f, x, y, z);
+        auto coord = [&](int d, int i) { return wg.lo[d] + (2 * tr[d] + i / K + wg.qx[i % K]) * h; };
+        if (f.type == 1) {
+            // sums of Gaussians: the factors along each direction once per node (3 x 2k exponentials per Gaussian instead
+            // of (2k)^3; they were most of a projection), eight Gaussians at a time
+            for (int g0 = 0; g0 < f.nterm; g0 += kGaussBatch) {
+                const int ng = min(kGaussBatch, f.nterm - g0);
+                if (g0 > 0) __syncthreads();  // the previous factors are read
+                for (int e = threadIdx.x; e < ng * 3 * K2; e += B::NTHR) {
+                    const int g = e / (3 * K2), d = (e / K2) % 3, i = e % K2;
+                    const double* q = f.p + 1 + 8 * (g0 + g);
+                    const double u = coord(d, i) - q[2 + d];
+                    double v = d == 0 ? q[0] : 1.0;
+                    for (int j = 0; j < (int)q[5 + d]; ++j) v *= u;
+                    gf[g][d][i] = v * exp(-q[1] * u * u);
+                }
+                __syncthreads();
+                for (int e = threadIdx.x; e < BS; e += B::NTHR) {
+                    const int a = e % K2, b = (e / K2) % K2, c = e / (K2 * K2);
+                    double v = g0 > 0 ? X[at(a, b, c)] : 0.0;
+                    for (int g = 0; g < ng; ++g) v = fma(gf[g][0][a] * gf[g][1][b], gf[g][2][c], v);
+                    X[at(a, b, c)] = v;
+                }
+            }
+            if (f.nterm <= 0)
+                for (int e = threadIdx.x; e < B::VOL; e += B::NTHR) X[e] = 0.0;
+        } else {
+            for (int e = threadIdx.x; e < BS; e += B::NTHR) {
+                const int a = e % K2, b = (e / K2) % K2, c = e / (K2 * K2);
+                X[at(a, b, c)] = eval_func(f, coord(0, a), coord(1, b), coord(2, c));
+            }
         }
     } else if (mode == TM_COMPRESS) {
         const int c0 = t.child0[node];
@@ -289,43 +307,6 @@ __global__ void k_node_norms(TView t, int begin, int end) {
     }
 }
 
-__global__ void k_split_flags(const double* __restrict__ wnorm2, const uint64_t* __restrict__ key, int begin,
-                              int end, double thr, int depth_limit, int* flags) {
-    const int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= end) return;
-    flags[i - begin] = (key_depth(key[i]) < depth_limit && sqrt(wnorm2[i]) > thr) ? 1 : 0;
-}
-__global__ void k_internal_flags(const int* __restrict__ child0, int begin, int end, int* flags) {
-    const int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= end) return;
-    flags[i - begin] = child0[i] >= 0 ? 1 : 0;
-}
-__global__ void k_scatter_list(const int* __restrict__ flags, const int* __restrict__ pos, int begin, int n,
-                               int* list) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (flags[i]) list[pos[i]] = begin + i;
-}
-__global__ void k_make_children(TView t, const int* __restrict__ list, int nsplit, int nold) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nsplit) return;
-    const int p = list[q];
-    const int c0 = nold + 8 * q;
-    t.child0[p] = c0;
-    long long tr[3];
-    const uint64_t key = t.key[p];
-    key_trans(key, tr);
-    const int d = key_depth(key) + 1;
-    for (int c = 0; c < 8; ++c) {
-        const int i = c0 + c;
-        t.key[i] = make_key(d, 2 * tr[0] + (c & 1), 2 * tr[1] + ((c >> 1) & 1), 2 * tr[2] + ((c >> 2) & 1));
-        t.parent[i] = p;
-        t.child0[i] = -1;
-        t.norm2[i] = 0.0;
-        t.wnorm2[i] = 0.0;
-    }
-}
-
 // children of the split nodes of several trees in one launch: entry q of the flat list belongs to tree
 // tree_of[q]; its 8 children are appended after the tree's first nold nodes (in list order) and
 // entered into the tree's hash index
@@ -403,34 +384,109 @@ __global__ void k_reduce_norm2_many(const NormSrc* __restrict__ src, int nt, dou
     if (threadIdx.x == 0) out[mx * nt + t] = s;
 }
 
+// Split decisions of a tree's last level in one block: the threshold from the leaves' norm (the same sum as
+// k_reduce_norm2), then the level's nodes above it, in order.  fac = 2^{-depth / 2}; out[0] = count, list follows
+__global__ void __launch_bounds__(1024) k_level_split(const double* __restrict__ norm2, const double* __restrict__ wnorm2,
+                                                      const int* __restrict__ child0, int begin, int end, double prec,
+                                                      double fac, int may_split, int* out) {
+    __shared__ double thr;
+    __shared__ int wsum[32];
+    const double s2 = reduce_norm2_block(norm2, child0, 0, end, 1, 0);
+    if (threadIdx.x == 0) thr = prec * sqrt(s2) * fac;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int base = 0;
+    for (int b = begin; b < end; b += 1024) {
+        const int i = b + threadIdx.x;
+        const bool f = i < end && may_split && sqrt(wnorm2[i]) > thr;
+        const unsigned m = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) wsum[warp] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (f) out[1 + base + before + __popc(m & ((1u << lane) - 1u))] = i;
+        base += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[0] = base;
+}
+// children of the listed nodes, appended after the first nold nodes and entered into the hash index
+__global__ void k_make_children(TView t, uint64_t* hkey, int* hval, uint32_t hcap, const int* __restrict__ list, int nsplit, int nold) {
+    const int q = (blockIdx.x * blockDim.x + threadIdx.x) / 8, c = threadIdx.x & 7;
+    if (q >= nsplit) return;
+    const int p = list[q], i = nold + 8 * q + c;
+    if (c == 0) t.child0[p] = nold + 8 * q;
+    long long tr[3];
+    const uint64_t key = t.key[p];
+    key_trans(key, tr);
+    const uint64_t ck = make_key(key_depth(key) + 1, 2 * tr[0] + (c & 1), 2 * tr[1] + ((c >> 1) & 1), 2 * tr[2] + ((c >> 2) & 1));
+    t.key[i] = ck;
+    t.parent[i] = p;
+    t.child0[i] = -1;
+    t.norm2[i] = 0.0;
+    t.wnorm2[i] = 0.0;
+    hash_insert_one(hkey, hval, hcap, ck, i);
+}
+
 __global__ void k_rescale(double* coef, size_t n, double c) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         coef[i] *= c;
 }
 
-// per node of a: <a_node|b_node> over the wavelet part (all components at depth 0)
+// <a|b>: per node of a (four warps, so that a small block's loads are all in flight at once) the product over the wavelet part (all components at depth 0), then the last block to
+// finish adds the nodes' parts in a fixed order and writes the sum where the host reads it (mapped memory).  A second
+// launch for the sum, a copy and two scalar loads per element took twice as long.
+constexpr int kDotThreads = 256;
 template <int K>
-__global__ void k_dot_nodes(TView a, int na, const double* __restrict__ bcoef, const uint64_t* hk, const int* hv,
-                            uint32_t hcap, double* part) {
+__global__ void __launch_bounds__(kDotThreads) k_dot(TView a, int na, const double* __restrict__ bcoef, const uint64_t* hk,
+                                                     const int* hv, uint32_t hcap, double* part, unsigned* ticket, double* out) {
     using G = Geo<K>;
-    const int node = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-    const int lane = threadIdx.x & 31;
-    if (node >= na) return;
-    const uint64_t key = a.key[node];
-    const int j = hlookup(hk, hv, hcap, key);
+    __shared__ double red[64];
+    __shared__ unsigned done;
+    __shared__ double ws[kDotThreads / 32];
+    const int node = blockIdx.x * (kDotThreads / 128) + threadIdx.x / 128, t = threadIdx.x & 127;
     double s = 0.0;
-    if (j >= 0) {
-        const bool root = key_depth(key) == 0;
-        const double* x = a.coef + (size_t)node * G::BS;
-        const double* y = bcoef + (size_t)j * G::BS;
-        for (int e = lane; e < G::BS; e += 32) {
-            const int aa = e % G::K2, bb = (e / G::K2) % G::K2, cc = e / (G::K2 * G::K2);
-            if (!root && aa < K && bb < K && cc < K) continue;
-            s += x[e] * y[e];
+    if (node < na) {
+        const uint64_t key = a.key[node];
+        const int j = hlookup(hk, hv, hcap, key);
+        if (j >= 0) {
+            const bool root = key_depth(key) == 0;
+            const double2* x = reinterpret_cast<const double2*>(a.coef + (size_t)node * G::BS);
+            const double2* y = reinterpret_cast<const double2*>(bcoef + (size_t)j * G::BS);
+#pragma unroll 8
+            for (int e = t; e < G::BS / 2; e += 128) {
+                const double2 u = x[e], v = y[e];
+                const int aa = 2 * (e % K), bb = (e / K) % G::K2, cc = e / (K * G::K2);
+                const bool sc = !root && bb < K && cc < K;
+                if (!(sc && aa < K)) s = fma(u.x, v.x, s);
+                if (!(sc && aa + 1 < K)) s = fma(u.y, v.y, s);
+            }
         }
     }
     for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) part[node] = s;
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (t == 0 && node < na) {
+        const double* w = ws + (threadIdx.x >> 5);
+        part[node] = (w[0] + w[1]) + (w[2] + w[3]);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) done = atomicAdd(ticket, 1u);
+    __syncthreads();
+    if (done != gridDim.x - 1) return;
+    __threadfence();
+    double d = 0.0;
+    s = 0.0;
+    for (int i = threadIdx.x; i < na; i += kDotThreads) s += __ldcg(part + i);
+    block_sum2(s, d, red);
+    if (threadIdx.x == 0) {
+        *ticket = 0u;  // for the next call on this stream
+        *out = s;
+    }
 }
 // ||a - b||^2 contributions of a's nodes (one warp per node): root scaling parts and all wavelet
 // parts of a - b, where b's node is missing its block counts as zero; with `only_missing` the
@@ -496,30 +552,28 @@ static WorldGeo world_geo(const Mra& m) {
 }
 
 void world_fragments(Mra& m, const std::vector<double>& PF, const std::vector<double>& MV, const std::vector<double>& FT) {
-    auto image = [&](const std::vector<double>& M) {
-        std::vector<double> f;
+    std::vector<double> f;
+    const std::vector<double>* mats[4] = {&m.F, &FT, &PF, &MV};
 #define L_FR(KK)                                                                            \
     {                                                                                       \
         constexpr int N = BX<KK, 2 * KK>::FRAG, W = 2 * KK;                                  \
-        f.resize(2 * N);                                                                     \
-        auto entry = [&](int o, int i) { return M[(size_t)o * W + i]; };                     \
-        for (int e = 0; e < N; ++e) {                                                        \
-            f[e] = bx_frag_a<KK, 2 * KK>(e, entry);                                          \
-            f[N + e] = bx_frag_b<KK, 2 * KK>(e, entry);                                      \
+        m.fr_n = N;                                                                          \
+        f.resize(8 * N);                                                                     \
+        for (int q = 0; q < 4; ++q) {                                                        \
+            auto entry = [&](int o, int i) { return (*mats[q])[(size_t)o * W + i]; };        \
+            for (int e = 0; e < N; ++e) {                                                    \
+                f[2 * q * N + e] = bx_frag_a<KK, 2 * KK>(e, entry);                          \
+                f[(2 * q + 1) * N + e] = bx_frag_b<KK, 2 * KK>(e, entry);                    \
+            }                                                                                \
         }                                                                                    \
     }
-        MWB_DISPATCH_K(m.k, L_FR)
+    MWB_DISPATCH_K(m.k, L_FR)
 #undef L_FR
-        m.fr_n = (int)f.size() / 2;
-        double* d = (double*)dalloc(m.ctx, sizeof(double) * f.size());
-        MWB_CUDA(cudaMemcpyAsync(d, f.data(), sizeof(double) * f.size(), cudaMemcpyHostToDevice, m.ctx->stream));
-        MWB_CUDA(cudaStreamSynchronize(m.ctx->stream));  // f leaves scope
-        return d;
-    };
-    m.d_frF = image(m.F);
-    m.d_frFT = image(FT);
-    m.d_frPF = image(PF);
-    m.d_frMV = image(MV);
+    m.d_frF = (double*)dalloc(m.ctx, sizeof(double) * f.size());  // one allocation for the four
+    m.d_frFT = m.d_frF + 2 * m.fr_n;
+    m.d_frPF = m.d_frF + 4 * m.fr_n;
+    m.d_frMV = m.d_frF + 6 * m.fr_n;
+    upload_bytes(m.ctx, m.d_frF, f.data(), sizeof(double) * f.size());
 }
 
 void launch_transform_nodes(Tree& t, int mode, const int* d_nodes, int nnodes, const FuncDesc* f, cudaStream_t s,
@@ -543,8 +597,9 @@ void launch_transform_nodes(Tree& t, int mode, const int* d_nodes, int nnodes, c
 }
 
 // Finishing transforms of a batch of trees on one world, one launch per level for all trees:
-// sum-up top-down (sumup), then compress bottom-up (compress), then the norms of every node (norms).
-void trees_finish(const std::vector<Tree*>& ts, bool sumup, bool compress, bool norms, cudaStream_t s) {
+// sum-up top-down (sumup), then compress bottom-up, then the norms of every node (the sums an upload makes, so that a
+// tree read back has them bit for bit).
+void trees_finish(const std::vector<Tree*>& ts, bool sumup, cudaStream_t s) {
     if (ts.empty()) return;
     const Mra& m = *ts[0]->mra;
     Ctx* ctx = m.ctx;
@@ -585,9 +640,8 @@ void trees_finish(const std::vector<Tree*>& ts, bool sumup, bool compress, bool 
     };
     if (sumup)
         for (int d = 0; d + 1 < maxl; ++d) level(TM_SUMUP, d);
-    if (compress)
-        for (int d = maxl - 2; d >= 0; --d) level(TM_COMPRESS, d);
-    if (norms) {
+    for (int d = maxl - 2; d >= 0; --d) level(TM_COMPRESS, d);
+    {
         const int n = (int)items.size();
 #define L_NNM(KK) k_node_norms_multi<KK><<<(n * 32 + 255) / 256, 256, 0, s>>>(d_items, n, d_views);
         MWB_DISPATCH_K(m.k, L_NNM)
@@ -622,53 +676,29 @@ void launch_hash_insert(Tree& t, int begin, int end, cudaStream_t s) {
     count(t.mra->ctx);
 }
 
-// flags -> exclusive scan -> list; returns the count (synchronises the stream)
-static int compact_flags(Ctx* ctx, int* d_flags, int n, int begin, int* d_list, cudaStream_t s) {
-    if (n <= 0) return 0;
-    int* d_pos = (int*)dalloc(ctx, sizeof(int) * (n + 1));
-    size_t tmp = 0;
-    MWB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, d_flags, d_pos, n + 1, s));
-    void* d_tmp = dalloc(ctx, tmp);
-    MWB_CUDA(cub::DeviceScan::ExclusiveSum(d_tmp, tmp, d_flags, d_pos, n + 1, s));
-    k_scatter_list<<<(n + 255) / 256, 256, 0, s>>>(d_flags, d_pos, begin, n, d_list);
-    MWB_CUDA(cudaGetLastError());
-    count(ctx);
-    int total = 0;
-    MWB_CUDA(cudaMemcpyAsync(&total, d_pos + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MWB_CUDA(cudaStreamSynchronize(s));
-    dfree(ctx, d_tmp);
-    dfree(ctx, d_pos);
-    return total;
-}
-
-int launch_split(Tree& t, int begin, int end, int depth, double thr, int depth_limit, int* d_list,
-                 cudaStream_t s) {
-    (void)depth;
-    const int n = end - begin;
-    if (n <= 0) return 0;
+// split the nodes of the tree's last level whose wavelet norm exceeds prec ||f|| 2^{-depth/2}; returns the number of
+// new nodes (two launches and one read-back)
+int tree_refine_last_level(Tree& t, double prec) {
     Ctx* ctx = t.mra->ctx;
-    int* d_flags = (int*)dalloc(ctx, sizeof(int) * (n + 1));
-    MWB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (n + 1), s));
-    k_split_flags<<<(n + 255) / 256, 256, 0, s>>>(t.wnorm2, t.key, begin, end, thr, depth_limit, d_flags);
+    cudaStream_t s = ctx->stream;
+    const int depth = t.levels() - 1, b = t.level_begin[depth], e = t.level_begin[depth + 1];
+    int* d_out = (int*)dalloc(ctx, sizeof(int) * (e - b + 1));
+    k_level_split<<<1, 1024, 0, s>>>(t.norm2, t.wnorm2, t.child0, b, e, prec, std::pow(2.0, -0.5 * depth),
+                                     depth < t.mra->depth_limit, d_out);
     MWB_CUDA(cudaGetLastError());
     count(ctx);
-    int cnt = compact_flags(ctx, d_flags, n, begin, d_list, s);
-    dfree(ctx, d_flags);
-    return cnt;
-}
-
-int launch_internal_list(Tree& t, int begin, int end, int* d_list, cudaStream_t s) {
-    const int n = end - begin;
-    if (n <= 0) return 0;
-    Ctx* ctx = t.mra->ctx;
-    int* d_flags = (int*)dalloc(ctx, sizeof(int) * (n + 1));
-    MWB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (n + 1), s));
-    k_internal_flags<<<(n + 255) / 256, 256, 0, s>>>(t.child0, begin, end, d_flags);
-    MWB_CUDA(cudaGetLastError());
-    count(ctx);
-    int cnt = compact_flags(ctx, d_flags, n, begin, d_list, s);
-    dfree(ctx, d_flags);
-    return cnt;
+    int ns = 0;
+    readback(ctx, {{&ns, d_out, sizeof(int)}});
+    if (ns > 0) {
+        tree_reserve(t, t.n + 8 * ns);
+        k_make_children<<<(ns + 15) / 16, 128, 0, s>>>(view(t), t.hkey, t.hval, t.hcap, d_out + 1, ns, t.n);
+        MWB_CUDA(cudaGetLastError());
+        count(ctx);
+        t.n += 8 * ns;
+        t.level_begin.push_back(t.n);
+    }
+    dfree(ctx, d_out);
+    return 8 * ns;
 }
 
 void trees_add_children(const std::vector<Tree*>& ts, const std::vector<std::vector<int>>& lists, cudaStream_t s) {
@@ -709,18 +739,11 @@ void trees_add_children(const std::vector<Tree*>& ts, const std::vector<std::vec
     dfree(ctx, d_ct);
 }
 
-void launch_make_children(Tree& t, const int* d_list, int nsplit, cudaStream_t s) {
-    if (nsplit <= 0) return;
-    k_make_children<<<(nsplit + 127) / 128, 128, 0, s>>>(view(t), d_list, nsplit, t.n);
-    MWB_CUDA(cudaGetLastError());
-    count(t.mra->ctx);
-}
-
-static double reduce_impl(Tree& t, int begin, int end, int leaves, int mx, cudaStream_t s) {
-    if (end <= begin) return 0.0;
+double reduce_leaf_norm2(Tree& t, cudaStream_t s) {
+    if (t.n <= 0) return 0.0;
     Ctx* ctx = t.mra->ctx;
     double* d = (double*)dalloc(ctx, sizeof(double));
-    k_reduce_norm2<<<1, 1024, 0, s>>>(t.norm2, t.child0, begin, end, leaves, mx, d);
+    k_reduce_norm2<<<1, 1024, 0, s>>>(t.norm2, t.child0, 0, t.n, 1, 0, d);
     MWB_CUDA(cudaGetLastError());
     count(ctx);
     double h = 0.0;
@@ -729,7 +752,6 @@ static double reduce_impl(Tree& t, int begin, int end, int leaves, int mx, cudaS
     dfree(ctx, d);
     return h;
 }
-double reduce_leaf_norm2(Tree& t, cudaStream_t s) { return reduce_impl(t, 0, t.n, 1, 0, s); }
 
 // squared norm (leaves) and largest node norm^2 of several trees with one synchronisation
 void reduce_norms_many(const std::vector<Tree*>& ts, std::vector<double>& leaf2, std::vector<double>& max2,
@@ -756,8 +778,6 @@ void reduce_norms_many(const std::vector<Tree*>& ts, std::vector<double>& leaf2,
         max2[i] = h[n + i];
     }
 }
-double reduce_range_norm2(Tree& t, int begin, int end, cudaStream_t s) { return reduce_impl(t, begin, end, 0, 0, s); }
-double reduce_max_norm2(Tree& t, cudaStream_t s) { return reduce_impl(t, 0, t.n, 0, 1, s); }
 
 void launch_rescale(Tree& t, double c, cudaStream_t s) {
     if (t.n == 0) return;
@@ -771,21 +791,23 @@ void launch_rescale(Tree& t, double c, cudaStream_t s) {
 double launch_dot(Tree& a, Tree& b, cudaStream_t s) {
     if (a.n == 0 || b.n == 0) return 0.0;
     Ctx* ctx = a.mra->ctx;
+    if (!ctx->ticket) {
+        ctx->ticket = (unsigned*)dalloc(ctx, sizeof(unsigned));
+        MWB_CUDA(cudaMemsetAsync(ctx->ticket, 0, sizeof(unsigned), s));
+    }
     double* part = (double*)dalloc(ctx, sizeof(double) * a.n);
-    double* d = (double*)dalloc(ctx, sizeof(double));
+    double* res = mailbox(ctx);
     TView av = view(a);
-#define L_DOT(KK) k_dot_nodes<KK><<<(a.n * 32 + 255) / 256, 256, 0, s>>>(av, a.n, b.coef, b.hkey, b.hval, b.hcap, part);
+#define L_DOT(KK)                                                                                                        \
+    k_dot<KK><<<(a.n + kDotThreads / 128 - 1) / (kDotThreads / 128), kDotThreads, 0, s>>>(av, a.n, b.coef, b.hkey, b.hval, b.hcap, part, \
+                                                                                 ctx->ticket, res);
     MWB_DISPATCH_K(a.mra->k, L_DOT)
 #undef L_DOT
-    k_sum_array<<<1, 1024, 0, s>>>(part, a.n, d);
     MWB_CUDA(cudaGetLastError());
-    count(ctx, 2);
-    double h = 0.0;
-    MWB_CUDA(cudaMemcpyAsync(&h, d, sizeof(double), cudaMemcpyDeviceToHost, s));
-    MWB_CUDA(cudaStreamSynchronize(s));
+    count(ctx);
     dfree(ctx, part);
-    dfree(ctx, d);
-    return h;
+    MWB_CUDA(cudaStreamSynchronize(s));
+    return *reinterpret_cast<volatile double*>(ctx->mbox);
 }
 
 // ||a - b|| of two compressed trees on one world (any grids)

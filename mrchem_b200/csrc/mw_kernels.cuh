@@ -34,25 +34,15 @@ struct InView {
 void launch_transform_nodes(Tree& t, int mode, const int* d_nodes, int nnodes, const FuncDesc* f, cudaStream_t s,
                             int begin = 0);
 void launch_node_norms(Tree& t, int begin, int end, cudaStream_t s);
-// sum-up top-down, compress bottom-up and/or node norms of several trees, one launch per level
-void trees_finish(const std::vector<Tree*>& ts, bool sumup, bool compress, bool norms, cudaStream_t s);
+// sum-up top-down, compress bottom-up and node norms of several trees, one launch per level
+void trees_finish(const std::vector<Tree*>& ts, bool sumup, cudaStream_t s);
 void launch_hash_reset(Tree& t, cudaStream_t s);
 void launch_hash_insert(Tree& t, int begin, int end, cudaStream_t s);
-// flags[i - begin] = sqrt(wnorm2[i]) > thr(depth) for i in [begin, end); returns number of splits
-// and writes the split list (tree indices) to d_list
-int launch_split(Tree& t, int begin, int end, int depth, double thr, int depth_limit, int* d_list,
-                 cudaStream_t s);
-// append 8 children for each node in d_list (n_split entries)
-void launch_make_children(Tree& t, const int* d_list, int nsplit, cudaStream_t s);
 // append 8 children for every node in lists[i] of tree ts[i] (one level per tree), enter them into the
 // hash indices and push the new level start; one launch for all trees
 void trees_add_children(const std::vector<Tree*>& ts, const std::vector<std::vector<int>>& lists, cudaStream_t s);
-// internal node list of [begin, end) (returns count)
-int launch_internal_list(Tree& t, int begin, int end, int* d_list, cudaStream_t s);
-// deterministic reductions: sum of norm2 over leaves (or over [begin,end) when all=true), max norm2
+// deterministic reductions: sum of norm2 over leaves; with the largest norm2, of several trees
 double reduce_leaf_norm2(Tree& t, cudaStream_t s);
-double reduce_range_norm2(Tree& t, int begin, int end, cudaStream_t s);
-double reduce_max_norm2(Tree& t, cudaStream_t s);
 void reduce_norms_many(const std::vector<Tree*>& ts, std::vector<double>& leaf2, std::vector<double>& max2,
                        cudaStream_t s);
 void launch_rescale(Tree& t, double c, cudaStream_t s);
@@ -63,14 +53,13 @@ void launch_gather_blocks(const double* src, const int* perm, int n, size_t bs, 
 
 // tree bookkeeping shared by the drivers (mw_api.cu)
 void tree_reserve(Tree& t, int need);
-void tree_make_roots(Tree& t);
 // the root level of several trees of one world at once (two launches for the batch)
 void trees_make_roots(const std::vector<Tree*>& ts);
 // rebuild the hash indices of several trees of one context from their node keys (two launches)
 void trees_rehash(const std::vector<Tree*>& ts);
 void tree_compress_bottom_up(Tree& t);
-// split the nodes of the last level whose wavelet norm exceeds thr; returns the number of new nodes
-int tree_refine_last_level(Tree& t, double thr);
+// split the nodes of the last level whose wavelet norm exceeds prec ||f|| 2^{-depth/2}; returns the number of new nodes
+int tree_refine_last_level(Tree& t, double prec);
 
 // fragment images of the world's block transforms (mw_kernels.cu); row-major matrices
 void world_fragments(Mra& m, const std::vector<double>& PF, const std::vector<double>& MV, const std::vector<double>& FT);

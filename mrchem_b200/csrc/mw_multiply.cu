@@ -359,17 +359,143 @@ std::vector<uint64_t> children_keys(uint64_t k) {
     return c;
 }
 
-// extend the grid of `out` by the grid of `inp` (both on one world)
+// keys of `inp` that `out` lacks, in order (one block; key order is level order): n[0] = count
+__global__ void __launch_bounds__(1024) k_grid_missing(const uint64_t* __restrict__ ikey, int ni, const uint64_t* __restrict__ hk,
+                                                       const int* __restrict__ hv, uint32_t hcap, uint64_t* add, int* n) {
+    __shared__ int wsum[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int base = 0;
+    for (int b = 0; b < ni; b += 1024) {
+        const int i = b + threadIdx.x;
+        const uint64_t k = i < ni ? ikey[i] : 0;
+        const bool f = i < ni && hlookup(hk, hv, hcap, k) < 0;
+        const unsigned m = __ballot_sync(0xffffffffu, f);
+        if (lane == 0) wsum[warp] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (f) add[base + before + __popc(m & ((1u << lane) - 1u))] = k;
+        base += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) n[0] = base;
+}
+struct GridArrays {
+    uint64_t* key;
+    double* coef;
+    double* norm2;
+    double* wnorm2;
+};
+// merge of two key-ordered node lists (the tree's n0 nodes, na new ones with zero blocks) into new arrays: one
+// block per node, whose place is its rank in its own list plus its rank in the other
+__global__ void __launch_bounds__(256) k_grid_merge(GridArrays old, int n0, const uint64_t* __restrict__ add, int na, size_t bs,
+                                                    GridArrays out) {
+    const int i = blockIdx.x;
+    const bool fresh = i >= n0;
+    const uint64_t key = fresh ? add[i - n0] : old.key[i];
+    const uint64_t* other = fresh ? old.key : add;
+    int lo = 0, hi = fresh ? n0 : na;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (other[mid] < key) lo = mid + 1;
+        else hi = mid;
+    }
+    const size_t at = (size_t)lo + (fresh ? i - n0 : i);
+    double2* d = reinterpret_cast<double2*>(out.coef + at * bs);
+    const double2* c = reinterpret_cast<const double2*>(old.coef + (size_t)(fresh ? 0 : i) * bs);
+    for (size_t e = threadIdx.x; e < bs / 2; e += blockDim.x) d[e] = fresh ? make_double2(0.0, 0.0) : c[e];
+    if (threadIdx.x == 0) {
+        out.key[at] = key;
+        out.norm2[at] = fresh ? 0.0 : old.norm2[i];
+        out.wnorm2[at] = fresh ? 0.0 : old.wnorm2[i];
+    }
+}
+// parents and first children from the hash index; the first 32 threads also find the level starts
+__global__ void k_grid_link(const uint64_t* __restrict__ key, int n, const uint64_t* __restrict__ hk, const int* __restrict__ hv,
+                            uint32_t hcap, int* parent, int* child0, int* level) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 32) {
+        const uint64_t first = (uint64_t)i << 59;
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key[mid] < first) lo = mid + 1;
+            else hi = mid;
+        }
+        level[i] = lo;
+    }
+    if (i >= n) return;
+    const uint64_t k = key[i];
+    const int d = key_depth(k);
+    long long t[3];
+    key_trans(k, t);
+    parent[i] = d > 0 ? hlookup(hk, hv, hcap, make_key(d - 1, t[0] >> 1, t[1] >> 1, t[2] >> 1)) : -1;
+    child0[i] = hlookup(hk, hv, hcap, make_key(d + 1, 2 * t[0], 2 * t[1], 2 * t[2]));
+}
+
+// Extend the grid of `out` by the grid of `inp` (both on one world).  On the device, with two read-backs (the number of
+// new nodes, the level starts) and one copy of the blocks; sorting and relinking on the host took 0.45 ms per call.
 void build_grid(Tree& out, Tree& inp) {
-    cudaStream_t s = out.mra->ctx->stream;
-    if (out.n == 0) tree_make_roots(out);
-    const std::vector<uint64_t> ko = host_keys(out, s), ki = host_keys(inp, s);
-    std::vector<uint64_t> add;
-    std::vector<uint64_t> so(ko);
-    std::sort(so.begin(), so.end());
-    for (uint64_t k : ki)
-        if (!std::binary_search(so.begin(), so.end(), k)) add.push_back(k);
-    tree_add_keys(out, add, s);
+    Ctx* ctx = out.mra->ctx;
+    cudaStream_t s = ctx->stream;
+    const size_t BS = out.mra->bsize();
+    if (out.n == 0) trees_make_roots({&out});
+    if (inp.n == 0) return;
+    uint64_t* d_add = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * (inp.n + 1));
+    int* d_n = (int*)dalloc(ctx, sizeof(int) * 33);
+    k_grid_missing<<<1, 1024, 0, s>>>(inp.key, inp.n, out.hkey, out.hval, out.hcap, d_add, d_n);
+    MWB_CUDA(cudaGetLastError());
+    ctx->launches++;
+    int na = 0;
+    readback(ctx, {{&na, d_n, sizeof(int)}});
+    if (na > 0) {
+        const int n0 = out.n, n = n0 + na;
+        Tree m;  // the merged arrays, with room to grow
+        m.mra = nullptr;
+        const int cap = n > out.cap ? std::max(n, 2 * out.cap) : out.cap;
+        m.key = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * cap);
+        m.parent = (int*)dalloc(ctx, sizeof(int) * cap);
+        m.child0 = (int*)dalloc(ctx, sizeof(int) * cap);
+        m.coef = (double*)dalloc(ctx, sizeof(double) * BS * cap);
+        m.norm2 = (double*)dalloc(ctx, sizeof(double) * cap);
+        m.wnorm2 = (double*)dalloc(ctx, sizeof(double) * cap);
+        k_grid_merge<<<n, 256, 0, s>>>(GridArrays{out.key, out.coef, out.norm2, out.wnorm2}, n0, d_add, na, BS,
+                                       GridArrays{m.key, m.coef, m.norm2, m.wnorm2});
+        MWB_CUDA(cudaGetLastError());
+        std::swap(out.key, m.key);
+        std::swap(out.parent, m.parent);
+        std::swap(out.child0, m.child0);
+        std::swap(out.coef, m.coef);
+        std::swap(out.norm2, m.norm2);
+        std::swap(out.wnorm2, m.wnorm2);
+        for (void* p : {(void*)m.key, (void*)m.parent, (void*)m.child0, (void*)m.coef, (void*)m.norm2, (void*)m.wnorm2}) dfree(ctx, p);
+        out.cap = cap;
+        out.n = n;
+        uint32_t hneed = 1024;  // hash index at most half full
+        while (hneed < 2u * (uint32_t)n) hneed <<= 1;
+        if (hneed > out.hcap) {
+            dfree(ctx, out.hkey);
+            dfree(ctx, out.hval);
+            out.hcap = hneed;
+            out.hkey = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * out.hcap);
+            out.hval = (int*)dalloc(ctx, sizeof(int) * out.hcap);
+        }
+        launch_hash_reset(out, s);
+        launch_hash_insert(out, 0, n, s);
+        k_grid_link<<<(n + 255) / 256, 256, 0, s>>>(out.key, n, out.hkey, out.hval, out.hcap, out.parent, out.child0, d_n + 1);
+        MWB_CUDA(cudaGetLastError());
+        ctx->launches += 2;
+        int level[32];
+        readback(ctx, {{level, d_n + 1, sizeof(level)}});
+        out.level_begin.clear();
+        for (int d = 0; d < 32 && (d == 0 || level[d] < n); ++d) out.level_begin.push_back(level[d]);
+        out.level_begin.push_back(n);
+    }
+    dfree(ctx, d_add);
+    dfree(ctx, d_n);
 }
 
 // split flags of the last levels of several trees in one launch: item q = (tree, node)
@@ -514,7 +640,7 @@ void refine_passes(double prec, int n, Tree** out, int max_iter, LaunchF&& launc
         }
         if (!any) break;
     }
-    trees_finish(std::vector<Tree*>(out, out + n), false, true, true, s);
+    trees_finish(std::vector<Tree*>(out, out + n), false, s);
     MWB_CUDA(cudaStreamSynchronize(s));
 }
 

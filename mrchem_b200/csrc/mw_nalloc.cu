@@ -3,8 +3,8 @@
 // Why it exists: some callers cannot allocate device memory at the moment they need a result -- code
 // running under a fixed memory budget that pre-reserves everything at start-up, a caller that has
 // handed the whole device memory pool to another framework, or a thread that must not touch the
-// allocator while other work is being recorded on its device.  mw_dot() allocates two small scratch
-// buffers from the stream-ordered pool on every call; mw_nalloc_dot() computes the same sum with its
+// allocator while other work is being recorded on its device.  mw_dot() allocates a scratch buffer
+// from the stream-ordered pool on every call; mw_nalloc_dot() computes the same sum with its
 // scratch in a fixed, file-scope device array instead.  The call itself ends with a blocking read of
 // the result into host memory, so it is not a call to place inside a CUDA graph capture.
 //
