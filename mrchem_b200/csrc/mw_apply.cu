@@ -3,8 +3,8 @@
 // A batch is any number of (output tree, operator, input tree) triples sharing one world (e.g. 32
 // orbitals with 32 Helmholtz operators).  The refinement passes run in lock-step over the batch:
 // pass d handles the depth-d output nodes of every tree with one launch per stage:
-//   1. candidates: one warp per output node walks its operator's offset list, looks the input node
-//      up in the input tree's hash index (or its leaf ancestor -> generated node) and screens it;
+//   1. candidates: a block of four warps per output node walks its operator's offset list, looks the input
+//      node up in the input tree's hash index (or its leaf ancestor -> generated node) and screens it;
 //   2. generated (scaling-only) input nodes are de-duplicated per tree and built once;
 //   3. per candidate, the number of terms that pass the screening (the triples it contributes);
 //   4. GEMM-tiled engine: the triples are expanded and sorted per output node by (term, dz, dy), and
@@ -15,6 +15,10 @@
 //   5. the contraction kernel runs one CTA per chunk; multi-chunk nodes write partial blocks that
 //      a reduction kernel adds in chunk order (deterministic), single-chunk nodes write directly;
 //   6. norms and split flags; children are appended to each tree.
+// At small sizes a pass is bound by its launches, transfers and allocations, not by the contraction: what the
+// host sends goes in one transfer, the counters are cleared by one memset, per-item arrays share one allocation,
+// and chunk and partial-slot counts travel packed through one scan (a Poisson apply at order 5, seven passes:
+// 2.11 -> 1.69 ms; at order 7: 4.35 -> 4.12 ms).
 // Results are identical to the per-node sequential order up to FP64 rounding.
 #include <cub/cub.cuh>
 
@@ -83,22 +87,26 @@ struct Chunk {
 // ---------------------------------------------------------------------------------------------
 // 1. candidates
 // ---------------------------------------------------------------------------------------------
-__global__ void k_bcand(const Item* __restrict__ items, int nitems, const BTree* __restrict__ trees, int fill,
-                        int* count, const int* offs, int* cdelta, int* csrc, uint64_t* greq_key, int* greq_leaf,
-                        int* ngreq) {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-    const int lane = threadIdx.x & 31;
-    if (w >= nitems) return;
+// One block of four warps per output node (a warp per node walked the root's 6,859 offsets in 214 dependent steps of hash
+// probes, 40 us a launch).  First pass (offs == nullptr): counts; second: the candidates in offset order, with their item.
+constexpr int kCandThreads = 128;
+__global__ void __launch_bounds__(kCandThreads) k_bcand(const Item* __restrict__ items, const BTree* __restrict__ trees,
+                                                        int* count, const int* __restrict__ offs, int* cdelta, int* csrc,
+                                                        int* cand_item, uint64_t* greq_key, int* greq_leaf, int* ngreq) {
+    __shared__ int ws[2][kCandThreads / 32];
+    const int w = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool fill = offs != nullptr;
     const Item it = items[w];
     const BTree& T = trees[it.tree];
     const int depth = T.depth;
     const long long ext[3] = {T.ext[0], T.ext[1], T.ext[2]};
     long long to[3];
     key_trans(T.okey[it.node], to);
-    int kept = 0;
+    int kept = 0, gens = 0;  // count pass: this warp's; fill pass: candidates of the earlier offsets
     const int base = fill ? offs[w] : 0;
-    for (int b0 = 0; b0 < T.nprefix; b0 += 32) {
-        const int e = b0 + lane;
+    int par = 0;
+    for (int b0 = 0; b0 < T.nprefix; b0 += kCandThreads, par ^= 1) {
+        const int e = b0 + threadIdx.x;
         int ok = 0, src = 0, leaf = -1;
         uint64_t gk = kEmptyKey;
         if (e < T.nprefix) {
@@ -131,12 +139,21 @@ __global__ void k_bcand(const Item* __restrict__ items, int nitems, const BTree*
         }
         const unsigned bal = __ballot_sync(0xffffffffu, ok);
         if (!fill) {  // the counting pass also counts the generated-node requests
-            const unsigned gb = __ballot_sync(0xffffffffu, ok && gk != kEmptyKey);
-            if (lane == 0 && gb) atomicAdd(ngreq, __popc(gb));
+            kept += __popc(bal);
+            gens += __popc(__ballot_sync(0xffffffffu, ok && gk != kEmptyKey));
+            continue;
         }
-        if (fill && ok) {
-            const int pos = base + kept + __popc(bal & ((1u << lane) - 1u));
+        if (lane == 0) ws[par][warp] = __popc(bal);
+        __syncthreads();  // (the other half of ws is free again: every warp has passed this barrier's predecessor)
+        int before = 0, all = 0;
+        for (int q = 0; q < kCandThreads / 32; ++q) {
+            if (q < warp) before += ws[par][q];
+            all += ws[par][q];
+        }
+        if (ok) {
+            const int pos = base + kept + before + __popc(bal & ((1u << lane) - 1u));
             cdelta[pos] = e;
+            cand_item[pos] = w;
             if (gk != kEmptyKey) {
                 const int r = atomicAdd(ngreq, 1);
                 greq_key[r] = gk;
@@ -146,9 +163,19 @@ __global__ void k_bcand(const Item* __restrict__ items, int nitems, const BTree*
                 csrc[pos] = src;
             }
         }
-        kept += __popc(bal);
+        kept += all;
     }
-    if (!fill && lane == 0) count[w] = kept;
+    if (fill) return;
+    if (lane == 0) {
+        ws[0][warp] = kept;
+        if (gens) atomicAdd(ngreq, gens);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int n = 0;
+        for (int q = 0; q < kCandThreads / 32; ++q) n += ws[0][q];
+        count[w] = n;
+    }
 }
 
 __global__ void k_bunique_flags(const uint64_t* __restrict__ k, int n, int* flags) {
@@ -245,38 +272,33 @@ __global__ void k_bterms(const int* __restrict__ cand_item, int ncand, const Ite
         for (int t = de.t0; t < de.t1 && !(T.terms[t].bound * nu < T.theta); ++t) ++n;
     ntrip[i] = n;
 }
-__global__ void k_cand_item(const int* __restrict__ offs, int nitems, int* cand_item) {
-    const int w = blockIdx.x;
-    if (w >= nitems) return;
-    for (int c = offs[w] + threadIdx.x; c < offs[w + 1]; c += blockDim.x) cand_item[c] = w;
-}
 // greedy cut of each node's candidates into chunks of at most `limit` triples (whole
 // candidates; at least one chunk per node so that every output block gets written)
+// counts and their prefix sums are packed: chunks in the low word, partial slots (of nodes with several chunks) in the high
+__device__ __forceinline__ unsigned long long pack_chunks(int nch) {
+    return (unsigned)nch | ((unsigned long long)(nch > 1 ? nch : 0) << 32);
+}
 __global__ void k_bchunks(const int* __restrict__ offs, int nitems, const int* __restrict__ ntrip, int limit, int fill,
-                          int* nchunk, const int* __restrict__ choff, const int* __restrict__ slotoff, Chunk* chunks) {
+                          unsigned long long* nchunk, const unsigned long long* __restrict__ choff, Chunk* chunks) {
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= nitems) return;
     const int c0 = offs[w], c1 = offs[w + 1];
     int nch = 0, acc = 0, start = c0;
-    const int multi = fill ? (choff[w + 1] - choff[w] > 1) : 0;
+    const int at = fill ? (int)(uint32_t)choff[w] : 0, slot = fill ? (int)(choff[w] >> 32) : 0;
+    const int multi = fill ? ((int)(uint32_t)choff[w + 1] - at > 1) : 0;
     for (int c = c0; c < c1; ++c) {
         const int t = ntrip[c];
         if (acc > 0 && acc + t > limit) {
-            if (fill) chunks[choff[w] + nch] = Chunk{w, start, c, multi ? slotoff[w] + nch : -1};
+            if (fill) chunks[at + nch] = Chunk{w, start, c, multi ? slot + nch : -1};
             ++nch;
             acc = 0;
             start = c;
         }
         acc += t;
     }
-    if (fill) chunks[choff[w] + nch] = Chunk{w, start, c1, multi ? slotoff[w] + nch : -1};
+    if (fill) chunks[at + nch] = Chunk{w, start, c1, multi ? slot + nch : -1};
     ++nch;
-    if (!fill) nchunk[w] = nch;
-}
-__global__ void k_multi_slots(const int* __restrict__ nchunk, int nitems, int* nslot) {
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= nitems) return;
-    nslot[w] = nchunk[w] > 1 ? nchunk[w] : 0;
+    if (!fill) nchunk[w] = pack_chunks(nch);
 }
 // triples of the line-ordered contraction: candidate c contributes its first ntrip[c] term entries,
 // at positions toff[c] ..; key = item << 32 | term << 20 | line rank (dz rank << 10 | dy rank),
@@ -314,18 +336,19 @@ __global__ void k_texpand(const int* __restrict__ offs, const int* __restrict__ 
 // node: the plane starts of 32 triples at a time come from one ballot, and the cut walks the planes
 // in order (a plane's size is known when the next one starts)
 __global__ void k_tchunks(const int* __restrict__ offs, const int* __restrict__ toff, int nitems,
-                          const unsigned long long* __restrict__ key, int limit, int fill, int* nchunk,
-                          const int* __restrict__ choff, const int* __restrict__ slotoff, Chunk* chunks) {
+                          const unsigned long long* __restrict__ key, int limit, int fill, unsigned long long* nchunk,
+                          const unsigned long long* __restrict__ choff, Chunk* chunks) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= nitems) return;  // uniform over the warp
     const int t0 = toff[offs[w]], t1 = toff[offs[w + 1]];
     int nch = 0, acc = 0, start = t0, ps = -1;  // ps: start of the plane being measured
-    const int multi = fill ? (choff[w + 1] - choff[w] > 1) : 0;
+    const int at = fill ? (int)(uint32_t)choff[w] : 0, slot = fill ? (int)(choff[w] >> 32) : 0;
+    const int multi = fill ? ((int)(uint32_t)choff[w + 1] - at > 1) : 0;
     auto plane_done = [&](int end) {  // plane [ps, end) is complete: cut before it if it overflows
         const int sz = end - ps;
         if (acc > 0 && acc + sz > limit) {
-            if (fill && lane == 0) chunks[choff[w] + nch] = Chunk{w, start, ps, multi ? slotoff[w] + nch : -1};
+            if (fill && lane == 0) chunks[at + nch] = Chunk{w, start, ps, multi ? slot + nch : -1};
             ++nch;
             acc = 0;
             start = ps;
@@ -347,9 +370,9 @@ __global__ void k_tchunks(const int* __restrict__ offs, const int* __restrict__ 
         }
     }
     if (ps >= 0) plane_done(t1);
-    if (fill && lane == 0) chunks[choff[w] + nch] = Chunk{w, start, t1, multi ? slotoff[w] + nch : -1};
+    if (fill && lane == 0) chunks[at + nch] = Chunk{w, start, t1, multi ? slot + nch : -1};
     ++nch;
-    if (!fill && lane == 0) nchunk[w] = nch;
+    if (!fill && lane == 0) nchunk[w] = pack_chunks(nch);
 }
 // FP32 block images for the line-ordered contraction: image row a (a < 2k) holds X[a][b + P c] of the
 // node block (P = 2k rounded up to 4; zero where b or c >= 2k), so that a CTA stages a block with
@@ -1177,13 +1200,13 @@ __global__ void k_chunk_len(const Chunk* __restrict__ chunks, int n, int* __rest
 
 // add the partial blocks of a multi-chunk node in chunk order; write block and norms
 template <int K>
-__global__ void __launch_bounds__(256) k_breduce(const Chunk* __restrict__ chunks, const int* __restrict__ choff,
-                                                 const int* __restrict__ multi_items, const Item* __restrict__ items,
-                                                 const BTree* __restrict__ trees, const double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) k_breduce(const Chunk* __restrict__ chunks, const unsigned long long* __restrict__ choff,
+                                                 const Item* __restrict__ items, const BTree* __restrict__ trees,
+                                                 const double* __restrict__ partials) {
     using G = Geo<K>;
     __shared__ double red[64];
-    const int w = multi_items ? multi_items[blockIdx.x] : blockIdx.x;  // no list: one block per item
-    const int cb = choff[w], ce = choff[w + 1];
+    const int w = blockIdx.x;
+    const int cb = (int)(uint32_t)choff[w], ce = (int)(uint32_t)choff[w + 1];
     if (ce - cb < 2) return;  // a single chunk wrote the node itself
     const Item it = items[w];
     const BTree& TR = trees[it.tree];
@@ -1206,21 +1229,19 @@ __global__ void __launch_bounds__(256) k_breduce(const Chunk* __restrict__ chunk
 // ---------------------------------------------------------------------------------------------
 // 6. per-tree root norms, split flags
 // ---------------------------------------------------------------------------------------------
-__global__ void k_tree_item_norm2(const Item* __restrict__ items, const int* __restrict__ item_off,
-                                  const BTree* __restrict__ trees, double* out) {
+// per entry: the square norm of its nodes, and a root entry's split threshold from it: prec g0 with g0 the root level's
+// norm (the same operations as the host's prec g0 2^(-depth/2) at depth 0)
+__global__ void k_root_thr(const Item* __restrict__ items, const int* __restrict__ item_off, BTree* trees,
+                           const double* __restrict__ prec, double* out) {
     __shared__ double red[64];
     const int t = blockIdx.x;
     double s = 0.0, d = 0.0;
     for (int i = item_off[t] + threadIdx.x; i < item_off[t + 1]; i += blockDim.x) s += trees[t].onorm2[items[i].node];
     block_sum2(s, d, red);
-    if (threadIdx.x == 0) out[t] = s;
-}
-// split thresholds of the root entries from their output norms: prec g0 with g0 the square root of the
-// root level's square norm (the same operations as the host's prec g0 2^(-depth/2) at depth 0)
-__global__ void k_root_thr(BTree* trees, const double* __restrict__ g, const double* __restrict__ prec, int nt) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nt || trees[t].depth != 0) return;
-    const double g0 = sqrt(g[t]);
+    if (threadIdx.x != 0) return;
+    out[t] = s;
+    if (trees[t].depth != 0) return;
+    const double g0 = sqrt(s);
     trees[t].thr = (prec[t] > 0.0 && g0 > 0.0) ? prec[t] * g0 : INFINITY;
 }
 __global__ void k_bsplit_flags(const Item* __restrict__ items, int nitems, const BTree* __restrict__ trees,
@@ -1248,14 +1269,10 @@ static bool contraction_pencil() {
     return v;
 }
 
+// exclusive sum of d_in[0 .. n) into d_out[0 .. n] (the total lands in d_out[n]; d_in[n] is read, its value is not
+// used); no host read-back
 template <typename T>
-static T* upload(Ctx* ctx, const std::vector<T>& v) {
-    T* d = (T*)dalloc(ctx, sizeof(T) * std::max<size_t>(1, v.size()));
-    upload_bytes(ctx, d, v.data(), sizeof(T) * v.size());
-    return d;
-}
-// exclusive sum of d_in[0 .. n] into d_out (the total lands in d_out[n]); no host read-back
-static void scan_only(Ctx* ctx, const int* d_in, int* d_out, int n) {
+static void scan_only(Ctx* ctx, const T* d_in, T* d_out, int n) {
     size_t tmp = 0;
     MWB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, d_in, d_out, n + 1, ctx->stream));
     void* d_tmp = dalloc(ctx, tmp);
@@ -1375,19 +1392,41 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     const int ni = (int)items.size();
     bp.nitems = ni;
     if (ni == 0) return;
-    Item* d_items = upload(ctx, items);
-    BTree* d_trees = upload(ctx, bt);
-    int* d_item_off = upload(ctx, item_off);
+    // everything the pass takes from the host, in one transfer
+    std::vector<double> precs(nt);
+    std::vector<ImgSrc> srcs(nt);
+    bool any_root = false;
+    for (int t = 0; t < nt; ++t) {
+        precs[t] = bp.trees[t].prec;
+        srcs[t] = ImgSrc{bp.trees[t].inp->coef, bt[t].img_base, bt[t].img_lb, bt[t].img_le - bt[t].img_lb};
+        any_root |= bp.trees[t].depth == 0;
+    }
+    UploadPack up(ctx);
+    const size_t o_items = up.add(items), o_trees = up.add(bt), o_off = up.add(item_off), o_prec = up.add(precs), o_src = up.add(srcs);
+    char* d_up = up.send();
+    Item* d_items = reinterpret_cast<Item*>(d_up + o_items);
+    BTree* d_trees = reinterpret_cast<BTree*>(d_up + o_trees);
+    int* d_item_off = reinterpret_cast<int*>(d_up + o_off);
+    const double* d_prec = reinterpret_cast<const double*>(d_up + o_prec);
+    const ImgSrc* d_srcs = reinterpret_cast<const ImgSrc*>(d_up + o_src);
+    // the pass's counters and flags, cleared together
+    struct Counters {
+        unsigned long long ntrip;  // contracted triples
+        int kerr, pad;             // set by the contraction on a wait timeout
+        int ngreq, ngreq2, terr;   // generated-node requests (counted, numbered), the expansion's error word
+    };
+    Counters* d_cnt = (Counters*)dalloc(ctx, sizeof(Counters));
+    MWB_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(Counters), s));
+    unsigned long long* d_ntrip_tot = &d_cnt->ntrip;
+    int *d_kerr = &d_cnt->kerr, *d_ngreq = &d_cnt->ngreq, *d_terr = &d_cnt->terr;
 
-    // 1. candidates
-    int* d_count = (int*)dalloc(ctx, sizeof(int) * (ni + 1));
-    int* d_offs = (int*)dalloc(ctx, sizeof(int) * (ni + 1));
-    int* d_ngreq = (int*)dalloc(ctx, sizeof(int));
-    MWB_CUDA(cudaMemsetAsync(d_count, 0, sizeof(int) * (ni + 1), s));
-    MWB_CUDA(cudaMemsetAsync(d_ngreq, 0, sizeof(int), s));
-    const int cblocks = (ni * 32 + 255) / 256;
-    k_bcand<<<cblocks, 256, 0, s>>>(d_items, ni, d_trees, 0, d_count, nullptr, nullptr, nullptr, nullptr, nullptr,
-                                    d_ngreq);
+    // 1. candidates; per item: candidate and chunk counts with their sums, split flags
+    unsigned long long* d_nchunk = (unsigned long long*)dalloc(ctx, (sizeof(unsigned long long) * 2 + sizeof(int) * 3) * (ni + 1));
+    unsigned long long* d_choff = d_nchunk + (ni + 1);
+    int* d_count = reinterpret_cast<int*>(d_choff + (ni + 1));
+    int* d_offs = d_count + (ni + 1);
+    int* d_sflags = d_offs + (ni + 1);
+    k_bcand<<<ni, kCandThreads, 0, s>>>(d_items, d_trees, d_count, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, d_ngreq);
     MWB_CUDA(cudaGetLastError());
     count(ctx);
     scan_only(ctx, d_count, d_offs, ni);
@@ -1395,15 +1434,17 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     readback(ctx, {{&tot0[0], d_offs + ni, sizeof(int)}, {&tot0[1], d_ngreq, sizeof(int)}});
     const int ncand = tot0[0];
     const int ngreq = tot0[1];
-    MWB_CUDA(cudaMemsetAsync(d_ngreq, 0, sizeof(int), s));  // the fill pass numbers the requests again
     const int ncap = std::max(1, ncand);
-    int* d_cdelta = (int*)dalloc(ctx, sizeof(int) * ncap);
-    int* d_csrc = (int*)dalloc(ctx, sizeof(int) * ncap);
-    uint64_t* d_greq_key = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * ncap);
-    int* d_greq_leaf = (int*)dalloc(ctx, sizeof(int) * ncap);
+    uint64_t* d_greq_key = (uint64_t*)dalloc(ctx, (sizeof(uint64_t) + 6 * sizeof(int)) * (ncap + 1));
+    int* d_greq_leaf = reinterpret_cast<int*>(d_greq_key + (ncap + 1));
+    int* d_cdelta = d_greq_leaf + (ncap + 1);
+    int* d_csrc = d_cdelta + (ncap + 1);
+    int* d_cand_item = d_csrc + (ncap + 1);
+    int* d_ntrip = d_cand_item + (ncap + 1);
+    int* d_toff = d_ntrip + (ncap + 1);
     if (ncand > 0) {
-        k_bcand<<<cblocks, 256, 0, s>>>(d_items, ni, d_trees, 1, d_count, d_offs, d_cdelta, d_csrc, d_greq_key,
-                                        d_greq_leaf, d_ngreq);
+        k_bcand<<<ni, kCandThreads, 0, s>>>(d_items, d_trees, d_count, d_offs, d_cdelta, d_csrc, d_cand_item, d_greq_key,
+                                            d_greq_leaf, &d_cnt->ngreq2);
         MWB_CUDA(cudaGetLastError());
         count(ctx);
     }
@@ -1424,7 +1465,6 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
         dfree(ctx, d_tmp);
         int* d_flags = (int*)dalloc(ctx, sizeof(int) * (ngreq + 1));
         int* d_pos = (int*)dalloc(ctx, sizeof(int) * (ngreq + 1));
-        MWB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (ngreq + 1), s));
         k_bunique_flags<<<(ngreq + 255) / 256, 256, 0, s>>>(d_sk, ngreq, d_flags);
         nu = scan_total(ctx, d_flags, d_pos, ngreq);
         d_ukey = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * nu);
@@ -1466,39 +1506,24 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     lined = fp64 || hyb || lined32;
     MWB_DISPATCH_K(K, L_ENG)
 #undef L_ENG
-    int* d_cand_item = (int*)dalloc(ctx, sizeof(int) * ncap);
-    int* d_ntrip = (int*)dalloc(ctx, sizeof(int) * (ncap + 1));
-    MWB_CUDA(cudaMemsetAsync(d_ntrip, 0, sizeof(int) * (ncap + 1), s));
     if (ncand > 0) {
-        k_cand_item<<<ni, 128, 0, s>>>(d_offs, ni, d_cand_item);
         k_bterms<<<(ncand + 255) / 256, 256, 0, s>>>(d_cand_item, ncand, d_items, d_trees, d_cdelta, d_csrc, d_gnorm2,
                                                      d_ntrip);
         MWB_CUDA(cudaGetLastError());
-        count(ctx, 2);
+        count(ctx);
     }
-    int* d_nchunk = (int*)dalloc(ctx, sizeof(int) * (ni + 1));
-    int* d_choff = (int*)dalloc(ctx, sizeof(int) * (ni + 1));
-    int* d_nslot = (int*)dalloc(ctx, sizeof(int) * (ni + 1));
-    int* d_slotoff = (int*)dalloc(ctx, sizeof(int) * (ni + 1));
-    MWB_CUDA(cudaMemsetAsync(d_nchunk, 0, sizeof(int) * (ni + 1), s));
-    MWB_CUDA(cudaMemsetAsync(d_nslot, 0, sizeof(int) * (ni + 1), s));
     const int chunk_limit = ctx->chunk_triples[std::min(std::max(bp.precision, 0), 3)];
-    int* d_toff = nullptr;
-    int* d_terr = nullptr;
-    unsigned long long *d_tkey = nullptr, *d_tval = nullptr;
+    unsigned long long *d_tri = nullptr, *d_tkey = nullptr, *d_tval = nullptr;
     void* d_ximg = nullptr;
     int nchunks = 0, nslots = 0;
     Chunk* d_chunks = nullptr;
     if (lined) {
-        d_terr = (int*)dalloc(ctx, sizeof(int));
-        MWB_CUDA(cudaMemsetAsync(d_terr, 0, sizeof(int), s));
-        d_toff = (int*)dalloc(ctx, sizeof(int) * (ncap + 1));
         const int ntri = scan_total(ctx, d_ntrip, d_toff, ncand);
         const size_t tcap = (size_t)std::max(1, ntri);
-        unsigned long long* d_tkey_in = (unsigned long long*)dalloc(ctx, sizeof(unsigned long long) * tcap);
-        unsigned long long* d_tval_in = (unsigned long long*)dalloc(ctx, sizeof(unsigned long long) * tcap);
-        d_tkey = (unsigned long long*)dalloc(ctx, sizeof(unsigned long long) * tcap);
-        d_tval = (unsigned long long*)dalloc(ctx, sizeof(unsigned long long) * tcap);
+        d_tri = (unsigned long long*)dalloc(ctx, 4 * sizeof(unsigned long long) * tcap);
+        unsigned long long *d_tkey_in = d_tri, *d_tval_in = d_tri + tcap;
+        d_tkey = d_tri + 2 * tcap;
+        d_tval = d_tri + 3 * tcap;
         if (ntri > 0) {
             k_texpand<<<(ncand + 255) / 256, 256, 0, s>>>(d_offs, d_cand_item, ncand, d_items, d_trees, d_cdelta, d_ntrip,
                                                           d_toff, d_csrc, d_tkey_in, d_tval_in, d_terr);
@@ -1512,30 +1537,20 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
             dfree(ctx, d_tmp);
             count(ctx, 2);
         }
-        dfree(ctx, d_tkey_in);
-        dfree(ctx, d_tval_in);
-        k_tchunks<<<(ni * 32 + 127) / 128, 128, 0, s>>>(d_offs, d_toff, ni, d_tkey, chunk_limit, 0, d_nchunk, nullptr,
-                                                   nullptr, nullptr);
-        k_multi_slots<<<(ni + 127) / 128, 128, 0, s>>>(d_nchunk, ni, d_nslot);
-        count(ctx, 2);
+        k_tchunks<<<(ni * 32 + 127) / 128, 128, 0, s>>>(d_offs, d_toff, ni, d_tkey, chunk_limit, 0, d_nchunk, nullptr, nullptr);
+        count(ctx);
         scan_only(ctx, d_nchunk, d_choff, ni);
-        scan_only(ctx, d_nslot, d_slotoff, ni);
-        int tot[3] = {0, 0, 0};  // chunks, partial slots, the expansion's error word: one read-back
-        readback(ctx, {{&tot[0], d_choff + ni, sizeof(int)}, {&tot[1], d_slotoff + ni, sizeof(int)},
-                       {&tot[2], d_terr, sizeof(int)}});
-        if (tot[2] != 0) throw Error(-3, "input tree nodes are not in level order");
-        nchunks = tot[0];
-        nslots = tot[1];
+        unsigned long long tot = 0;  // chunks, partial slots
+        int terr = 0;                // the expansion's error word: one read-back
+        readback(ctx, {{&tot, d_choff + ni, sizeof(tot)}, {&terr, d_terr, sizeof(int)}});
+        if (terr != 0) throw Error(-3, "input tree nodes are not in level order");
+        nchunks = (int)(uint32_t)tot;
+        nslots = (int)(tot >> 32);
         d_chunks = (Chunk*)dalloc(ctx, sizeof(Chunk) * std::max(1, nchunks));
-        k_tchunks<<<(ni * 32 + 127) / 128, 128, 0, s>>>(d_offs, d_toff, ni, d_tkey, chunk_limit, 1, d_nchunk, d_choff,
-                                                   d_slotoff, d_chunks);
+        k_tchunks<<<(ni * 32 + 127) / 128, 128, 0, s>>>(d_offs, d_toff, ni, d_tkey, chunk_limit, 1, d_nchunk, d_choff, d_chunks);
         // block images of this pass's input nodes (the entries' depth levels) and generated nodes
         const long long nimg = nreal + nu;
         if (nimg > 0) {
-            std::vector<ImgSrc> srcs(nt);
-            for (int t = 0; t < nt; ++t)
-                srcs[t] = ImgSrc{bp.trees[t].inp->coef, bt[t].img_base, bt[t].img_lb, bt[t].img_le - bt[t].img_lb};
-            ImgSrc* d_srcs = upload(ctx, srcs);
 #define L_IMG(KK)                                                                                               \
     {                                                                                                           \
         if (hyb) {                                                                                              \
@@ -1554,22 +1569,17 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
 #undef L_IMG
             MWB_CUDA(cudaGetLastError());
             count(ctx);
-            dfree(ctx, d_srcs);
         }
     } else {
-        k_bchunks<<<(ni + 127) / 128, 128, 0, s>>>(d_offs, ni, d_ntrip, chunk_limit, 0, d_nchunk, nullptr, nullptr,
-                                                   nullptr);
-        k_multi_slots<<<(ni + 127) / 128, 128, 0, s>>>(d_nchunk, ni, d_nslot);
-        count(ctx, 2);
+        k_bchunks<<<(ni + 127) / 128, 128, 0, s>>>(d_offs, ni, d_ntrip, chunk_limit, 0, d_nchunk, nullptr, nullptr);
+        count(ctx);
         scan_only(ctx, d_nchunk, d_choff, ni);
-        scan_only(ctx, d_nslot, d_slotoff, ni);
-        int tot[2] = {0, 0};
-        readback(ctx, {{&tot[0], d_choff + ni, sizeof(int)}, {&tot[1], d_slotoff + ni, sizeof(int)}});
-        nchunks = tot[0];
-        nslots = tot[1];
+        unsigned long long tot = 0;
+        readback(ctx, {{&tot, d_choff + ni, sizeof(tot)}});
+        nchunks = (int)(uint32_t)tot;
+        nslots = (int)(tot >> 32);
         d_chunks = (Chunk*)dalloc(ctx, sizeof(Chunk) * std::max(1, nchunks));
-        k_bchunks<<<(ni + 127) / 128, 128, 0, s>>>(d_offs, ni, d_ntrip, chunk_limit, 1, d_nchunk, d_choff, d_slotoff,
-                                                   d_chunks);
+        k_bchunks<<<(ni + 127) / 128, 128, 0, s>>>(d_offs, ni, d_ntrip, chunk_limit, 1, d_nchunk, d_choff, d_chunks);
     }
     MWB_CUDA(cudaGetLastError());
     count(ctx);
@@ -1594,9 +1604,6 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     }
 
     // 5. contraction + reduction of multi-chunk nodes
-    unsigned long long* d_ntrip_tot = (unsigned long long*)dalloc(ctx, 2 * sizeof(unsigned long long));
-    int* d_kerr = reinterpret_cast<int*>(d_ntrip_tot + 1);  // set by the tensor-core kernel on a wait timeout
-    MWB_CUDA(cudaMemsetAsync(d_ntrip_tot, 0, 2 * sizeof(unsigned long long), s));
     if (ctx->prof) MWB_CUDA(cudaEventRecord(ctx->ev0, s));
 #define L_AP(KK)                                                                                             \
     {                                                                                                        \
@@ -1643,7 +1650,7 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     ctx->apply_launches++;
     ctx->apply_ctas += nchunks;
     if (nslots > 0) {  // one block per item; items whose node took one chunk leave at once
-#define L_RED(KK) k_breduce<KK><<<ni, 256, 0, s>>>(d_chunks, d_choff, nullptr, d_items, d_trees, d_partials);
+#define L_RED(KK) k_breduce<KK><<<ni, 256, 0, s>>>(d_chunks, d_choff, d_items, d_trees, d_partials);
         MWB_DISPATCH_K(K, L_RED)
 #undef L_RED
         MWB_CUDA(cudaGetLastError());
@@ -1651,21 +1658,13 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     }
 
     // 6. root norms and thresholds (root entries), split flags; one read-back for the pass's results
-    bool any_root = false;
-    for (int t = 0; t < nt; ++t) any_root |= bp.trees[t].depth == 0;
     double* d_g = nullptr;
     if (any_root) {
         d_g = (double*)dalloc(ctx, sizeof(double) * nt);
-        std::vector<double> precs(nt);
-        for (int t = 0; t < nt; ++t) precs[t] = bp.trees[t].prec;
-        double* d_prec = upload(ctx, precs);
-        k_tree_item_norm2<<<nt, 256, 0, s>>>(d_items, d_item_off, d_trees, d_g);
-        k_root_thr<<<(nt + 127) / 128, 128, 0, s>>>(d_trees, d_g, d_prec, nt);
+        k_root_thr<<<nt, 256, 0, s>>>(d_items, d_item_off, d_trees, d_prec, d_g);
         MWB_CUDA(cudaGetLastError());
-        count(ctx, 2);
-        dfree(ctx, d_prec);
+        count(ctx);
     }
-    int* d_sflags = (int*)dalloc(ctx, sizeof(int) * (ni + 1));
     k_bsplit_flags<<<(ni + 255) / 256, 256, 0, s>>>(d_items, ni, d_trees, d_sflags);
     MWB_CUDA(cudaGetLastError());
     count(ctx);
@@ -1689,10 +1688,8 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
         for (int i = item_off[t]; i < item_off[t + 1]; ++i)
             if (sflags[i]) bp.split_lists[t].push_back(items[i].node);
     dfree(ctx, d_g);
-    for (void* p : std::initializer_list<void*>{d_items, d_trees, d_item_off, d_count, d_offs, d_ngreq, d_cdelta, d_csrc,
-                                                d_greq_key, d_greq_leaf, d_ukey, d_uleaf, d_gblk, d_gnorm2, d_cand_item,
-                                                d_ntrip, d_nchunk, d_choff, d_nslot, d_slotoff, d_chunks, d_partials,
-                                                d_ntrip_tot, d_sflags, d_toff, d_tkey, d_tval, d_terr, d_ximg})
+    for (void* p : std::initializer_list<void*>{d_up, d_cnt, d_nchunk, d_greq_key, d_ukey, d_uleaf, d_gblk, d_gnorm2, d_chunks,
+                                                d_partials, d_tri, d_ximg})
         dfree(ctx, p);
     bp.nchunks = nchunks;
     bp.nslots = nslots;

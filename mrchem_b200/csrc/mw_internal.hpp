@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -182,6 +183,28 @@ void dfree(Ctx* ctx, void* p);
 void upload_bytes(Ctx* ctx, void* dst, const void* src, size_t bytes);
 // the same on stream s: through the arena when s is the context's stream, else a pageable copy on s
 void upload_bytes(Ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes);
+// several small host arrays to the device in one transfer: add() returns an array's offset, send() a device buffer of all
+// of them (the caller frees it); the arrays may go when send() returns
+class UploadPack {
+public:
+    explicit UploadPack(Ctx* ctx) : ctx_(ctx) {}
+    template <typename T>
+    size_t add(const std::vector<T>& v) {
+        const size_t at = (buf_.size() + 15) & ~(size_t)15;
+        buf_.resize(at + sizeof(T) * v.size());
+        if (!v.empty()) std::memcpy(buf_.data() + at, v.data(), sizeof(T) * v.size());
+        return at;
+    }
+    char* send() {
+        char* d = (char*)dalloc(ctx_, buf_.size());
+        upload_bytes(ctx_, d, buf_.data(), buf_.size());
+        return d;
+    }
+
+private:
+    Ctx* ctx_;
+    std::vector<char> buf_;
+};
 // device-to-device copy on the context's stream by a copy kernel (the DMA engines may be queued with
 // large host transfers of other contexts)
 void device_copy(Ctx* ctx, void* dst, const void* src, size_t bytes);

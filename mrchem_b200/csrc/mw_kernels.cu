@@ -618,10 +618,11 @@ void trees_finish(const std::vector<Tree*>& ts, bool sumup, cudaStream_t s) {
     if (items.empty()) return;
     std::vector<TView> views;
     for (Tree* t : ts) views.push_back(view(*t));
-    int2* d_items = (int2*)dalloc(ctx, sizeof(int2) * items.size());
-    TView* d_views = (TView*)dalloc(ctx, sizeof(TView) * views.size());
-    upload_bytes(ctx, d_items, items.data(), sizeof(int2) * items.size());
-    upload_bytes(ctx, d_views, views.data(), sizeof(TView) * views.size());
+    UploadPack up(ctx);
+    const size_t o_items = up.add(items), o_views = up.add(views);
+    char* d_up = up.send();
+    const int2* d_items = reinterpret_cast<const int2*>(d_up + o_items);
+    const TView* d_views = reinterpret_cast<const TView*>(d_up + o_views);
     WorldGeo wg = world_geo(m);
     auto level = [&](int mode, int d) {
         const int n = lvl_off[d + 1] - lvl_off[d];
@@ -649,8 +650,7 @@ void trees_finish(const std::vector<Tree*>& ts, bool sumup, cudaStream_t s) {
         MWB_CUDA(cudaGetLastError());
         count(ctx);
     }
-    dfree(ctx, d_items);
-    dfree(ctx, d_views);
+    dfree(ctx, d_up);
 }
 
 void launch_node_norms(Tree& t, int begin, int end, cudaStream_t s) {
@@ -721,10 +721,11 @@ void trees_add_children(const std::vector<Tree*>& ts, const std::vector<std::vec
         }
         off += ns;
     }
-    int* d_buf = (int*)dalloc(ctx, sizeof(int) * buf.size());
-    ChildTree* d_ct = (ChildTree*)dalloc(ctx, sizeof(ChildTree) * ct.size());
-    upload_bytes(ctx, d_buf, buf.data(), sizeof(int) * buf.size());
-    upload_bytes(ctx, d_ct, ct.data(), sizeof(ChildTree) * ct.size());
+    UploadPack up(ctx);
+    const size_t o_buf = up.add(buf), o_ct = up.add(ct);
+    char* d_up = up.send();
+    const int* d_buf = reinterpret_cast<const int*>(d_up + o_buf);
+    const ChildTree* d_ct = reinterpret_cast<const ChildTree*>(d_up + o_ct);
     k_make_children_many<<<(int)((tot + 127) / 128), 128, 0, s>>>(d_ct, d_buf + tot, d_buf, (int)tot);
     MWB_CUDA(cudaGetLastError());
     count(ctx);
@@ -735,8 +736,7 @@ void trees_add_children(const std::vector<Tree*>& ts, const std::vector<std::vec
         t.n += 8 * ns;
         t.level_begin.push_back(t.n);
     }
-    dfree(ctx, d_buf);  // stream-ordered; the host vectors were staged by upload_bytes
-    dfree(ctx, d_ct);
+    dfree(ctx, d_up);  // stream-ordered; the host vectors were staged
 }
 
 double reduce_leaf_norm2(Tree& t, cudaStream_t s) {
@@ -943,17 +943,17 @@ void trees_make_roots(const std::vector<Tree*>& ts) {
         rt.push_back(RootTree{t->key, t->parent, t->child0, t->norm2, t->wnorm2, t->hkey, t->hval, t->hcap});
         maxcap = std::max(maxcap, t->hcap);
     }
-    uint64_t* d_rk = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * nroot);
-    RootTree* d_rt = (RootTree*)dalloc(ctx, sizeof(RootTree) * rt.size());
-    upload_bytes(ctx, d_rk, keys.data(), sizeof(uint64_t) * nroot);
-    upload_bytes(ctx, d_rt, rt.data(), sizeof(RootTree) * rt.size());
+    UploadPack up(ctx);
+    const size_t o_rk = up.add(keys), o_rt = up.add(rt);
+    char* d_up = up.send();
+    const uint64_t* d_rk = reinterpret_cast<const uint64_t*>(d_up + o_rk);
+    const RootTree* d_rt = reinterpret_cast<const RootTree*>(d_up + o_rt);
     const unsigned nt = (unsigned)rt.size();
     k_hash_reset_many<<<dim3(std::min<uint32_t>((maxcap + 255) / 256, 1024), nt), 256, 0, s>>>(d_rt);
     k_roots_many<<<dim3((nroot + 255) / 256, nt), 256, 0, s>>>(d_rt, d_rk, nroot);
     MWB_CUDA(cudaGetLastError());
     count(ctx, 2);
-    dfree(ctx, d_rk);
-    dfree(ctx, d_rt);
+    dfree(ctx, d_up);
     for (Tree* t : ts) {
         t->n = nroot;
         t->level_begin = {0, nroot};
