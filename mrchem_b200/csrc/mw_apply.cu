@@ -729,64 +729,72 @@ __global__ void __launch_bounds__(ACfg<K, R>::NT, 1)
 //     data operand in shared memory as k-major rows (row = contracted index, columns = the other two
 //     indices), and every step writes its result in the row layout the next step reads:
 //        X [a][b + P c]  --x-->  T1 [b][a' + P c]  --y-->  T2 [c][a' + P b']  --z-->  acc [c'][a' + P b']
-//     (P = 2k rounded up to a multiple of 4, padding zero).  A thread owns an MT x NT tile of every
-//     step; a warp is 4 row tiles x 8 column tiles, so per contracted index a warp reads MT broadcast
-//     operator values and NT data values per lane and issues MT*NT FMAs.  Operators are staged
+//     (P = 2k rounded up to a multiple of 4, padding zero).  A thread owns MT rows of NH groups of GW
+//     consecutive columns, the groups P/NH slices apart; per contracted index it reads MT operator and
+//     NT = NH GW data values with 8- and 16-byte loads and issues MT*NT/2 packed FMAs.
+//     Two limits bound the tile: a warp is tied to its SM sub-partition, so the tiles have to give all four
+//     the same work; and a shared-memory load delivers 128 bytes a clock to the registers of the whole SM,
+//     broadcast or not, so a tile costs MT*NT FMA clocks of its sub-partition and 4 (MT + NT) load clocks
+//     of the SM.  P = 20: 5 x 10 tiles were 160 threads in 5 warps, two of them on one sub-partition (density
+//     potential at order 9: 39.7 ms contracting); 4 x 8 in 8 warps is even but bound by the loads (33.9 ms: loads
+//     busy 78 %, FMA pipe 58 % of active clocks); 4 x 16 in 125 of 128 threads 31.7 ms; 10 x 8 in 100 of 128
+//     threads 33.2 ms.  P = 12: 4 x 4 in 108 of 128 threads (3 x 6 in 96 before: 1.52 -> 1.38 ms at k = 6);
+//     P = 16 and 24 divide evenly at 4 x 8 and 6 x 6 (wider loads: 2.94 -> 2.25 at k = 8, 10.1 -> 8.3 at k = 12).
+//     Operators are staged
 //     transposed (At[k][o] = M[o][k]); the z step uses the beta-scaled tables.
 //     Below the root the s->s block is taken out with three k x k x k GEMMs on the top-left k x k
-//     operator blocks (U1, U2, Uc); the owners of the z tiles subtract Uc one phase later.
-//     Generated inputs (scaling part only) contract over k instead of 2k and skip the tiles that
-//     only see their zero wavelet part.
+//     operator blocks (U1, U2, Uc), each thread one column and all or half of the rows; the owners of the z tiles
+//     subtract Uc one phase later.
+//     Generated inputs (scaling part only) contract over k instead of 2k and skip the column groups that
+//     only see their zero wavelet part: the upper half of every thread's groups in the x and y steps.
 //     Barriers per term: after x, after y.  Shared-memory hazards across terms are resolved by
 //     loading each operator in a phase that the two barriers separate from its readers:
 //     Mx(t+1) and Mz(t) during y(t), My(t+1) during z(t).
 // ---------------------------------------------------------------------------------------------
-__host__ __device__ constexpr int gcfg_nc(int k, int nthr) {
-    int d = 1;
-    while (d < k && (k % d != 0 || 2 * k * k / d > nthr)) ++d;
-    return d;
-}
-// Row-stride padding of the T1 (x-step output) and T2 (y-step output) buffers, chosen per basis size
-// so that the epilogue stores of a warp fall into few banks (counted wavefronts per step, consecutive
-// column tiles per warp).  The T1 stride matches the 16-byte staging rows (T1 replaces a staged block at
-// a line's end), which leaves two-way conflicts on the once-per-line T1 stores at k = 9, 10.
-__host__ __device__ constexpr int gcfg_pad1(int k) {
-    return (k == 5 || k == 6 || k == 9 || k == 10 || k == 11 || k == 12) ? 4 : 0;
-}
-__host__ __device__ constexpr int gcfg_pad2(int k) {
-    return (k == 5 || k == 6 || k == 9 || k == 10) ? 0 : (k == 11 || k == 12) ? 8 : 2;
-}
-
 template <int K>
 struct GCfg {
     static constexpr int K2 = 2 * K;
     static constexpr int KP = (K2 + 3) / 4 * 4;
     static constexpr int NN = KP * KP;
-    static constexpr int MT = KP / 4;
-    static constexpr int NT = MT * (KP / 2) <= 50 ? KP / 2 : KP / 4;
-    static constexpr int LDX = NN + 4;  // 16-byte rows: staged by cp.async from the block images
-    static constexpr int LD1 = NN + gcfg_pad1(K);
-    static constexpr int LD2 = NN + gcfg_pad2(K);
-    static constexpr int NTILE = NN / NT;
-    static constexpr int NWARP = (NTILE + 7) / 8;
-    static constexpr int NTHR = 32 * NWARP;
+    static constexpr int MT = KP == 8 ? 2 : KP == 24 ? 6 : 4;   // rows of a thread
+    static constexpr int GW = KP == 24 ? 6 : 4;                 // columns of a group (within one slice: GW divides P)
+    static constexpr int NH = KP == 20 ? 4 : KP == 16 ? 2 : 1;     // groups of a thread
+    static constexpr int NT = NH * GW;
+    static constexpr int RT = KP / MT;            // row tiles
+    static constexpr int NA = KP / GW;            // groups per slice
+    static constexpr int NS = KP / NH;            // slices of first groups
+    static constexpr int GS = NN / NH;            // column distance of a thread's groups
+    static constexpr int NTILE = RT * NA * NS;
+    static constexpr int NTHR = (NTILE + 63) / 64 * 64;
+    static constexpr int NWARP = NTHR / 32;
+    // Row strides: 16-byte rows.  Of the T1 (x-step output) and T2 (y-step output) buffers they are those with the
+    // fewest counted shared-memory wavefronts of a CTA's epilogue stores (P = 20: 704 and 960 against 1208 and 1008 unpadded).
+    static constexpr int LDX = NN + 4;  // staged by cp.async from the block images
+    static constexpr int LD1 = NN + 4;
+    static constexpr int LD2 = NN + (KP == 20 ? 4 : 0);
     static constexpr int KK = K * K;
     static constexpr int KKK = K * K * K;
-    static constexpr int NC = gcfg_nc(K, NTHR);  // correction tile columns
-    static constexpr int NCT = KK / NC;
-    static constexpr int ND = MT * NT;  // accumulators per thread
+    // correction tiles: one column and all rows (P = 20: k^2 threads are 3 or 4 warps, one per sub-partition) or half of them
+    static constexpr int CH = KP == 20 ? 1 : 2;
+    static constexpr int RH = CH == 1 ? (K + 1) / 2 * 2 : (K + 3) / 4 * 2;  // rows of a thread, even
+    // contracted indices per step of the tile products' loops (loads of a step are in flight together)
+    static constexpr int KU = K % 5 == 0 ? 5 : K % 4 == 0 ? 4 : K % 3 == 0 ? 3 : K == 7 ? 7 : 4;
+    static constexpr int ND = MT * NT;          // accumulators per thread
     // accumulators in TMEM, 2 columns per double, warps sharing a lane quarter side by side
     static constexpr int TCOLS_NEED = ((NWARP + 3) / 4) * 2 * ND;
     static constexpr int TCOLS = TCOLS_NEED <= 32 ? 32 : TCOLS_NEED <= 64 ? 64 : TCOLS_NEED <= 128 ? 128
                                  : TCOLS_NEED <= 256 ? 256 : 512;
-    static constexpr int XBUF = KP * (LDX > LD1 ? LDX : LD1);  // one staging buffer: X, or T1 at a line's end
+    static constexpr int XBUF = KP * LDX;                        // one staging buffer: X, or T1 at a line's end
     static constexpr int IMG = K2 * NN;                          // block image: rows a < 2k of X, unpadded
     static constexpr size_t SMEM =
         sizeof(float) * (2 * (size_t)XBUF + (size_t)KP * LD2 + 4 * (size_t)KP * KP + 3 * (size_t)KKK) + 64;
-    static constexpr int MINB = 2 * (SMEM + 16 + 1024) <= 233472 ? 2 : 1;
-    static constexpr bool FITS = SMEM + 16 + 1024 <= 232448 && 2 * NCT <= NTHR && TCOLS_NEED <= 512 &&
+    // resident CTAs: what shared memory allows, at most 8 (P = 8), 5 (12: 96 registers a thread), 3 (16: 168), 2 (20: 128)
+    static constexpr int SMB = (int)(233472 / (SMEM + 16 + 1024));
+    static constexpr int REGB = KP == 8 ? 8 : KP == 12 ? 5 : KP == 16 ? 3 : KP == 20 ? 2 : 1;
+    static constexpr int MINB = SMB < 1 ? 1 : SMB < REGB ? SMB : REGB;
+    static constexpr bool FITS = SMEM + 16 + 1024 <= 232448 && CH * KK <= NTHR && TCOLS_NEED <= 512 &&
                                  (size_t)KP * LDX * sizeof(float) >= 64 * sizeof(double) && TCOLS * MINB <= 512;
-    static_assert(NT % 2 == 0, "column pairs");
+    static_assert(MT % 2 == 0 && GW % 2 == 0 && KP % MT == 0 && KP % GW == 0 && KP % NH == 0, "tiles");
 };
 
 // packed FP32 pairs (sm_100 f32x2 arithmetic): two independent round-to-nearest FMAs per instruction,
@@ -806,64 +814,89 @@ __device__ __forceinline__ void unpack_f32x2(unsigned long long v, float& lo, fl
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
-// FP32 tile with packed accumulators kept across calls: pc[i][j] (+)= sum_k At[k lda + o0 + i] times the
-// column pair B[k ldb + n0 + 2j], B[k ldb + n0 + 2j + 1], one f32x2 FMA per pair and contracted index
-template <int MT, int NP>
-__device__ __forceinline__ void gemm_tile_packed(const float* __restrict__ At, int lda, const float* __restrict__ B,
-                                                 int ldb, int o0, int n0, int kdim, unsigned long long (&pc)[MT][NP]) {
-    const float* ap = At + o0;
-    const float* bp = B + n0;
-#pragma unroll 2
-    for (int k = 0; k < kdim; ++k) {
-        unsigned long long a2[MT], b2[NP];
+// N floats from shared memory by 16-byte (N a multiple of 4: 16-byte aligned) or 8-byte loads
+template <int N>
+__device__ __forceinline__ void load_row(const float* __restrict__ p, float (&v)[N]) {
+    if constexpr (N % 4 == 0) {
 #pragma unroll
-        for (int i = 0; i < MT; ++i) a2[i] = pack_f32x2(ap[i], ap[i]);
+        for (int i = 0; i < N; i += 4) {
+            const float4 x = *reinterpret_cast<const float4*>(p + i);
+            v[i] = x.x, v[i + 1] = x.y, v[i + 2] = x.z, v[i + 3] = x.w;
+        }
+    } else {
 #pragma unroll
-        for (int j = 0; j < NP; ++j) b2[j] = *reinterpret_cast<const unsigned long long*>(bp + 2 * j);
+        for (int i = 0; i < N; i += 2) {
+            const float2 x = *reinterpret_cast<const float2*>(p + i);
+            v[i] = x.x, v[i + 1] = x.y;
+        }
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_row(float* __restrict__ p, const float (&v)[N]) {
+    if constexpr (N % 4 == 0) {
 #pragma unroll
-        for (int i = 0; i < MT; ++i)
+        for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    } else {
 #pragma unroll
-            for (int j = 0; j < NP; ++j) pc[i][j] = fma_f32x2(a2[i], b2[j], pc[i][j]);
+        for (int i = 0; i < N; i += 2) *reinterpret_cast<float2*>(p + i) = make_float2(v[i], v[i + 1]);
+    }
+}
+
+// FP32 tile with packed accumulators kept across calls: pc[g][i][j] (+)= sum_k At[k lda + i] times the column pair
+// B[k ldb + gs g + 2j], B[k ldb + gs g + 2j + 1] of group g < NG, one f32x2 FMA per pair and contracted index
+template <int KD, int KU, int NG, int MT, int NH, int NP>
+__device__ __forceinline__ void gemm_tile_packed(const float* __restrict__ ap, int lda, const float* __restrict__ bp,
+                                                 int ldb, int gs, unsigned long long (&pc)[NH][MT][NP]) {
+#pragma unroll KU
+    for (int k = 0; k < KD; ++k) {
+        float a[MT];
+        load_row<MT>(ap, a);
+        unsigned long long a2[MT];
+#pragma unroll
+        for (int i = 0; i < MT; ++i) a2[i] = pack_f32x2(a[i], a[i]);
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            float b[2 * NP];
+            load_row<2 * NP>(bp + g * gs, b);
+#pragma unroll
+            for (int j = 0; j < NP; ++j) {
+                const unsigned long long b2 = pack_f32x2(b[2 * j], b[2 * j + 1]);
+#pragma unroll
+                for (int i = 0; i < MT; ++i) pc[g][i][j] = fma_f32x2(a2[i], b2, pc[g][i][j]);
+            }
+        }
         ap += lda;
         bp += ldb;
     }
 }
 
-// c = At^T B on a thread tile: packed products, unpacked result
-template <int MT, int NT>
-__device__ __forceinline__ void gemm_tile(const float* __restrict__ At, int lda, const float* __restrict__ B, int ldb,
-                                          int o0, int n0, int kdim, float (&c)[MT][NT]) {
-    unsigned long long pc[MT][NT / 2];
+// one column of a correction product: c[i] = sum_{k<kdim} At[k lda + i] B[k ldb], row pairs packed
+// (A16: the rows of At start on 16-byte boundaries, else on 8-byte ones)
+template <int KD, int KU, bool A16, int RH>
+__device__ __forceinline__ void gemm_column(const float* __restrict__ ap, int lda, const float* __restrict__ bp, int ldb,
+                                            float (&c)[RH]) {
+    unsigned long long pc[RH / 2];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int i = 0; i < RH / 2; ++i) pc[i] = 0ull;
+#pragma unroll KU
+    for (int k = 0; k < KD; ++k) {
+        const float b = *bp;
+        const unsigned long long b2 = pack_f32x2(b, b);
+        constexpr int R4 = A16 ? RH / 4 * 4 : 0;
 #pragma unroll
-        for (int j = 0; j < NT / 2; ++j) pc[i][j] = 0ull;
-    gemm_tile_packed<MT, NT / 2>(At, lda, B, ldb, o0, n0, kdim, pc);
+        for (int i = 0; i < R4; i += 4) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(ap + i);
+            pc[i / 2] = fma_f32x2(a.x, b2, pc[i / 2]);
+            pc[i / 2 + 1] = fma_f32x2(a.y, b2, pc[i / 2 + 1]);
+        }
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT / 2; ++j) unpack_f32x2(pc[i][j], c[i][2 * j], c[i][2 * j + 1]);
-}
-
-// the same with per-column offsets (correction GEMMs; columns not contiguous)
-template <int MT, int NT>
-__device__ __forceinline__ void gemm_tile_off(const float* __restrict__ At, int lda, const float* __restrict__ B, int ldb,
-                                              int o0, const int (&off)[NT], int kdim, float (&c)[MT][NT]) {
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) c[i][j] = 0.0f;
-    for (int k = 0; k < kdim; ++k) {
-        float a[MT], b[NT];
-#pragma unroll
-        for (int i = 0; i < MT; ++i) a[i] = At[k * lda + o0 + i];
-#pragma unroll
-        for (int j = 0; j < NT; ++j) b[j] = B[k * ldb + off[j]];
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NT; ++j) c[i][j] = fmaf(a[i], b[j], c[i][j]);
+        for (int i = R4; i < RH; i += 2)
+            pc[i / 2] = fma_f32x2(*reinterpret_cast<const unsigned long long*>(ap + i), b2, pc[i / 2]);
+        ap += lda;
+        bp += ldb;
     }
+#pragma unroll
+    for (int i = 0; i < RH / 2; ++i) unpack_f32x2(pc[i], c[2 * i], c[2 * i + 1]);
 }
 
 // Line-ordered GEMM-tiled contraction.  A chunk is a range of one output node's surviving triples,
@@ -885,8 +918,9 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
              const int* __restrict__ csrc, const float* __restrict__ ximg, long long gbase, double* partials,
              unsigned long long* ntrip_out) {
     using C = GCfg<K>;
-    constexpr int K2 = C::K2, KP = C::KP, MT = C::MT, NT = C::NT, NC = C::NC, ND = C::ND;
-    constexpr int LDX = C::LDX, LD1 = C::LD1, LD2 = C::LD2, NN = C::NN, IMG = C::IMG;
+    constexpr int K2 = C::K2, KP = C::KP, MT = C::MT, NT = C::NT, GW = C::GW, NH = C::NH, RH = C::RH, KU = C::KU, ND = C::ND;
+    constexpr bool A16 = C::CH == 1 || RH % 4 == 0;
+    constexpr int LDX = C::LDX, LD1 = C::LD1, LD2 = C::LD2, NN = C::NN, GS = C::GS, IMG = C::IMG;
     constexpr int KK = C::KK, KKK = C::KKK;
     constexpr int BS = K2 * K2 * K2;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -907,18 +941,17 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
     const float* mats = TR.matsT32;
     const float* matsb = TR.matsbT32;
     const bool root = TR.root != 0;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // tiles: 4 row tiles x 8 consecutive column tiles per warp
-    const int rt = lane & 3;
-    const int ct_c = warp * 8 + (lane >> 2);
-    const bool own = ct_c < C::NTILE;
-    const int o0 = rt * MT;
-    const int n0 = own ? ct_c * NT : 0;
-    const int tb0 = n0 % KP, tc0 = n0 / KP;     // x tile: first b, c;  y tile: first a', c;  z tile: first a', b'
-    // correction tile
-    const int crt = tid & 1, cct = tid >> 1;
-    const bool cown = !root && cct < C::NCT;
-    const int co0 = crt * MT, cn0 = cown ? cct * NC : 0;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    // tiles: the groups of a slice fastest, then row tiles (fewest wavefronts of the T2 sums), then slices
+    const bool own = tid < C::NTILE;
+    const int tile = own ? tid : 0;
+    const int o0 = (tile / C::NA) % C::RT * MT;
+    const int tb0 = tile % C::NA * GW, tc0 = tile / (C::NA * C::RT);  // x tile: first b, c;  y tile: first a', c;
+    const int n0 = tb0 + KP * tc0;                                    // z tile: first a', b' (of the first group)
+    // correction tile: column n of k^2, rows co0 .. co0 + RH of k (the same rows for a whole warp)
+    const int ch0 = tid / (C::NTHR / C::CH), cn = tid - ch0 * (C::NTHR / C::CH);
+    const bool cown = !root && cn < KK;
+    const int co0 = ch0 * RH, cnl = cown ? cn % K : 0, cnh = cown ? cn / K : 0;
 
     // accumulators: this thread's TMEM lane
     if (warp == 0) {
@@ -936,8 +969,8 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
     unsigned long long ntrip = 0;
     bool pend2 = false;     // c2 holds a correction block not yet written to Uc
     bool uc_valid = false;  // Uc holds a correction block not yet subtracted
-    float c2[MT][NC];
-    unsigned long long xp[MT][NT / 2];  // x sums of the current line (this thread's x tile), column pairs packed
+    float c2[RH], u1[RH];   // correction blocks: of the plane, x sums of the line
+    unsigned long long xp[NH][MT][GW / 2];  // x sums of the current line (this thread's x tile), column pairs packed
 
     // asynchronous copy of a transposed operator (At[k][o] = M[o][k], P x P) into shared memory, as
     // one commit group
@@ -967,16 +1000,14 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
     };
     // correction block of element (c', a', b') of this thread's z tile, 0 outside s->s
     auto uc_at = [&](int i, int j) -> double {
-        const int cz = o0 + i, n = n0 + j, ax = n % KP, by = n / KP;
+        const int cz = o0 + i, ax = tb0 + j % GW, by = tc0 + j / GW * C::NS;
         return (cz < K && ax < K && by < K) ? (double)Uc[cz * KK + ax + K * by] : 0.0;
     };
     auto write_c2 = [&]() {
         if (!cown) return;
 #pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NC; ++j)
-                if (co0 + i < K) Uc[(co0 + i) * KK + cn0 + j] = c2[i][j];
+        for (int i = 0; i < RH; ++i)
+            if (co0 + i < K) Uc[(co0 + i) * KK + cn] = c2[i];
     };
 
     auto line_of = [&](int t) -> uint32_t { return (uint32_t)(tkey[t] & 0xffffffffull); };
@@ -1013,31 +1044,23 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
         const float* Mxq = q ? Mx1 : Mx0;
         // ---- x: xp[a'][b + P c] (+)= sum_a Mx[a'][a] X[a][b + P c]   (a line sums its triples)
         if (own) {
-            const bool live = !gen || (tb0 < K && tc0 < K);  // other tiles of a generated input are zero
             if (lstart) {
 #pragma unroll
-                for (int i = 0; i < MT; ++i)
+                for (int g = 0; g < NH; ++g)
 #pragma unroll
-                    for (int j = 0; j < NT / 2; ++j) xp[i][j] = 0ull;
+                    for (int i = 0; i < MT; ++i)
+#pragma unroll
+                        for (int j = 0; j < GW / 2; ++j) xp[g][i][j] = 0ull;
             }
-            if (live) gemm_tile_packed<MT, NT / 2>(Mxq, KP, Xq, LDX, o0, n0, gen ? K : K2, xp);
+            // of a generated input, groups outside b, c < k are zero (the upper half of a thread's are: P/2 >= k)
+            if (!gen) gemm_tile_packed<K2, KU, NH>(Mxq + o0, KP, Xq + n0, LDX, GS, xp);
+            else if (tb0 < K && tc0 < K) gemm_tile_packed<K, KU, (NH + 1) / 2>(Mxq + o0, KP, Xq + n0, LDX, GS, xp);
         }
         if (cown) {  // U1[b][a' + k c] (+)= sum_{a<k} Tx[a'][a] X[a][b + P c]   (summed over the line)
-            int off[NC];
+            float c[RH];
+            gemm_column<K, KU, A16>(Mxq + co0, KP, Xq + cnl + KP * cnh, LDX, c);
 #pragma unroll
-            for (int j = 0; j < NC; ++j) off[j] = (cn0 + j) % K + KP * ((cn0 + j) / K);
-            float c[MT][NC];
-            gemm_tile_off<MT, NC>(Mxq, KP, Xq, LDX, co0, off, K, c);
-#pragma unroll
-            for (int i = 0; i < MT; ++i)
-#pragma unroll
-                for (int j = 0; j < NC; ++j) {
-                    const int n = cn0 + j;
-                    if (co0 + i < K) {
-                        float& d = U1[(n % K) * KK + co0 + i + K * (n / K)];
-                        d = lstart ? c[i][j] : d + c[i][j];
-                    }
-                }
+            for (int i = 0; i < RH; ++i) u1[i] = lstart ? c[i] : u1[i] + c[i];
         }
         ++ntrip;
         if (!lend) continue;
@@ -1045,14 +1068,21 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
         float* T1 = Xq;       // [KP][LD1]
         if (own) {
 #pragma unroll
-            for (int j = 0; j < NT / 2; ++j)
+            for (int g = 0; g < NH; ++g)
 #pragma unroll
-                for (int i = 0; i < MT; ++i) {
-                    float lo, hi;
-                    unpack_f32x2(xp[i][j], lo, hi);
-                    T1[(tb0 + 2 * j) * LD1 + o0 + i + KP * tc0] = lo;
-                    T1[(tb0 + 2 * j + 1) * LD1 + o0 + i + KP * tc0] = hi;
+                for (int j = 0; j < GW / 2; ++j) {
+                    float lo[MT], hi[MT];
+#pragma unroll
+                    for (int i = 0; i < MT; ++i) unpack_f32x2(xp[g][i][j], lo[i], hi[i]);
+                    float* col = T1 + (tb0 + 2 * j) * LD1 + o0 + KP * (tc0 + g * C::NS);
+                    store_row<MT>(col, lo);
+                    store_row<MT>(col + LD1, hi);
                 }
+        }
+        if (cown) {
+#pragma unroll
+            for (int i = 0; i < RH; ++i)
+                if (co0 + i < K) U1[cnl * KK + co0 + i + K * cnh] = u1[i];
         }
         // My (and Mz) were committed before the next triple's staging group
         if (more) cp_async_wait_group<1>();
@@ -1065,74 +1095,68 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
             uc_valid = true;
         }
         if (own) {
-            const bool zero = line_gen && !(tc0 < K);  // this tile is zero for generated inputs
-            if (!zero || first_line) {
-                float c[MT][NT];
-                if (zero) {
+            // sums of group g: those of a generated line are zero for c >= k (the upper half of the groups)
+            unsigned long long pc[NH][MT][GW / 2];
 #pragma unroll
-                    for (int i = 0; i < MT; ++i)
+            for (int g = 0; g < NH; ++g)
 #pragma unroll
-                        for (int j = 0; j < NT; ++j) c[i][j] = float(0);
-                } else {
-                    gemm_tile<MT, NT>(My, KP, T1, LD1, o0, n0, line_gen ? K : K2, c);
-                }
+                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                    for (int j = 0; j < GW / 2; ++j) pc[g][i][j] = 0ull;
+            if (!line_gen) gemm_tile_packed<K2, KU, NH>(My + o0, KP, T1 + n0, LD1, GS, pc);
+            else if (tc0 < K) gemm_tile_packed<K, KU, (NH + 1) / 2>(My + o0, KP, T1 + n0, LD1, GS, pc);
+#pragma unroll
+            for (int g = 0; g < NH; ++g) {
+                if (line_gen && !first_line && !(tc0 + g * C::NS < K)) continue;
 #pragma unroll
                 for (int i = 0; i < MT; ++i) {
-                    float* row = T2 + tc0 * LD2 + tb0 + KP * (o0 + i);
+                    float* row = T2 + (tc0 + g * C::NS) * LD2 + tb0 + KP * (o0 + i);
+                    float c[GW], v[GW];
 #pragma unroll
-                    for (int j = 0; j < NT; j += 2) {
-                        float2 v;
-                        if (first_line) {
-                            v.x = c[i][j];
-                            v.y = c[i][j + 1];
-                        } else {
-                            v = *reinterpret_cast<const float2*>(row + j);
-                            v.x += c[i][j];
-                            v.y += c[i][j + 1];
-                        }
-                        *reinterpret_cast<float2*>(row + j) = v;
+                    for (int j = 0; j < GW / 2; ++j) unpack_f32x2(pc[g][i][j], c[2 * j], c[2 * j + 1]);
+                    if (!first_line) {
+                        load_row<GW>(row, v);
+#pragma unroll
+                        for (int j = 0; j < GW; ++j) c[j] = v[j] + c[j];
                     }
+                    store_row<GW>(row, c);
                 }
             }
         }
         if (cown) {  // U2[c][a' + k b'] (+)= sum_{b<k} Ty[b'][b] U1[b][a' + k c]
-            int off[NC];
+            float c[RH];
+            gemm_column<K, KU, A16>(My + co0, KP, U1 + cn, KK, c);
 #pragma unroll
-            for (int j = 0; j < NC; ++j) off[j] = cn0 + j;
-            float c[MT][NC];
-            gemm_tile_off<MT, NC>(My, KP, U1, KK, co0, off, K, c);
-#pragma unroll
-            for (int i = 0; i < MT; ++i)
-#pragma unroll
-                for (int j = 0; j < NC; ++j) {
-                    const int n = cn0 + j;
-                    if (co0 + i < K) {
-                        float& d = U2[(n / K) * KK + (n % K) + K * (co0 + i)];
-                        d = first_line ? c[i][j] : d + c[i][j];
-                    }
+            for (int i = 0; i < RH; ++i)
+                if (co0 + i < K) {
+                    float& d = U2[cnh * KK + cnl + K * (co0 + i)];
+                    d = first_line ? c[i] : d + c[i];
                 }
         }
         first_line = false;
         if (!pend) continue;
         __syncthreads();  // T2, U2 and Uc of the plane are complete
         // ---- z: acc[c'][a' + P b'] += sum_c (beta Mz)[c'][c] T2[c][a' + P b']  (- previous correction)
-        const int kdz = plane_gen ? K : K2;
         {
-            float c[MT][NT];
-            if (own) {
-                gemm_tile<MT, NT>(Mz, KP, T2, LD2, o0, n0, kdz, c);
-            } else {
+            unsigned long long pc[NH][MT][GW / 2];
+#pragma unroll
+            for (int g = 0; g < NH; ++g)
 #pragma unroll
                 for (int i = 0; i < MT; ++i)
 #pragma unroll
-                    for (int j = 0; j < NT; ++j) c[i][j] = 0.0f;
+                    for (int j = 0; j < GW / 2; ++j) pc[g][i][j] = 0ull;
+            if (own) {
+                if (plane_gen) gemm_tile_packed<K, KU, NH>(Mz + o0, KP, T2 + n0, LD2, GS, pc);
+                else gemm_tile_packed<K2, KU, NH>(Mz + o0, KP, T2 + n0, LD2, GS, pc);
             }
             const bool fold = uc_valid && own;
             tmem_visit<ND, true>(tacc, [&](int d0, int n, auto& r) {
 #pragma unroll
                 for (int q2 = 0; q2 < n; ++q2) {
                     const int d = d0 + q2, i = d / NT, j = d % NT;
-                    double v = words_to_double(r[2 * q2], r[2 * q2 + 1]) + (double)c[i][j];
+                    float lo, hi;
+                    unpack_f32x2(pc[j / GW][i][j % GW / 2], lo, hi);
+                    double v = words_to_double(r[2 * q2], r[2 * q2 + 1]) + (double)(j % 2 ? hi : lo);
                     if (fold) v -= uc_at(i, j);
                     double_to_words(v, r[2 * q2], r[2 * q2 + 1]);
                 }
@@ -1140,10 +1164,7 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
         }
         uc_valid = false;
         if (cown) {  // c2[c'][a' + k b'] = sum_{c<k} (beta Tz)[c'][c] U2[c][a' + k b']
-            int off[NC];
-#pragma unroll
-            for (int j = 0; j < NC; ++j) off[j] = cn0 + j;
-            gemm_tile_off<MT, NC>(Mz, KP, U2, KK, co0, off, K, c2);
+            gemm_column<K, KU, A16>(Mz + co0, KP, U2 + cn, KK, c2);
         }
         pend2 = !root;
     }
@@ -1155,7 +1176,7 @@ __global__ void __launch_bounds__(GCfg<K>::NTHR, GCfg<K>::MINB)
     double* dst = ch.slot < 0 ? TR.ocoef + (size_t)it.node * BS : partials + (size_t)ch.slot * BS;
     double n2 = 0.0, w2 = 0.0;
     auto emit = [&](int i, int j, double v) {
-        const int cz = o0 + i, n = n0 + j, ax = n % KP, by = n / KP;
+        const int cz = o0 + i, ax = tb0 + j % GW, by = tc0 + j / GW * C::NS;
         if (uc_valid) v -= uc_at(i, j);
         if (cz < K2 && ax < K2 && by < K2) {
             dst[ax + K2 * (by + K2 * cz)] = v;
