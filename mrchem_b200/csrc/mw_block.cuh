@@ -32,7 +32,11 @@ struct BX {
     static constexpr int LDP = dcfg_ld(LDA == K2 ? (K2 * K2 + 7) / 8 * 8 : LDA * K2);
     static constexpr int VOL = LDP * K2;
     static constexpr int FRAG = S * RT * 32;  // one operator
-    static constexpr int NWARP = K, NTHR = 32 * NWARP;
+    // A warp belongs to one SM sub-partition: with k warps of two slices each, k = 9, 10 loads two of the four half as much
+    // again as the others, eight warps with slices dealt in turn load them evenly (28 pair products: k = 9 8.80 -> 8.07 ms,
+    // k = 10 8.18 -> 7.92, k = 11 10.95 -> 10.77; k = 5, 6, 7 do not gain).  The sums' kernel (RO = k) holds a block in
+    // registers and needs the threads (k = 11: 4 % slower with eight warps).
+    static constexpr int NWARP = RO == K2 && K >= 9 && K <= 11 ? 8 : K, NTHR = 32 * NWARP;
 };
 
 // b of column n of an x tile (>= 2k: padding)

@@ -15,8 +15,8 @@
 // Refinement follows the adaptive projection: after every pass the leaves whose wavelet norm exceeds
 // prec ||out|| 2^{-depth/2} are split and their children computed.
 //
-// Work per node: 9 to 9 + 6 L in-place pencil transforms of a (2k)^3 FP64 tensor (L = levels of
-// generation), 2 blocks read and 1 written: compute-bound on the FP64 pipe, off the apply's hot path.
+// Work per node: 9 mode products of a (2k)^3 FP64 tensor on the FP64 matrix instruction (mw_block.cuh), whatever the
+// number of levels of generation, 2 blocks read and 1 written: bound by the FP64 pipe.
 #include <algorithm>
 #include <cmath>
 #include <string>
