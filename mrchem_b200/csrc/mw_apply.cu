@@ -7,10 +7,10 @@
 //      node up in the input tree's hash index (or its leaf ancestor -> generated node) and screens it;
 //   2. generated (scaling-only) input nodes are de-duplicated per tree and built once;
 //   3. per candidate, the number of terms that pass the screening (the triples it contributes);
-//   4. GEMM-tiled engine: the triples are expanded and sorted per output node by (term, dz, dy), and
+//   4. line-ordered engines (FP64, FP32, BF16x3): the triples are expanded and sorted per output node by (term, dz, dy), and
 //      each node's sorted triples are cut at plane boundaries into chunks of about chunk_triples
 //      triples (a per-engine context setting, 48 unless tuned); the input blocks of the pass get
-//      images in the kernel's staging layout.  Tensor-core and pencil engines: each node's candidate
+//      images in the kernel's staging layout.  TF32 and pencil engines: each node's candidate
 //      list is cut into chunks of at most chunk_triples triples;
 //   5. the contraction kernel runs one CTA per chunk; multi-chunk nodes write partial blocks that
 //      a reduction kernel adds in chunk order (deterministic), single-chunk nodes write directly;
@@ -1280,8 +1280,8 @@ __global__ void k_bsplit_flags(const Item* __restrict__ items, int nitems, const
 
 static inline void count(Ctx* c, int n = 1) { c->launches += n; }
 
-// MWB200_CONTRACTION=pencil selects the pencil contraction kernel even where the GEMM-tiled one fits
-// (both compute the same sums; kept for comparison and for bases too large for the tiled kernel)
+// MWB200_CONTRACTION=pencil selects the pencil contraction kernel in place of the FP64 and FP32 engines
+// (both compute the same sums; kept for comparison)
 static bool contraction_pencil() {
     static const bool v = [] {
         const char* e = std::getenv("MWB200_CONTRACTION");

@@ -13,8 +13,8 @@
 // instructions alone, padded rows included: 17.8), 20-atom Poisson at k = 12 302 -> 41.2 ms (37.3), three-charge
 // Poisson at k = 8 5.2 -> 2.2 ms and at k = 6 1.42 -> 0.63 ms.
 //
-// Work split (k <= 8; beyond, eight warps and extra units, see DCfg).  Warp p owns the z-index pair (c = p, p + k): one slice of the scaling half and one of the
-// wavelet half, so that generated (scaling-only) inputs and the s->s correction load every warp alike.
+// Work split (k = 6 and k > 8 share the last pairs out as extra units, see DCfg).  Warp p owns the z-index pair
+// (c = p, p + k): one slice of the scaling half and one of the wavelet half, so that generated (scaling-only) inputs and the s->s correction load every warp alike.
 // The x product of its 2 x 2k columns (b, c) accumulates in registers over the line's triples (rows a',
 // columns b: the FP64 C fragment), and that fragment is the A operand of the y product as it stands: a
 // lane's two C values are columns 2j and 2j+1, so with columns ordered b = 8t + 4e + j (e the parity) each
@@ -48,10 +48,12 @@ struct DCfg {
     static constexpr int FT = K2 / 8, REM = K2 % 8;
     static constexpr int WOFF = FT + (REM != 0 ? 1 : 0);               // first own tile of the wavelet slice
     static constexpr int NTP = 2 * FT + (REM == 0 ? 0 : REM <= 4 ? 1 : 2);  // column tiles of a pair
-    // one pair per warp; from k = 9 up eight warps (two per SM sub-partition, 255 registers each) take a pair
+    // one pair per warp; at k = 6 and from k = 9 up fewer: eight warps (two per SM sub-partition, 255 registers each) take a pair
     // each and share the last K - 8 pairs by slices: an extra unit = one slice c, at most one per warp.  (One warp
-    // per pair puts three warps on one or two sub-partitions and two on the others at k = 9, 10.)
-    static constexpr int NWARP = K > 8 ? 8 : K, NTHR = 32 * NWARP;
+    // per pair puts three warps on one or two sub-partitions and two on the others at k = 9, 10.)  k = 6 likewise
+    // with four warps of a pair and an extra unit each: 1.33 -> 1.23 ms in the three-charge Poisson; at k = 5 the two extra
+    // units leave two warps idle for a third of the time (1.13 -> 1.16, not used).
+    static constexpr int NWARP = K > 8 ? 8 : K == 6 ? 4 : K, NTHR = 32 * NWARP;
     static constexpr int NXU = 2 * (K - NWARP);  // extra units: pair 8 + u / 2, slice u mod 2
     static constexpr bool XU = NXU > 0;
     static constexpr int RS = (K + 7) / 8;    // row and column tiles of the scaling corner
