@@ -24,6 +24,7 @@
 
 #include "mw_device.cuh"
 #include "mw_kernels.cuh"
+#include "mw_opplan.hpp"
 #include "mw_slice.hpp"
 
 namespace mwb {
@@ -228,7 +229,7 @@ __device__ __forceinline__ double bound3_dev(double beta, const double* t, const
 // operator | dx | dy | dz (bits each, offset by lm), bound, term)
 __global__ void k_op_list(const OpTerm* __restrict__ terms, int nterm, long long nrows, const double* __restrict__ t2,
                           const double* __restrict__ x2, int lcap, int root, int lm, int bits, int* count,
-                          const int* __restrict__ offs, unsigned long long* key, double* bound, int* term) {
+                          const long long* __restrict__ offs, unsigned long long* key, double* bound, int* term) {
     const long long row = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (row >= nrows) return;
     int lo = 0, hi = nterm - 1;  // last term with row0 <= row (inactive terms have no rows)
@@ -246,7 +247,7 @@ __global__ void k_op_list(const OpTerm* __restrict__ terms, int nterm, long long
     const int ix = abs(dx), iy = abs(dy);
     const double ax = t2r[ix] + x2r[ix], ay = t2r[iy] + x2r[iy];
     int n = 0;
-    const int p0 = offs ? offs[row] : 0;
+    const long long p0 = offs ? offs[row] : 0;
     if (root || !(tm.beta * sqrt(ax) * S2 < tm.cut || tm.beta * sqrt(ax * ay * S2) < tm.cut)) {
         for (int dz = -tm.L; dz <= tm.L; ++dz) {
             const int iz = abs(dz);
@@ -447,11 +448,13 @@ int bits_for(int n) {
     while ((1 << b) < n) ++b;
     return b;
 }
-void exclusive_sum(Ctx* ctx, const int* in, int* out, int n) {
+// (the sums have the type of `out`)
+template <typename T>
+void exclusive_sum(Ctx* ctx, const int* in, T* out, int n) {
     size_t tmp = 0;
-    MWB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, in, out, n, ctx->stream));
+    MWB_CUDA(cub::DeviceScan::ExclusiveScan(nullptr, tmp, in, out, ::cuda::std::plus<>{}, T(0), n, ctx->stream));
     void* d = dalloc(ctx, tmp);
-    MWB_CUDA(cub::DeviceScan::ExclusiveSum(d, tmp, in, out, n, ctx->stream));
+    MWB_CUDA(cub::DeviceScan::ExclusiveScan(d, tmp, in, out, ::cuda::std::plus<>{}, T(0), n, ctx->stream));
     dfree(ctx, d);
 }
 template <typename KT>
@@ -596,6 +599,39 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         release();
         throw Error(-4, "operator band wider than 1024 offsets per direction");
     }
+    upload_bytes(ctx, d_terms, terms.data(), sizeof(OpTerm) * nt);
+    // lists
+    const int bits = bits_for(2 * lm + 1), obits = bits_for(nop);
+    // records per operator, counted before anything is made from them
+    OpPlan plan = op_plan_rows(nop, nrows);
+    int* d_cnt = nullptr;
+    long long* d_offs = nullptr;
+    std::vector<long long> first(nop + 1, 0);
+    if (nrows > 0 && plan == OpPlan::together) {
+        d_cnt = alloc<int>(ctx, nrows + 1);
+        d_offs = alloc<long long>(ctx, nrows + 1);
+        tmp.insert(tmp.end(), {(void*)d_cnt, (void*)d_offs});
+        MWB_CUDA(cudaMemsetAsync(d_cnt + nrows, 0, sizeof(int), s));
+        k_op_list<<<blocks_of(nrows, 128), 128, 0, s>>>(d_terms, nt, nrows, d_t2, d_x2, lcap, root, lm, bits, d_cnt, nullptr,
+                                                        nullptr, nullptr, nullptr);
+        MWB_CUDA(cudaGetLastError());
+        exclusive_sum(ctx, d_cnt, d_offs, (int)nrows + 1);
+        // the row offsets at the operators' first terms
+        std::vector<ReadReq> rq;
+        for (int o = 0; o <= nop; ++o)
+            rq.push_back(ReadReq{&first[o], d_offs + (o < nop ? terms[t0[o]].row0 : nrows), sizeof(long long)});
+        for (size_t q = 0; q < rq.size(); q += 8) {
+            auto at = [&](size_t i) { return q + i < rq.size() ? rq[q + i] : ReadReq{nullptr, nullptr, 0}; };
+            readback(ctx, {at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7)});
+        }
+        plan = op_plan_records(nop, first[nop]);
+    }
+    if (plan != OpPlan::together) {
+        release();
+        if (plan == OpPlan::refuse) throw Error(-4, "operator offset list too large");
+        for (Op* o : ops) op_build_group({o}, depth, lcap);
+        return;
+    }
     std::vector<std::unique_ptr<OpDepth>> ods;
     for (int o = 0; o < nop; ++o) {
         ods.push_back(std::make_unique<OpDepth>());
@@ -612,34 +648,10 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         dfree(ctx, d_src);
         dfree(ctx, d_beta);
     }
-    upload_bytes(ctx, d_terms, terms.data(), sizeof(OpTerm) * nt);
-    // lists
-    const int bits = bits_for(2 * lm + 1), obits = bits_for(nop);
-    std::vector<int> rec0(nop + 1, 0), del0(nop + 1, 0);
+    std::vector<int> rec0(first.begin(), first.end()), del0(nop + 1, 0);
     std::vector<double> maxb;
     if (nrows > 0) {
-        if (nrows > (1ll << 30)) throw Error(-4, "operator offset list too large");
-        int* d_cnt = alloc<int>(ctx, nrows + 1);
-        int* d_offs = alloc<int>(ctx, nrows + 1);
-        tmp.insert(tmp.end(), {d_cnt, d_offs});
-        MWB_CUDA(cudaMemsetAsync(d_cnt + nrows, 0, sizeof(int), s));
-        k_op_list<<<blocks_of(nrows, 128), 128, 0, s>>>(d_terms, nt, nrows, d_t2, d_x2, lcap, root, lm, bits, d_cnt, nullptr,
-                                                        nullptr, nullptr, nullptr);
-        MWB_CUDA(cudaGetLastError());
-        exclusive_sum(ctx, d_cnt, d_offs, (int)nrows + 1);
-        // records per operator: the row offsets at the operators' first terms
-        std::vector<int> first(nop + 1);
-        {
-            std::vector<ReadReq> rq;
-            for (int o = 0; o <= nop; ++o)
-                rq.push_back(ReadReq{&first[o], d_offs + (o < nop ? terms[t0[o]].row0 : nrows), sizeof(int)});
-            for (size_t q = 0; q < rq.size(); q += 8) {
-                auto at = [&](size_t i) { return q + i < rq.size() ? rq[q + i] : ReadReq{nullptr, nullptr, 0}; };
-                readback(ctx, {at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7)});
-            }
-        }
-        rec0 = first;
-        const int nrec = first[nop];
+        const int nrec = rec0[nop];
         const int rb = blocks_of(nrec, 256);
         if (nrec > 0) {
             auto* d_key = alloc<unsigned long long>(ctx, nrec);
@@ -716,7 +728,8 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
 }
 
 void op_build_tables(const std::vector<Op*>& ops, int depth) {
-    // at most eight operators at a time: bounds the scratch (8 x 134 terms x 64 offsets x 4.6 KB at k = 12)
+    // at most eight operators at a time: bounds the matrices' scratch (8 x 134 terms x 64 offsets x 4.6 KB at k = 12);
+    // that of the lists is bounded by the plan
     for (size_t q = 0; q < ops.size(); q += 8)
         op_build_group(std::vector<Op*>(ops.begin() + q, ops.begin() + std::min(ops.size(), q + 8)), depth, 64);
 }

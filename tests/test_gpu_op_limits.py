@@ -1,0 +1,45 @@
+"""Operator tables at the limits of their construction (mw_optab.cu): groups whose lists are built one operator at a time,
+and lists beyond 32-bit positions.
+
+Bar: tables equal those of an operator built alone bit for bit; what is refused is an error and leaves the context usable."""
+import pytest
+
+from test_gpu_parity import assert_same_tree
+
+pytestmark = pytest.mark.gpu
+
+
+def row_world(G, boxes, order=3):
+    """a row of boxes: the bands of the wide terms reach over all of it, in every direction"""
+    return G.MultiResolutionAnalysis(-2, (-(boxes // 2), 0, 0), (boxes, 1, 1), order, 10)
+
+
+def test_large_lists_of_a_group(gpu_mod):
+    """about 14 million records each at the root: more than one group holds, 32-bit counts apart"""
+    G = gpu_mod
+    m = row_world(G, 40)
+    f = G.FunctionTree(m)
+    G.project(1e-2, f, G.gauss_params([1.0], [2.0], [(0.3, 1.9, 2.2)]))
+    precs = [1e-3, 2e-3, 5e-3]
+    ops = [G.PoissonOperator(m, p) for p in precs]
+    outs = [G.FunctionTree(m) for _ in ops]
+    G.apply_batched(1e-2, outs, ops, [f] * 3)
+    for p, out in zip(precs, outs):
+        one = G.FunctionTree(m)
+        G.apply(1e-2, one, G.PoissonOperator(m, p), f)
+        assert one.square_norm() > 0.0
+        assert_same_tree(out.export(), one.export(), tol=0.0)
+
+
+def test_lists_beyond_32_bit_positions_are_refused(gpu_mod):
+    """about 4e9 records of one operator"""
+    G = gpu_mod
+    m = row_world(G, 256)
+    f = G.FunctionTree(m)
+    G.project(1e-2, f, G.gauss_params([1.0], [2.0], [(0.3, 1.9, 2.2)]))
+    out = G.FunctionTree(m)
+    for ops in ([G.PoissonOperator(m, 1e-3)], [G.PoissonOperator(m, 1e-3), G.PoissonOperator(m, 2e-3)]):
+        with pytest.raises(G.MWError, match="offset list too large"):
+            G.apply_batched(1e-2, [out, G.FunctionTree(m)][: len(ops)], ops, [f] * len(ops))
+    G.apply(1e-2, out, G.HelmholtzOperator(m, 20.0, 1e-3), f)  # the context goes on
+    assert out.square_norm() > 0.0
