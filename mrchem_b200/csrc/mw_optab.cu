@@ -557,14 +557,14 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
             ctx->launches++;
         }
     }
-    k_op_band<<<blocks_of(nt, 128), 128, 0, s>>>(d_terms, nt, d_t2, d_x2, lcap, depth, extent, d_flag);
-    MWB_CUDA(cudaGetLastError());
-    ctx->launches++;
+    if (nt > 0) {  // (an expansion whose range is empty has no terms)
+        k_op_band<<<blocks_of(nt, 128), 128, 0, s>>>(d_terms, nt, d_t2, d_x2, lcap, depth, extent, d_flag);
+        MWB_CUDA(cudaGetLastError());
+        ctx->launches++;
+    }
     int flag = 0;
-    std::vector<double> c2;  // root: squared norms at l = 0 (the operator scale B0)
     readback(ctx, {{terms.data(), d_terms, sizeof(OpTerm) * nt}, {&flag, d_flag, sizeof(int)}});
-    if (root) {
-        std::vector<double> t2(nt), x2(nt);
+    if (root) {  // the operator scale B0, from the squared norms at l = 0
         std::vector<double> a2((size_t)nt * lcap), b2((size_t)nt * lcap);
         readback(ctx, {{a2.data(), d_t2, sizeof(double) * a2.size()}, {b2.data(), d_x2, sizeof(double) * b2.size()}});
         for (int t = 0; t < nt; ++t) {
@@ -619,7 +619,7 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         // the row offsets at the operators' first terms
         std::vector<ReadReq> rq;
         for (int o = 0; o <= nop; ++o)
-            rq.push_back(ReadReq{&first[o], d_offs + (o < nop ? terms[t0[o]].row0 : nrows), sizeof(long long)});
+            rq.push_back(ReadReq{&first[o], d_offs + (t0[o] < nt ? terms[t0[o]].row0 : nrows), sizeof(long long)});
         for (size_t q = 0; q < rq.size(); q += 8) {
             auto at = [&](size_t i) { return q + i < rq.size() ? rq[q + i] : ReadReq{nullptr, nullptr, 0}; };
             readback(ctx, {at(0), at(1), at(2), at(3), at(4), at(5), at(6), at(7)});

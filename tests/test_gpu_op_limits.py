@@ -2,9 +2,11 @@
 and lists beyond 32-bit positions.
 
 Bar: tables equal those of an operator built alone bit for bit; what is refused is an error and leaves the context usable."""
+import math
+
 import pytest
 
-from test_gpu_parity import assert_same_tree
+from test_gpu_parity import WORLD, assert_same_tree, two_gaussians
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +45,35 @@ def test_lists_beyond_32_bit_positions_are_refused(gpu_mod):
             G.apply_batched(1e-2, [out, G.FunctionTree(m)][: len(ops)], ops, [f] * len(ops))
     G.apply(1e-2, out, G.HelmholtzOperator(m, 20.0, 1e-3), f)  # the context goes on
     assert out.square_norm() > 0.0
+
+
+def test_operator_without_terms(gpu_mod):
+    """a decay length far below the finest scale leaves no term of the expansion: the operator gives zero, alone and at
+    any place of a batch"""
+    G = gpu_mod
+    prec, depth = 1e-3, 10
+    m = G.MultiResolutionAnalysis(*WORLD, 5, depth)
+    eps, r_min = 0.1 * prec, 0.01 * 4.0 * 2.0 ** -depth
+    h = math.pi ** 2 / (2.0 * math.log(2.0 * math.sqrt(2.0) / eps))
+    s_hi = math.log((math.sqrt(-math.log(0.1 * eps)) + 1.0) / r_min)
+    mu = 2.0 * math.sqrt(-math.log(1e-3 * eps)) * math.exp(s_hi + 1.5 * h)  # one and a half steps beyond the range
+    none = G.HelmholtzOperator(m, mu, prec)
+    assert len(none.terms()[0]) == 0
+    f = G.FunctionTree(m)
+    G.project(prec, f, two_gaussians(G))
+    out = G.FunctionTree(m)
+    G.apply(prec, out, none, f)
+    assert out.square_norm() == 0.0 and out.nnodes() == 1000
+    some = G.HelmholtzOperator(m, 1.0, prec)
+    one = G.FunctionTree(m)
+    G.apply(prec, one, some, f)
+    for where in range(3):
+        ops = [G.HelmholtzOperator(m, 1.0, prec) for _ in range(2)]
+        ops.insert(where, G.HelmholtzOperator(m, mu, prec))
+        outs = [G.FunctionTree(m) for _ in ops]
+        G.apply_batched(prec, outs, ops, [f] * 3)
+        for q, t in enumerate(outs):
+            if q == where:
+                assert t.square_norm() == 0.0
+            else:
+                assert_same_tree(t.export(), one.export(), tol=0.0)
