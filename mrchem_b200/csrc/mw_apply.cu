@@ -1541,10 +1541,12 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
     if (lined) {
         const int ntri = scan_total(ctx, d_ntrip, d_toff, ncand);
         const size_t tcap = (size_t)std::max(1, ntri);
-        d_tri = (unsigned long long*)dalloc(ctx, 4 * sizeof(unsigned long long) * tcap);
-        unsigned long long *d_tkey_in = d_tri, *d_tval_in = d_tri + tcap;
-        d_tkey = d_tri + 2 * tcap;
-        d_tval = d_tri + 3 * tcap;
+        // the sorted triples stay for the contraction, the unsorted ones go before its partial blocks are allocated
+        d_tri = (unsigned long long*)dalloc(ctx, 2 * sizeof(unsigned long long) * tcap);
+        unsigned long long* d_tkey_in = (unsigned long long*)dalloc(ctx, 2 * sizeof(unsigned long long) * tcap);
+        unsigned long long* d_tval_in = d_tkey_in + tcap;
+        d_tkey = d_tri;
+        d_tval = d_tri + tcap;
         if (ntri > 0) {
             k_texpand<<<(ncand + 255) / 256, 256, 0, s>>>(d_offs, d_cand_item, ncand, d_items, d_trees, d_cdelta, d_ntrip,
                                                           d_toff, d_csrc, d_tkey_in, d_tval_in, d_terr);
@@ -1558,6 +1560,7 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
             dfree(ctx, d_tmp);
             count(ctx, 2);
         }
+        dfree(ctx, d_tkey_in);
         k_tchunks<<<(ni * 32 + 127) / 128, 128, 0, s>>>(d_offs, d_toff, ni, d_tkey, chunk_limit, 0, d_nchunk, nullptr, nullptr);
         count(ctx);
         scan_only(ctx, d_nchunk, d_choff, ni);
