@@ -268,23 +268,7 @@ Op::~Op() {
     if (!mra) return;
     Ctx* c = mra->ctx;
     cudaSetDevice(c->device);
-    for (auto& kv : depths) {
-        dfree(c, kv.second->d_mats);
-        dfree(c, kv.second->d_mats32);
-        dfree(c, kv.second->d_matsb);
-        dfree(c, kv.second->d_matsb32);
-        dfree(c, kv.second->d_matsD);
-        dfree(c, kv.second->d_matsT32);
-        dfree(c, kv.second->d_matsE);
-        dfree(c, kv.second->d_matsbT32);
-        dfree(c, kv.second->d_matsI);
-        dfree(c, kv.second->d_matsbI);
-        dfree(c, kv.second->d_matsS32);
-        dfree(c, kv.second->d_matsbS32);
-        dfree(c, kv.second->d_matsX);
-        dfree(c, kv.second->d_deltas);
-        dfree(c, kv.second->d_terms);
-    }
+    depths.clear();
     cudaStreamSynchronize(c->stream);
 }
 
@@ -357,7 +341,7 @@ static std::unique_ptr<OpDepth> derivative_depth(Op& op, int depth, int dir) {
         rows.emplace_back(dr, tr);
     }
     std::stable_sort(rows.begin(), rows.end(), [](const auto& a, const auto& b) { return a.first.maxb > b.first.maxb; });
-    auto od = std::make_unique<OpDepth>();
+    auto od = std::make_unique<OpDepth>(m.ctx);
     std::vector<DeltaRec> deltas;
     std::vector<TermRec> terms;
     for (auto& r : rows) {
@@ -379,13 +363,10 @@ static std::unique_ptr<OpDepth> derivative_depth(Op& op, int depth, int dir) {
     od->d_terms = up(terms);
     std::vector<int2> src;
     for (int q = 0; q < 4; ++q) src.push_back(int2{q, 0});
-    double* d_blocks = up(mats);
-    int2* d_src = up(src);
-    double* d_beta = up(std::vector<double>(4, 1.0));
-    op_images(ctx, K2, *od, 4, d_src, d_blocks, d_beta);
-    dfree(ctx, d_blocks);
-    dfree(ctx, d_src);
-    dfree(ctx, d_beta);
+    Scratch sc(ctx);
+    const double* d_blocks = sc.up(mats);
+    const int2* d_src = sc.up(src);
+    op_images(ctx, K2, *od, 4, d_src, d_blocks, sc.up(std::vector<double>(4, 1.0)));
     return od;
 }
 

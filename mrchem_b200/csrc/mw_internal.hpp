@@ -110,7 +110,12 @@ struct TermRec {
     double bound;
 };
 
-struct OpDepth {
+struct OpDepth {  // owns its device arrays
+    Ctx* ctx;
+    explicit OpDepth(Ctx* c) : ctx(c) {}
+    OpDepth(const OpDepth&) = delete;
+    OpDepth& operator=(const OpDepth&) = delete;
+    ~OpDepth();
     std::vector<double> maxb;   // the offsets' largest bounds, descending (the order of d_deltas)
     double* d_mats = nullptr;   // NS matrices, (2k)^2 each
     float* d_mats32 = nullptr;  // FP32 copy of d_mats (mixed-precision apply)
@@ -183,6 +188,40 @@ void dfree(Ctx* ctx, void* p);
 void upload_bytes(Ctx* ctx, void* dst, const void* src, size_t bytes);
 // the same on stream s: through the arena when s is the context's stream, else a pageable copy on s
 void upload_bytes(Ctx* ctx, cudaStream_t s, void* dst, const void* src, size_t bytes);
+// device memory of one scope: given back (in stream order) when the scope is left, also by an exception
+class Scratch {
+public:
+    explicit Scratch(Ctx* ctx) : ctx_(ctx) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    ~Scratch() { release(); }
+    template <typename T>
+    T* get(size_t n) {
+        p_.push_back(nullptr);
+        p_.back() = dalloc(ctx_, sizeof(T) * (n > 0 ? n : 1));
+        return static_cast<T*>(p_.back());
+    }
+    template <typename T>
+    T* up(const std::vector<T>& v) {
+        T* d = get<T>(v.size());
+        upload_bytes(ctx_, d, v.data(), sizeof(T) * v.size());
+        return d;
+    }
+    void release() {
+        for (void* p : p_) dfree(ctx_, p);
+        p_.clear();
+    }
+    void keep() { p_.clear(); }  // the arrays have another owner now
+
+private:
+    Ctx* ctx_;
+    std::vector<void*> p_;
+};
+inline OpDepth::~OpDepth() {
+    for (void* p : std::initializer_list<void*>{d_mats, d_mats32, d_matsb, d_matsb32, d_matsD, d_matsE, d_matsT32, d_matsbT32, d_matsI,
+                                                d_matsbI, d_matsS32, d_matsbS32, d_matsX, d_deltas, d_terms})
+        dfree(ctx, p);
+}
 // several small host arrays to the device in one transfer: add() returns an array's offset, send() a device buffer of all
 // of them (the caller frees it); the arrays may go when send() returns
 class UploadPack {

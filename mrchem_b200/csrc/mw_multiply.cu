@@ -444,8 +444,9 @@ void build_grid(Tree& out, Tree& inp) {
     const size_t BS = out.mra->bsize();
     if (out.n == 0) trees_make_roots({&out});
     if (inp.n == 0) return;
-    uint64_t* d_add = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * (inp.n + 1));
-    int* d_n = (int*)dalloc(ctx, sizeof(int) * 33);
+    Scratch sc(ctx);
+    uint64_t* d_add = sc.get<uint64_t>(inp.n + 1);
+    int* d_n = sc.get<int>(33);
     k_grid_missing<<<1, 1024, 0, s>>>(inp.key, inp.n, out.hkey, out.hval, out.hcap, d_add, d_n);
     MWB_CUDA(cudaGetLastError());
     ctx->launches++;
@@ -453,35 +454,39 @@ void build_grid(Tree& out, Tree& inp) {
     readback(ctx, {{&na, d_n, sizeof(int)}});
     if (na > 0) {
         const int n0 = out.n, n = n0 + na;
-        Tree m;  // the merged arrays, with room to grow
-        m.mra = nullptr;
+        // the merged arrays, with room to grow; they and a larger index are all there before the tree takes them
         const int cap = n > out.cap ? std::max(n, 2 * out.cap) : out.cap;
-        m.key = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * cap);
-        m.parent = (int*)dalloc(ctx, sizeof(int) * cap);
-        m.child0 = (int*)dalloc(ctx, sizeof(int) * cap);
-        m.coef = (double*)dalloc(ctx, sizeof(double) * BS * cap);
-        m.norm2 = (double*)dalloc(ctx, sizeof(double) * cap);
-        m.wnorm2 = (double*)dalloc(ctx, sizeof(double) * cap);
+        uint32_t hcap = std::max(out.hcap, 1024u);  // hash index at most half full
+        while (hcap < 2u * (uint32_t)n) hcap <<= 1;
+        Scratch neu(ctx);
+        uint64_t* key = neu.get<uint64_t>(cap);
+        int* parent = neu.get<int>(cap);
+        int* child0 = neu.get<int>(cap);
+        double* coef = neu.get<double>(BS * cap);
+        double* norm2 = neu.get<double>(cap);
+        double* wnorm2 = neu.get<double>(cap);
+        uint64_t* hkey = hcap > out.hcap ? neu.get<uint64_t>(hcap) : nullptr;
+        int* hval = hcap > out.hcap ? neu.get<int>(hcap) : nullptr;
         k_grid_merge<<<n, 256, 0, s>>>(GridArrays{out.key, out.coef, out.norm2, out.wnorm2}, n0, d_add, na, BS,
-                                       GridArrays{m.key, m.coef, m.norm2, m.wnorm2});
+                                       GridArrays{key, coef, norm2, wnorm2});
         MWB_CUDA(cudaGetLastError());
-        std::swap(out.key, m.key);
-        std::swap(out.parent, m.parent);
-        std::swap(out.child0, m.child0);
-        std::swap(out.coef, m.coef);
-        std::swap(out.norm2, m.norm2);
-        std::swap(out.wnorm2, m.wnorm2);
-        for (void* p : {(void*)m.key, (void*)m.parent, (void*)m.child0, (void*)m.coef, (void*)m.norm2, (void*)m.wnorm2}) dfree(ctx, p);
+        neu.keep();
+        auto take = [&](auto*& old, auto* fresh) {
+            dfree(ctx, old);
+            old = fresh;
+        };
+        take(out.key, key);
+        take(out.parent, parent);
+        take(out.child0, child0);
+        take(out.coef, coef);
+        take(out.norm2, norm2);
+        take(out.wnorm2, wnorm2);
         out.cap = cap;
         out.n = n;
-        uint32_t hneed = 1024;  // hash index at most half full
-        while (hneed < 2u * (uint32_t)n) hneed <<= 1;
-        if (hneed > out.hcap) {
-            dfree(ctx, out.hkey);
-            dfree(ctx, out.hval);
-            out.hcap = hneed;
-            out.hkey = (uint64_t*)dalloc(ctx, sizeof(uint64_t) * out.hcap);
-            out.hval = (int*)dalloc(ctx, sizeof(int) * out.hcap);
+        if (hcap > out.hcap) {
+            take(out.hkey, hkey);
+            take(out.hval, hval);
+            out.hcap = hcap;
         }
         launch_hash_reset(out, s);
         launch_hash_insert(out, 0, n, s);
@@ -494,8 +499,6 @@ void build_grid(Tree& out, Tree& inp) {
         for (int d = 0; d < 32 && (d == 0 || level[d] < n); ++d) out.level_begin.push_back(level[d]);
         out.level_begin.push_back(n);
     }
-    dfree(ctx, d_add);
-    dfree(ctx, d_n);
 }
 
 // split flags of the last levels of several trees in one launch: item q = (tree, node)

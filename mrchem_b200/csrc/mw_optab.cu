@@ -437,12 +437,6 @@ template <typename T>
 T* alloc(Ctx* ctx, size_t n) {
     return (T*)dalloc(ctx, sizeof(T) * std::max<size_t>(1, n));
 }
-template <typename T>
-T* up(Ctx* ctx, const std::vector<T>& v) {
-    T* d = alloc<T>(ctx, v.size());
-    upload_bytes(ctx, d, v.data(), sizeof(T) * v.size());
-    return d;
-}
 int bits_for(int n) {
     int b = 1;
     while ((1 << b) < n) ++b;
@@ -453,9 +447,9 @@ template <typename T>
 void exclusive_sum(Ctx* ctx, const int* in, T* out, int n) {
     size_t tmp = 0;
     MWB_CUDA(cub::DeviceScan::ExclusiveScan(nullptr, tmp, in, out, ::cuda::std::plus<>{}, T(0), n, ctx->stream));
-    void* d = dalloc(ctx, tmp);
+    Scratch sc(ctx);
+    void* d = sc.get<char>(tmp);
     MWB_CUDA(cub::DeviceScan::ExclusiveScan(d, tmp, in, out, ::cuda::std::plus<>{}, T(0), n, ctx->stream));
-    dfree(ctx, d);
 }
 template <typename KT>
 void sort_pairs(Ctx* ctx, bool descending, const KT* kin, KT* kout, const int* vin, int* vout, int n, int b0, int b1) {
@@ -466,9 +460,8 @@ void sort_pairs(Ctx* ctx, bool descending, const KT* kin, KT* kout, const int* v
                           : cub::DeviceRadixSort::SortPairs(d, tmp, kin, kout, vin, vout, n, b0, b1, s);
     };
     MWB_CUDA(call(nullptr));
-    void* d = dalloc(ctx, tmp);
-    MWB_CUDA(call(d));
-    dfree(ctx, d);
+    Scratch sc(ctx);
+    MWB_CUDA(call(sc.get<char>(tmp)));
 }
 int blocks_of(long long n, int per) { return (int)((n + per - 1) / per); }
 
@@ -537,11 +530,12 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         if (ops[o]->terms.size() > 4096) throw Error(-4, "more than 4096 operator terms");
     }
     const int nt = (int)terms.size();
-    OpTerm* d_terms = up(ctx, terms);
-    double* d_ns = alloc<double>(ctx, (size_t)nt * lcap * K2 * K2);
-    double* d_t2 = alloc<double>(ctx, (size_t)nt * lcap);
-    double* d_x2 = alloc<double>(ctx, (size_t)nt * lcap);
-    int* d_flag = alloc<int>(ctx, 1);
+    Scratch sc(ctx);
+    OpTerm* d_terms = sc.up(terms);
+    double* d_ns = sc.get<double>((size_t)nt * lcap * K2 * K2);
+    double* d_t2 = sc.get<double>((size_t)nt * lcap);
+    double* d_x2 = sc.get<double>((size_t)nt * lcap);
+    int* d_flag = sc.get<int>(1);
     MWB_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
     const int cuts[4] = {0, std::min(4, lcap), std::min(12, lcap), lcap};
     for (int q = 0; q < 3; ++q) {
@@ -573,12 +567,8 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
             B0 = std::max(B0, terms[t].beta * std::pow(a2[(size_t)t * lcap] + b2[(size_t)t * lcap], 1.5));
         }
     }
-    std::vector<void*> tmp{d_terms, d_ns, d_t2, d_x2, d_flag};
-    auto release = [&] {
-        for (void* p : tmp) dfree(ctx, p);
-    };
     if (flag) {  // a band wider than the scratch: once more with all of it
-        release();
+        sc.release();
         if (lcap > kMaxBand) throw Error(-4, "operator band wider than 1024 offsets per direction");
         for (Op* o : ops) op_build_group({o}, depth, 8 * lcap);
         return;
@@ -595,10 +585,7 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         nrows += (long long)(2 * t.L + 1) * (2 * t.L + 1);
         nmat[t.op] += 2 * t.L + 1;
     }
-    if (lm > kMaxBand) {
-        release();
-        throw Error(-4, "operator band wider than 1024 offsets per direction");
-    }
+    if (lm > kMaxBand) throw Error(-4, "operator band wider than 1024 offsets per direction");
     upload_bytes(ctx, d_terms, terms.data(), sizeof(OpTerm) * nt);
     // lists
     const int bits = bits_for(2 * lm + 1), obits = bits_for(nop);
@@ -608,9 +595,8 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
     long long* d_offs = nullptr;
     std::vector<long long> first(nop + 1, 0);
     if (nrows > 0 && plan == OpPlan::together) {
-        d_cnt = alloc<int>(ctx, nrows + 1);
-        d_offs = alloc<long long>(ctx, nrows + 1);
-        tmp.insert(tmp.end(), {(void*)d_cnt, (void*)d_offs});
+        d_cnt = sc.get<int>(nrows + 1);
+        d_offs = sc.get<long long>(nrows + 1);
         MWB_CUDA(cudaMemsetAsync(d_cnt + nrows, 0, sizeof(int), s));
         k_op_list<<<blocks_of(nrows, 128), 128, 0, s>>>(d_terms, nt, nrows, d_t2, d_x2, lcap, root, lm, bits, d_cnt, nullptr,
                                                         nullptr, nullptr, nullptr);
@@ -627,14 +613,14 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         plan = op_plan_records(nop, first[nop]);
     }
     if (plan != OpPlan::together) {
-        release();
+        sc.release();
         if (plan == OpPlan::refuse) throw Error(-4, "operator offset list too large");
         for (Op* o : ops) op_build_group({o}, depth, lcap);
         return;
     }
     std::vector<std::unique_ptr<OpDepth>> ods;
     for (int o = 0; o < nop; ++o) {
-        ods.push_back(std::make_unique<OpDepth>());
+        ods.push_back(std::make_unique<OpDepth>(ctx));
         std::vector<int2> src;
         std::vector<double> beta;
         for (int t = t0[o]; t < t0[o + 1]; ++t)
@@ -642,11 +628,9 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
                 src.push_back(int2{t * lcap + std::abs(l), l < 0 ? 1 : 0});
                 beta.push_back(terms[t].beta);
             }
-        int2* d_src = up(ctx, src);
-        double* d_beta = up(ctx, beta);
-        op_images(ctx, K2, *ods[o], nmat[o], d_src, d_ns, d_beta);
-        dfree(ctx, d_src);
-        dfree(ctx, d_beta);
+        Scratch lists(ctx);
+        const int2* d_src = lists.up(src);
+        op_images(ctx, K2, *ods[o], nmat[o], d_src, d_ns, lists.up(beta));
     }
     std::vector<int> rec0(first.begin(), first.end()), del0(nop + 1, 0);
     std::vector<double> maxb;
@@ -654,17 +638,16 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         const int nrec = rec0[nop];
         const int rb = blocks_of(nrec, 256);
         if (nrec > 0) {
-            auto* d_key = alloc<unsigned long long>(ctx, nrec);
-            auto* d_key2 = alloc<unsigned long long>(ctx, nrec);
-            auto* d_key3 = alloc<unsigned long long>(ctx, nrec);
-            double* d_bound = alloc<double>(ctx, nrec);
-            double* d_b2 = alloc<double>(ctx, nrec);
-            int* d_term = alloc<int>(ctx, nrec);
-            int* d_i0 = alloc<int>(ctx, nrec);
-            int* d_i1 = alloc<int>(ctx, nrec);
-            int* d_head = alloc<int>(ctx, nrec + 1);
-            int* d_hpos = alloc<int>(ctx, nrec + 1);
-            tmp.insert(tmp.end(), {d_key, d_key2, d_key3, d_bound, d_b2, d_term, d_i0, d_i1, d_head, d_hpos});
+            auto* d_key = sc.get<unsigned long long>(nrec);
+            auto* d_key2 = sc.get<unsigned long long>(nrec);
+            auto* d_key3 = sc.get<unsigned long long>(nrec);
+            double* d_bound = sc.get<double>(nrec);
+            double* d_b2 = sc.get<double>(nrec);
+            int* d_term = sc.get<int>(nrec);
+            int* d_i0 = sc.get<int>(nrec);
+            int* d_i1 = sc.get<int>(nrec);
+            int* d_head = sc.get<int>(nrec + 1);
+            int* d_hpos = sc.get<int>(nrec + 1);
             k_op_list<<<blocks_of(nrows, 128), 128, 0, s>>>(d_terms, nt, nrows, d_t2, d_x2, lcap, root, lm, bits, d_cnt, d_offs,
                                                             d_key, d_bound, d_term);
             k_op_iota<<<rb, 256, 0, s>>>(nrec, d_i0);
@@ -690,16 +673,15 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
                 ods[o]->d_deltas = alloc<DeltaRec>(ctx, del0[o + 1] - del0[o]);
                 outs[o] = OpOut{ods[o]->d_terms, ods[o]->d_deltas, rec0[o], del0[o]};
             }
-            OpOut* d_outs = up(ctx, outs);
-            double* d_dmax = alloc<double>(ctx, nd);
-            double* d_dm2 = alloc<double>(ctx, nd);
-            double* d_maxb = alloc<double>(ctx, nd);
-            int* d_df = alloc<int>(ctx, nd);
-            int* d_o0 = alloc<int>(ctx, nd);
-            int* d_o1 = alloc<int>(ctx, nd);
-            int* d_k0 = alloc<int>(ctx, nd);
-            int* d_k1 = alloc<int>(ctx, nd);
-            tmp.insert(tmp.end(), {d_outs, d_dmax, d_dm2, d_maxb, d_df, d_o0, d_o1, d_k0, d_k1});
+            OpOut* d_outs = sc.up(outs);
+            double* d_dmax = sc.get<double>(nd);
+            double* d_dm2 = sc.get<double>(nd);
+            double* d_maxb = sc.get<double>(nd);
+            int* d_df = sc.get<int>(nd);
+            int* d_o0 = sc.get<int>(nd);
+            int* d_o1 = sc.get<int>(nd);
+            int* d_k0 = sc.get<int>(nd);
+            int* d_k1 = sc.get<int>(nd);
             k_op_terms<<<rb, 256, 0, s>>>(nrec, d_key3, bits, d_i0, d_bound, d_term, d_terms, d_head, d_hpos, d_outs, lm, d_dmax, d_df);
             k_op_iota<<<db, 256, 0, s>>>(nd, d_o0);
             sort_pairs(ctx, true, reinterpret_cast<const unsigned long long*>(d_dmax), reinterpret_cast<unsigned long long*>(d_dm2),
@@ -724,7 +706,6 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         std::lock_guard<std::mutex> g(ops[o]->mtx);
         ops[o]->depths.emplace(depth, std::move(ods[o]));
     }
-    release();
 }
 
 void op_build_tables(const std::vector<Op*>& ops, int depth) {
