@@ -408,17 +408,7 @@ static void op_init(Op& op, Mra* m, double mu, double prec) {
     r_max = std::sqrt(r_max);
     const double r_min = 0.01 * std::ldexp(root_edge, -m->max_depth);
     op.terms = kernel_expansion(mu, op.eps, r_min, r_max);
-    if (!m->builder) {  // the construction's basis tables, with the world's first operator
-        m->builder = std::make_unique<GaussianOperatorBuilder>(m->basis, m->F);
-        auto up = [&](const std::vector<double>& v) {
-            double* d = (double*)dalloc(m->ctx, sizeof(double) * v.size());
-            upload_bytes(m->ctx, d, v.data(), sizeof(double) * v.size());
-            return d;
-        };
-        m->d_cc = up(m->builder->device_coefficients());
-        m->d_px = up(m->builder->rule_x());
-        m->d_pw = up(m->builder->rule_w());
-    }
+    world_operator_tables(*m);
 }
 
 // ---------------------------------------------------------------------------------------------

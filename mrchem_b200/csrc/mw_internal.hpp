@@ -222,6 +222,20 @@ inline OpDepth::~OpDepth() {
                                                 d_matsbI, d_matsS32, d_matsbS32, d_matsX, d_deltas, d_terms})
         dfree(ctx, p);
 }
+// The basis tables of the operators' construction, with the world's first operator.  The builder marks them as there, so it
+// is set last: after a failed allocation the world has none of them and its next operator tries again
+inline void world_operator_tables(Mra& m) {
+    if (m.builder) return;
+    auto b = std::make_unique<GaussianOperatorBuilder>(m.basis, m.F);
+    Scratch t(m.ctx);
+    double* cc = t.up(b->device_coefficients());
+    double* px = t.up(b->rule_x());
+    m.d_pw = t.up(b->rule_w());
+    m.d_cc = cc;
+    m.d_px = px;
+    t.keep();
+    m.builder = std::move(b);
+}
 // several small host arrays to the device in one transfer: add() returns an array's offset, send() a device buffer of all
 // of them (the caller frees it); the arrays may go when send() returns
 class UploadPack {
