@@ -370,25 +370,15 @@ static std::unique_ptr<OpDepth> derivative_depth(Op& op, int depth, int dir) {
     return od;
 }
 
-// the tables of one depth, for all operators of a batch that lack them
-static void op_require(Op** op, int n, int depth) {
-    std::vector<Op*> need;
-    for (int i = 0; i < n; ++i) {
-        if (!op[i] || op[i]->kind != 0) continue;
-        std::lock_guard<std::mutex> g(op[i]->mtx);
-        if (op[i]->depths.find(depth) == op[i]->depths.end() && std::find(need.begin(), need.end(), op[i]) == need.end())
-            need.push_back(op[i]);
-    }
-    if (need.empty()) return;
-    if (depth > 0) op_require(need.data(), (int)need.size(), 0);  // the operator scale B0
-    op_build_tables(need, depth);
+static void op_require(Op* const* op, int n, int depth) {
+    if (n > 0) op_require(*op[0]->mra, op, n, depth, op_build_tables);
 }
 static const OpDepth& op_depth(Op& op, int depth, int dir = 0) {
     if (op.kind == 0) {
         Op* p = &op;
         op_require(&p, 1, depth);
     }
-    std::lock_guard<std::mutex> g(op.mtx);
+    std::lock_guard<std::mutex> g(op.mra->op_mtx);
     const int ckey = op.kind == 1 ? 3 * depth + dir : depth;
     auto it = op.depths.find(ckey);
     if (it == op.depths.end()) it = op.depths.emplace(ckey, derivative_depth(op, depth, dir)).first;

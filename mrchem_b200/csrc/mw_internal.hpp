@@ -3,6 +3,7 @@
 #include <initializer_list>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <map>
@@ -90,6 +91,7 @@ struct Mra {
     double* d_cc = nullptr;
     double* d_px = nullptr;
     double* d_pw = nullptr;
+    std::mutex op_mtx;  // the tables above and those of the world's operators: held from the look for one to its insertion
     double* d_MV = nullptr;  // evaluation matrix blkdiag(E, E) * F^T (pointwise product)
     // trees and operators that point here; a destroyed world is freed with the last of them
     int refs = 0;
@@ -155,8 +157,7 @@ struct Op {
     double mu = 0.0, prec = 0.0, eps = 0.0;
     std::vector<GaussTerm> terms;
     double B0 = 0.0;  // operator scale, from the root depth's tables
-    std::map<int, std::unique_ptr<OpDepth>> depths;
-    std::mutex mtx;
+    std::map<int, std::unique_ptr<OpDepth>> depths;  // under the world's op_mtx
     ~Op();
 };
 
@@ -225,6 +226,7 @@ inline OpDepth::~OpDepth() {
 // The basis tables of the operators' construction, with the world's first operator.  The builder marks them as there, so it
 // is set last: after a failed allocation the world has none of them and its next operator tries again
 inline void world_operator_tables(Mra& m) {
+    std::lock_guard<std::mutex> g(m.op_mtx);
     if (m.builder) return;
     auto b = std::make_unique<GaussianOperatorBuilder>(m.basis, m.F);
     Scratch t(m.ctx);
@@ -235,6 +237,24 @@ inline void world_operator_tables(Mra& m) {
     m.d_px = px;
     t.keep();
     m.builder = std::move(b);
+}
+// The tables of one depth for all convolution operators of a batch (one world) that lack them, each made once:
+// build(ops, depth) makes and inserts them.  The root's come first, they hold the operator scale B0
+template <typename Build>
+void op_require(Mra& m, Op* const* op, int n, int depth, Build&& build) {
+    auto missing = [&](int d) {
+        std::vector<Op*> need;
+        for (int i = 0; i < n; ++i)
+            if (op[i] && op[i]->kind == 0 && op[i]->depths.count(d) == 0 && std::find(need.begin(), need.end(), op[i]) == need.end())
+                need.push_back(op[i]);
+        return need;
+    };
+    std::lock_guard<std::mutex> g(m.op_mtx);
+    if (missing(depth).empty()) return;
+    for (int d : {0, depth}) {
+        const std::vector<Op*> need = missing(d);
+        if (!need.empty()) build(need, d);
+    }
 }
 // several small host arrays to the device in one transfer: add() returns an array's offset, send() a device buffer of all
 // of them (the caller frees it); the arrays may go when send() returns

@@ -509,7 +509,7 @@ void op_images(Ctx* ctx, int K2, OpDepth& od, int nmat, const int2* d_src, const
     ctx->launches++;
 }
 
-// tables of one depth for several convolution operators of one world, none of which has them yet
+// tables of one depth for several convolution operators of one world, none of which has them yet (under its op_mtx)
 static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
     const Mra& m = *ops[0]->mra;
     Ctx* ctx = m.ctx;
@@ -703,7 +703,6 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         if (!od.d_terms) od.d_terms = alloc<TermRec>(ctx, 0);
         if (!od.d_deltas) od.d_deltas = alloc<DeltaRec>(ctx, 0);
         od.maxb.assign(maxb.begin() + del0[o], maxb.begin() + del0[o + 1]);
-        std::lock_guard<std::mutex> g(ops[o]->mtx);
         ops[o]->depths.emplace(depth, std::move(ods[o]));
     }
 }
