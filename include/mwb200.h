@@ -182,16 +182,21 @@ int mw_apply_derivative(mw_tree out, mw_op op, mw_tree inp, int dir, int flags);
 int mw_op_destroy(mw_op op);
 int mw_op_nterms(mw_op op, int* n);
 int mw_op_terms(mw_op op, double* alpha, double* beta);
-/* The operator's 1-D matrices, evaluated on the host by the formulas of the device tables that the
- * contraction reads (for verification against independent quadrature; no reference counterpart, MRCPP
- * keeps them internal to its OperatorCalculator):
+/* The operator's 1-D matrices (for verification against independent quadrature; no reference counterpart,
+ * MRCPP keeps them internal to its OperatorCalculator):
  * T^n(l) (k x k, row-major) of exp(-alpha x^2) between scaling functions at scale n, translation
- * offset l -- entry (i, j) = 2^-n int_0^1 int_0^1 phi_i(u) phi_j(v) exp(-alpha 4^-n (u - v + l)^2);
+ * offset l -- entry (i, j) = 2^-n int_0^1 int_0^1 phi_i(u) phi_j(v) exp(-alpha 4^-n (u - v + l)^2) --
+ * evaluated on the host, by the formulas of the device tables;
  * and the non-standard-form matrix (2k x 2k, rows = output scaling|wavelet, columns = input) of term
  * `term` at scale n, offset l: F [[T(2l) T(2l-1)]; [T(2l+1) T(2l)]]_{n+1} F^T with the world's two-scale
- * filter F (mw_mra_filter). */
+ * filter F (mw_mra_filter).  Where the operator holds tables (below) it is read back from the device
+ * table of the FP64 contraction; elsewhere it is evaluated on the host.
+ * mw_op_band: half width L of the band of offsets -L .. L that the tables hold for a term at scale n, -1
+ * for none (the term is inactive there, or n is no scale of the world).  Both calls build the tables of
+ * the scale if no apply has. */
 int mw_op_scaling_matrix(mw_op op, double alpha, int n, long long l, double* T);
 int mw_op_ns_matrix(mw_op op, int term, int n, long long l, double* NS);
+int mw_op_band(mw_op op, int term, int n, int* half);
 
 /* out = op * inp, adaptive.  Replaces mrcpp::apply(prec, out, op, inp): reference
  * src/scf_solver/HelmholtzVector.cpp:176,180, src/qmoperators/two_electron/CoulombPotential.cpp:85,

@@ -385,6 +385,19 @@ static const OpDepth& op_depth(Op& op, int depth, int dir = 0) {
     return *it->second;
 }
 
+// the tables at scale n if the operator has some there: the scale is one of the world's, and the tables can be built
+static const OpDepth* op_tables_at(Op& op, int n) {
+    const int depth = n - op.mra->n0;
+    if (depth < 0 || depth > op.mra->depth_limit) return nullptr;
+    MWB_CUDA(cudaSetDevice(op.mra->ctx->device));
+    try {
+        return &op_depth(op, depth);
+    } catch (const Error& e) {
+        if (e.code == MW_ERR_CAPACITY) return nullptr;  // lists beyond the limits
+        throw;
+    }
+}
+
 static void op_init(Op& op, Mra* m, double mu, double prec) {
     if (!(prec > 0.0)) throw Error(MW_ERR_ARG, "operator precision must be positive");
     if (mu < 0.0) throw Error(MW_ERR_ARG, "mu must be non-negative");
@@ -1506,13 +1519,33 @@ int mw_op_scaling_matrix(mw_op op, double alpha, int n, long long l, double* T) 
     })
 }
 
+int mw_op_band(mw_op op, int term, int n, int* half) {
+    MW_TRY({
+        MW_ARG(op && half, "null pointer");
+        MW_ARG(op->kind == 0, "not a separated-Gaussian convolution operator");
+        MW_ARG(term >= 0 && term < (int)op->terms.size(), "term index out of range");
+        const OpDepth* od = op_tables_at(*op, n);
+        *half = od ? od->band[term] : -1;
+    })
+}
+
 int mw_op_ns_matrix(mw_op op, int term, int n, long long l, double* NS) {
     MW_TRY({
         MW_ARG(op && NS, "null pointer");
         MW_ARG(op->kind == 0, "not a separated-Gaussian convolution operator");
         MW_ARG(term >= 0 && term < (int)op->terms.size(), "term index out of range");
-        std::vector<std::pair<long, std::vector<double>>> cache;
-        op->mra->builder->ns(op->terms[term].alpha, n, (long)l, NS, cache);
+        const OpDepth* od = op_tables_at(*op, n);
+        if (od && l >= -od->band[term] && l <= od->band[term]) {  // the A fragments of the FP64 contraction
+            const int K2 = 2 * op->mra->k, RT = (K2 + 7) / 8, S = (K2 + 3) / 4;
+            std::vector<double> f((size_t)S * RT * 32);
+            const size_t mi = od->base[term] + (int)l + od->band[term];
+            readback(op->mra->ctx, {{f.data(), od->d_matsD + mi * f.size(), sizeof(double) * f.size()}});
+            for (int o = 0; o < K2; ++o)
+                for (int i = 0; i < K2; ++i) NS[o * K2 + i] = f[((i / 4) * RT + o / 8) * 32 + 4 * (o % 8) + i % 4];
+        } else {
+            std::vector<std::pair<long, std::vector<double>>> cache;
+            op->mra->builder->ns(op->terms[term].alpha, n, (long)l, NS, cache);
+        }
     })
 }
 

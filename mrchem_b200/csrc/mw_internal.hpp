@@ -119,6 +119,7 @@ struct OpDepth {  // owns its device arrays
     OpDepth& operator=(const OpDepth&) = delete;
     ~OpDepth();
     std::vector<double> maxb;   // the offsets' largest bounds, descending (the order of d_deltas)
+    std::vector<int> base, band;  // per term: its first matrix (offset -band) and its band's half width (-1: inactive)
     double* d_mats = nullptr;   // NS matrices, (2k)^2 each
     float* d_mats32 = nullptr;  // FP32 copy of d_mats (mixed-precision apply)
     double* d_matsb = nullptr;  // each matrix scaled by its term's beta (z-step operators)

@@ -702,6 +702,10 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         OpDepth& od = *ods[o];
         if (!od.d_terms) od.d_terms = alloc<TermRec>(ctx, 0);
         if (!od.d_deltas) od.d_deltas = alloc<DeltaRec>(ctx, 0);
+        for (int t = t0[o]; t < t0[o + 1]; ++t) {
+            od.base.push_back(terms[t].base);
+            od.band.push_back(terms[t].active ? terms[t].L : -1);
+        }
         od.maxb.assign(maxb.begin() + del0[o], maxb.begin() + del0[o + 1]);
         ops[o]->depths.emplace(depth, std::move(ods[o]));
     }

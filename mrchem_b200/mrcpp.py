@@ -60,6 +60,7 @@ SYMBOLS = [
     ("mw_mra_filter", ctypes.c_int, [_vp, _dp]),
     ("mw_op_scaling_matrix", ctypes.c_int, [_vp, ctypes.c_double, ctypes.c_int, ctypes.c_longlong, _dp]),
     ("mw_op_ns_matrix", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_longlong, _dp]),
+    ("mw_op_band", ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]),
     ("mw_mra_max_depth", ctypes.c_int, [_vp, _ip]),
     ("mw_tree_create", ctypes.c_int, [_vp, _vpp]),
     ("mw_tree_destroy", ctypes.c_int, [_vp]),
@@ -457,6 +458,12 @@ class ConvolutionOperator:
         NS = np.zeros((2 * k, 2 * k))
         _check(_lib.mw_op_ns_matrix(self._h, int(term), int(n), int(l), _d(NS)))
         return NS
+
+    def band(self, term, n):
+        """half width of the band of offsets held for a term at scale n, -1 for none (see mw_op_band)"""
+        half = ctypes.c_int()
+        _check(_lib.mw_op_band(self._h, int(term), int(n), ctypes.byref(half)))
+        return half.value
 
 
 class PoissonOperator(ConvolutionOperator):
