@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(BX<K, K>::NTHR, GenCfg<K>::MINB)
     long long t[3];
     key_trans(gkey & ((1ull << 57) - 1), t);
     bx_path_operators<K, false>(FT, nullptr, t, T.depth - key_depth(T.inkey[leaf]), X, f);
-    bx_load<K>(X, T.in.coef + (size_t)leaf * Geo<K>::BS);
+    bx_load<K, K>(X, T.in.coef + (size_t)leaf * Geo<K>::BS);
     cp_async_wait_all();
     __syncthreads();
     bx_slices<K, K>(X, f, f + B::FRAG);

@@ -111,7 +111,7 @@ __device__ __forceinline__ void bx_slice(double* X, int c, const double* fx, con
 }
 
 // z product of column tile q (one warp): v[r][h] = out at c' = 8 r + lane / 4, column 8 q + 2 (lane mod 4) + h of
-// (a', b').  nc: input slices that are not zero
+// (a', b')
 template <int K, int RO, int NQ>
 __device__ __forceinline__ void bx_z(const double* X, int q0, int dq, const double* fz, double (&v)[NQ][BX<K, RO>::RT][2]) {
     using C = BX<K, RO>;
@@ -155,10 +155,11 @@ __device__ __forceinline__ void bx_columns(const double* X, const double* fz, F&
     }
 }
 
-// a block from global memory (x fastest) into the shared layout, asynchronously
-template <int K>
+// a block from global memory (x fastest) into the shared layout, asynchronously, by the threads of a kernel whose products
+// are those of BX<K, RO> (which differ in number: at k = 9 to 11 eight warps against k)
+template <int K, int RO>
 __device__ __forceinline__ void bx_load(double* X, const double* __restrict__ blk) {
-    using C = BX<K, 2 * K>;
+    using C = BX<K, RO>;
     constexpr int H = K, N = C::K2 * C::K2 * H;  // 16-byte pairs
     for (int e = threadIdx.x; e < N; e += C::NTHR) {
         const int r = e / H, i = e - r * H, b = r % C::K2, c = r / C::K2;

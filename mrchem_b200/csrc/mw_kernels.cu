@@ -196,7 +196,7 @@ __device__ __forceinline__ void transform_node(int mode, int node, const TView& 
             else X[at(a, b, c)] = *src;
         }
     } else {
-        bx_load<K>(X, t.coef + (size_t)node * BS);
+        bx_load<K, K2>(X, t.coef + (size_t)node * BS);
     }
     cp_async_wait_all();
     __syncthreads();

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, MulCfg<K>::MINB)
             } else {
                 bx_path_operators<K, true>(FTg, MVg, tr, depth - da, X, fq);
             }
-            bx_load<K>(X, coef + (size_t)idx * BS);
+            bx_load<K, K2>(X, coef + (size_t)idx * BS);
         } else {  // outside the factor's roots (cannot happen on one world): zero
             for (int e = tid; e < B::VOL; e += B::NTHR) X[e] = 0.0;
             for (int e = tid; e < 3 * B::FRAG; e += B::NTHR) fq[e] = 0.0;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(BX<K, K>::NTHR, 1)
         }
         __syncthreads();  // X is free
         bx_path_operators<K, false>(FTg, nullptr, tr, depth - da, X, f);
-        bx_load<K>(X, blk);
+        bx_load<K, K>(X, blk);
         cp_async_wait_all();
         __syncthreads();
         bx_slices<K, K>(X, f, f + B::FRAG);
