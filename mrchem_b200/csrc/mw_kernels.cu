@@ -436,10 +436,15 @@ __global__ void k_rescale(double* coef, size_t n, double c) {
         coef[i] *= c;
 }
 
-// <a|b>: per node of a (four warps, so that a small block's loads are all in flight at once) the product over the wavelet part (all components at depth 0), then the last block to
-// finish adds the nodes' parts in a fixed order and writes the sum where the host reads it (mapped memory).  A second
-// launch for the sum, a copy and two scalar loads per element took twice as long.
-constexpr int kDotThreads = 256;
+// <a|b>: groups of four warps (so that a small block's loads are all in flight at once) take nodes of a in turn, the product
+// over the wavelet part (all components at depth 0), then the last block to finish adds the groups' parts in a fixed order
+// and writes the sum where the host reads it (mapped memory).  A second launch for the sum, a copy and two scalar loads per
+// element took twice as long.  A part for every node made the last block's loop over them a large share of the call on trees
+// of many small blocks, so below k = 8 the blocks are at most 8 per SM, whose groups take nodes in turn (64,000 nodes at
+// k = 4 141 -> 66 us, 34,264 at k = 5 103 -> 63).  From k = 8 up a group takes one node: a node's loads keep the SM busy, and
+// nodes in turn cost more than the loop saves (17,088 nodes at k = 10: 206 us, 258 in turn).
+constexpr int kDotThreads = 256, kDotGroups = kDotThreads / 128;
+constexpr bool dot_in_turn(int k) { return k < 8; }
 template <int K>
 __global__ void __launch_bounds__(kDotThreads) k_dot(TView a, int na, const double* __restrict__ bcoef, const uint64_t* hk,
                                                      const int* hv, uint32_t hcap, double* part, unsigned* ticket, double* out) {
@@ -447,31 +452,35 @@ __global__ void __launch_bounds__(kDotThreads) k_dot(TView a, int na, const doub
     __shared__ double red[64];
     __shared__ unsigned done;
     __shared__ double ws[kDotThreads / 32];
-    const int node = blockIdx.x * (kDotThreads / 128) + threadIdx.x / 128, t = threadIdx.x & 127;
+    const int group = blockIdx.x * kDotGroups + threadIdx.x / 128, ngroup = gridDim.x * kDotGroups, t = threadIdx.x & 127;
     double s = 0.0;
-    if (node < na) {
+    auto add = [&](int node) {
         const uint64_t key = a.key[node];
         const int j = hlookup(hk, hv, hcap, key);
-        if (j >= 0) {
-            const bool root = key_depth(key) == 0;
-            const double2* x = reinterpret_cast<const double2*>(a.coef + (size_t)node * G::BS);
-            const double2* y = reinterpret_cast<const double2*>(bcoef + (size_t)j * G::BS);
+        if (j < 0) return;
+        const bool root = key_depth(key) == 0;
+        const double2* x = reinterpret_cast<const double2*>(a.coef + (size_t)node * G::BS);
+        const double2* y = reinterpret_cast<const double2*>(bcoef + (size_t)j * G::BS);
 #pragma unroll 8
-            for (int e = t; e < G::BS / 2; e += 128) {
-                const double2 u = x[e], v = y[e];
-                const int aa = 2 * (e % K), bb = (e / K) % G::K2, cc = e / (K * G::K2);
-                const bool sc = !root && bb < K && cc < K;
-                if (!(sc && aa < K)) s = fma(u.x, v.x, s);
-                if (!(sc && aa + 1 < K)) s = fma(u.y, v.y, s);
-            }
+        for (int e = t; e < G::BS / 2; e += 128) {
+            const double2 u = x[e], v = y[e];
+            const int aa = 2 * (e % K), bb = (e / K) % G::K2, cc = e / (K * G::K2);
+            const bool sc = !root && bb < K && cc < K;
+            if (!(sc && aa < K)) s = fma(u.x, v.x, s);
+            if (!(sc && aa + 1 < K)) s = fma(u.y, v.y, s);
         }
+    };
+    if constexpr (dot_in_turn(K)) {
+        for (int node = group; node < na; node += ngroup) add(node);
+    } else {
+        if (group < na) add(group);
     }
     for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (t == 0 && node < na) {
+    if (t == 0) {
         const double* w = ws + (threadIdx.x >> 5);
-        part[node] = (w[0] + w[1]) + (w[2] + w[3]);
+        part[group] = (w[0] + w[1]) + (w[2] + w[3]);
     }
     __threadfence();
     __syncthreads();
@@ -481,7 +490,7 @@ __global__ void __launch_bounds__(kDotThreads) k_dot(TView a, int na, const doub
     __threadfence();
     double d = 0.0;
     s = 0.0;
-    for (int i = threadIdx.x; i < na; i += kDotThreads) s += __ldcg(part + i);
+    for (int i = threadIdx.x; i < ngroup; i += kDotThreads) s += __ldcg(part + i);
     block_sum2(s, d, red);
     if (threadIdx.x == 0) {
         *ticket = 0u;  // for the next call on this stream
@@ -795,12 +804,13 @@ double launch_dot(Tree& a, Tree& b, cudaStream_t s) {
         ctx->ticket = (unsigned*)dalloc(ctx, sizeof(unsigned));
         MWB_CUDA(cudaMemsetAsync(ctx->ticket, 0, sizeof(unsigned), s));
     }
-    double* part = (double*)dalloc(ctx, sizeof(double) * a.n);
+    int blocks = (a.n + kDotGroups - 1) / kDotGroups;
+    if (dot_in_turn(a.mra->k)) blocks = std::min(blocks, 8 * ctx->num_sms);
+    double* part = (double*)dalloc(ctx, sizeof(double) * kDotGroups * blocks);
     double* res = mailbox(ctx);
     TView av = view(a);
-#define L_DOT(KK)                                                                                                        \
-    k_dot<KK><<<(a.n + kDotThreads / 128 - 1) / (kDotThreads / 128), kDotThreads, 0, s>>>(av, a.n, b.coef, b.hkey, b.hval, b.hcap, part, \
-                                                                                 ctx->ticket, res);
+#define L_DOT(KK) \
+    k_dot<KK><<<blocks, kDotThreads, 0, s>>>(av, a.n, b.coef, b.hkey, b.hval, b.hcap, part, ctx->ticket, res);
     MWB_DISPATCH_K(a.mra->k, L_DOT)
 #undef L_DOT
     MWB_CUDA(cudaGetLastError());
