@@ -49,8 +49,6 @@ struct BTree {
     const TermRec* terms;
     const double* mats;
     const float* mats32;
-    const double* matsb;    // beta-scaled copies (z-step operators)
-    const float* matsb32;
     const double* matsD;      // fragment images (FP64 matrix-instruction contraction)
     const double* matsE;
     const float* matsT32;     // transposed, zero-padded copies (GEMM-tiled FP32 contraction)
@@ -1381,8 +1379,6 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
         d.terms = b.tab->d_terms;
         d.mats = b.tab->d_mats;
         d.mats32 = b.tab->d_mats32;
-        d.matsb = b.tab->d_matsb;
-        d.matsb32 = b.tab->d_matsb32;
         d.matsD = b.tab->d_matsD;
         d.matsE = b.tab->d_matsE;
         d.matsT32 = b.tab->d_matsT32;

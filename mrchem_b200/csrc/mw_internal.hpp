@@ -120,10 +120,8 @@ struct OpDepth {  // owns its device arrays
     ~OpDepth();
     std::vector<double> maxb;   // the offsets' largest bounds, descending (the order of d_deltas)
     std::vector<int> base, band;  // per term: its first matrix (offset -band) and its band's half width (-1: inactive)
-    double* d_mats = nullptr;   // NS matrices, (2k)^2 each
-    float* d_mats32 = nullptr;  // FP32 copy of d_mats (mixed-precision apply)
-    double* d_matsb = nullptr;  // each matrix scaled by its term's beta (z-step operators)
-    float* d_matsb32 = nullptr;
+    double* d_mats = nullptr;   // NS matrices, (2k)^2 each (pencil engine; the others read the forms below)
+    float* d_mats32 = nullptr;  // FP32 copy of d_mats
     // FP64 matrix-instruction contraction (k_dapply), RT = row tiles of 8, S = steps of 4, zero outside 2k:
     // every matrix as A fragments [s][r][lane 4 n + i] = M[8 r + n][4 s + i], and beta-scaled as B fragments
     // [j][s][lane 4 n + i] = beta M[8 j + 4 (n mod 2) + n / 2][4 s + i]
@@ -220,7 +218,7 @@ private:
     std::vector<void*> p_;
 };
 inline OpDepth::~OpDepth() {
-    for (void* p : std::initializer_list<void*>{d_mats, d_mats32, d_matsb, d_matsb32, d_matsD, d_matsE, d_matsT32, d_matsbT32, d_matsI,
+    for (void* p : std::initializer_list<void*>{d_mats, d_mats32, d_matsD, d_matsE, d_matsT32, d_matsbT32, d_matsI,
                                                 d_matsbI, d_matsS32, d_matsbS32, d_matsX, d_deltas, d_terms})
         dfree(ctx, p);
 }

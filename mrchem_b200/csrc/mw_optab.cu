@@ -341,8 +341,8 @@ __global__ void k_op_deltas(int n, const int* __restrict__ order, const int* __r
 // every engine's form of a matrix (layouts: OpDepth in mw_internal.hpp, XGeo in mw_slice.hpp).  src: block of
 // `blocks` and whether it is transposed (offset -l of offset l)
 struct OpImages {
-    double *mats, *matsb, *matsD, *matsE;
-    float *mats32, *matsb32, *matsT32, *matsbT32, *matsI, *matsbI, *matsS32, *matsbS32;
+    double *mats, *matsD, *matsE;
+    float *mats32, *matsT32, *matsbT32, *matsI, *matsbI, *matsS32, *matsbS32;
     unsigned char* matsX;
 };
 // FP32 -> TF32 (10 explicit mantissa bits), to nearest with ties away from zero; infinities and NaNs unchanged
@@ -363,11 +363,8 @@ __global__ void __launch_bounds__(128) k_op_images(const int2* __restrict__ src,
     __syncthreads();
     const size_t at = (size_t)mi * n2;
     for (int e = tid; e < n2; e += 128) {
-        const double v = M[e], w = b * v;
-        im.mats[at + e] = v;
-        im.matsb[at + e] = w;
-        im.mats32[at + e] = (float)v;
-        im.matsb32[at + e] = (float)w;
+        im.mats[at + e] = M[e];
+        im.mats32[at + e] = (float)M[e];
     }
     const int KP = (K2 + 3) / 4 * 4, RT = (K2 + 7) / 8, S = (K2 + 3) / 4, KP8 = RT * 8;
     auto val = [&](int o, int k) { return o < K2 && k < K2 ? M[o * K2 + k] : 0.0; };
@@ -486,9 +483,7 @@ void op_images(Ctx* ctx, int K2, OpDepth& od, int nmat, const int2* d_src, const
     const int KP = (K2 + 3) / 4 * 4, RT = (K2 + 7) / 8, S = (K2 + 3) / 4, KP8 = RT * 8;
     const size_t n = (size_t)nmat;
     od.d_mats = alloc<double>(ctx, n * K2 * K2);
-    od.d_matsb = alloc<double>(ctx, n * K2 * K2);
     od.d_mats32 = alloc<float>(ctx, n * K2 * K2);
-    od.d_matsb32 = alloc<float>(ctx, n * K2 * K2);
     od.d_matsT32 = alloc<float>(ctx, n * KP * KP);
     od.d_matsbT32 = alloc<float>(ctx, n * KP * KP);
     od.d_matsD = alloc<double>(ctx, n * RT * S * 32);
@@ -502,7 +497,7 @@ void op_images(Ctx* ctx, int K2, OpDepth& od, int nmat, const int2* d_src, const
         od.d_matsX = alloc<unsigned char>(ctx, n * xg.OPB);
     }
     if (nmat == 0) return;
-    const OpImages im{od.d_mats, od.d_matsb, od.d_matsD, od.d_matsE, od.d_mats32, od.d_matsb32, od.d_matsT32, od.d_matsbT32,
+    const OpImages im{od.d_mats, od.d_matsD, od.d_matsE, od.d_mats32, od.d_matsT32, od.d_matsbT32,
                       od.d_matsI, od.d_matsbI, od.d_matsS32, od.d_matsbS32, od.d_matsX};
     k_op_images<<<nmat, 128, 0, ctx->stream>>>(d_src, d_blocks, d_beta, K2, im);
     MWB_CUDA(cudaGetLastError());
