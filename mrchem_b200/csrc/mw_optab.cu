@@ -31,7 +31,8 @@ namespace mwb {
 
 namespace {
 
-constexpr int kMaxBand = 511;  // offsets per direction up to 2 * 511 + 1 (the sort keys' 10 bits)
+constexpr int kMaxBand = 4095;   // matrices of a term: offsets -L .. L with L up to this
+constexpr int kMaxOffset = 511;  // listed offsets per direction up to 2 * 511 + 1 (10 bits each in the line order)
 
 struct OpTerm {  // one (operator, term)
     double alpha, beta, cut;
@@ -226,10 +227,10 @@ __device__ __forceinline__ double bound3_dev(double beta, const double* t, const
 }
 
 // rows (term, dx, dy): the offsets dz whose bound reaches the cut (count, then fill at the row's place: key =
-// operator | dx | dy | dz (bits each, offset by lm), bound, term)
+// operator | dx | dy | dz (bits each, offset by lm), bound, term).  reach: the largest listed offset, where it is wanted
 __global__ void k_op_list(const OpTerm* __restrict__ terms, int nterm, long long nrows, const double* __restrict__ t2,
                           const double* __restrict__ x2, int lcap, int root, int lm, int bits, int* count,
-                          const long long* __restrict__ offs, unsigned long long* key, double* bound, int* term) {
+                          const long long* __restrict__ offs, unsigned long long* key, double* bound, int* term, int* reach) {
     const long long row = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (row >= nrows) return;
     int lo = 0, hi = nterm - 1;  // last term with row0 <= row (inactive terms have no rows)
@@ -246,7 +247,7 @@ __global__ void k_op_list(const OpTerm* __restrict__ terms, int nterm, long long
     for (int i = 0; i <= tm.L; ++i) S2 = fmax(S2, t2r[i] + x2r[i]);
     const int ix = abs(dx), iy = abs(dy);
     const double ax = t2r[ix] + x2r[ix], ay = t2r[iy] + x2r[iy];
-    int n = 0;
+    int n = 0, far = 0;
     const long long p0 = offs ? offs[row] : 0;
     if (root || !(tm.beta * sqrt(ax) * S2 < tm.cut || tm.beta * sqrt(ax * ay * S2) < tm.cut)) {
         for (int dz = -tm.L; dz <= tm.L; ++dz) {
@@ -254,6 +255,7 @@ __global__ void k_op_list(const OpTerm* __restrict__ terms, int nterm, long long
             const double t[3] = {t2r[ix], t2r[iy], t2r[iz]}, x[3] = {x2r[ix], x2r[iy], x2r[iz]};
             const double bd = bound3_dev(tm.beta, t, x, root != 0);
             if (bd <= 0.0 || bd < tm.cut) continue;
+            far = max(max(ix, iy), max(far, iz));
             if (offs) {
                 key[p0 + n] = ((((unsigned long long)tm.op << bits | (unsigned)(dx + lm)) << bits | (unsigned)(dy + lm)) << bits) |
                               (unsigned)(dz + lm);
@@ -264,6 +266,7 @@ __global__ void k_op_list(const OpTerm* __restrict__ terms, int nterm, long long
         }
     }
     if (!offs) count[row] = n;
+    if (reach && far > *reinterpret_cast<volatile int*>(reach)) atomicMax(reach, far);
 }
 
 __global__ void k_op_iota(int n, int* idx) {
@@ -318,7 +321,7 @@ __global__ void k_op_delta_keys(int n, const int* __restrict__ idx, const int* _
 }
 // offsets in their final order: record and largest bound
 __global__ void k_op_deltas(int n, const int* __restrict__ order, const int* __restrict__ dfirst, int nrec, int ndelta,
-                            const unsigned long long* __restrict__ key, int bits, int lm, const double* __restrict__ dmax,
+                            const unsigned long long* __restrict__ key, int bits, int lm, int reach, const double* __restrict__ dmax,
                             const OpOut* __restrict__ outs, double* maxb) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -332,7 +335,7 @@ __global__ void k_op_deltas(int n, const int* __restrict__ order, const int* __r
     r.d[2] = (int)(k & mask) - lm;
     r.t0 = r0 - o.rec0;
     r.t1 = r1 - o.rec0;
-    r.lrank = ((r.d[2] + lm) << 10) | (r.d[1] + lm);  // line order: increasing dz, then dy
+    r.lrank = ((r.d[2] + reach) << 10) | (r.d[1] + reach);  // line order: increasing dz, then dy
     r.maxb = dmax[d];
     o.deltas[i - o.del0] = r;
     maxb[i] = r.maxb;
@@ -564,13 +567,14 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
     }
     if (flag) {  // a band wider than the scratch: once more with all of it
         sc.release();
-        if (lcap > kMaxBand) throw Error(-4, "operator band wider than 1024 offsets per direction");
+        if (lcap > kMaxBand) throw Error(-4, "operator band wider than 8192 offsets per direction");
         for (Op* o : ops) op_build_group({o}, depth, 8 * lcap);
         return;
     }
     // bands -> matrices and list rows
     int lm = 0;
     long long nrows = 0;
+    double scan = 0.0;
     std::vector<int> nmat(nop, 0);
     for (OpTerm& t : terms) {
         t.row0 = nrows;
@@ -578,24 +582,30 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
         if (!t.active) continue;
         lm = std::max(lm, t.L);
         nrows += (long long)(2 * t.L + 1) * (2 * t.L + 1);
+        scan += std::pow(2.0 * t.L + 1.0, 3);
         nmat[t.op] += 2 * t.L + 1;
     }
-    if (lm > kMaxBand) throw Error(-4, "operator band wider than 1024 offsets per direction");
+    if (lm > kMaxBand) throw Error(-4, "operator band wider than 8192 offsets per direction");
     upload_bytes(ctx, d_terms, terms.data(), sizeof(OpTerm) * nt);
     // lists
     const int bits = bits_for(2 * lm + 1), obits = bits_for(nop);
     // records per operator, counted before anything is made from them
-    OpPlan plan = op_plan_rows(nop, nrows);
+    OpPlan plan = op_plan_rows(nop, nrows, scan);
     int* d_cnt = nullptr;
     long long* d_offs = nullptr;
+    int reach = lm;  // of the lists: a wide band's, where its scaling blocks have not decayed but its bounds have, is found below
     std::vector<long long> first(nop + 1, 0);
     if (nrows > 0 && plan == OpPlan::together) {
         d_cnt = sc.get<int>(nrows + 1);
         d_offs = sc.get<long long>(nrows + 1);
         MWB_CUDA(cudaMemsetAsync(d_cnt + nrows, 0, sizeof(int), s));
         k_op_list<<<blocks_of(nrows, 128), 128, 0, s>>>(d_terms, nt, nrows, d_t2, d_x2, lcap, root, lm, bits, d_cnt, nullptr,
-                                                        nullptr, nullptr, nullptr);
+                                                        nullptr, nullptr, nullptr, lm > kMaxOffset ? d_flag : nullptr);
         MWB_CUDA(cudaGetLastError());
+        if (lm > kMaxOffset) {
+            readback(ctx, {{&reach, d_flag, sizeof(int)}});  // (zero before: no band reached beyond the scratch)
+            if (reach > kMaxOffset) throw Error(-4, "operator offsets wider than 1024 per direction");
+        }
         exclusive_sum(ctx, d_cnt, d_offs, (int)nrows + 1);
         // the row offsets at the operators' first terms
         std::vector<ReadReq> rq;
@@ -644,7 +654,7 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
             int* d_head = sc.get<int>(nrec + 1);
             int* d_hpos = sc.get<int>(nrec + 1);
             k_op_list<<<blocks_of(nrows, 128), 128, 0, s>>>(d_terms, nt, nrows, d_t2, d_x2, lcap, root, lm, bits, d_cnt, d_offs,
-                                                            d_key, d_bound, d_term);
+                                                            d_key, d_bound, d_term, nullptr);
             k_op_iota<<<rb, 256, 0, s>>>(nrec, d_i0);
             sort_pairs(ctx, true, reinterpret_cast<const unsigned long long*>(d_bound), reinterpret_cast<unsigned long long*>(d_b2),
                        d_i0, d_i1, nrec, 0, 64);
@@ -686,7 +696,7 @@ static void op_build_group(const std::vector<Op*>& ops, int depth, int lcap) {
                 sort_pairs(ctx, false, d_k0, d_k1, d_o1, d_o0, nd, 0, obits);
                 std::swap(d_o0, d_o1);
             }
-            k_op_deltas<<<db, 256, 0, s>>>(nd, d_o1, d_df, nrec, nd, d_key3, bits, lm, d_dmax, d_outs, d_maxb);
+            k_op_deltas<<<db, 256, 0, s>>>(nd, d_o1, d_df, nrec, nd, d_key3, bits, lm, reach, d_dmax, d_outs, d_maxb);
             MWB_CUDA(cudaGetLastError());
             ctx->launches += 9;
             maxb.resize(nd);

@@ -77,3 +77,19 @@ def test_operator_without_terms(gpu_mod):
                 assert t.square_norm() == 0.0
             else:
                 assert_same_tree(t.export(), one.export(), tol=0.0)
+
+
+def test_bands_wider_than_the_lists(gpu_mod):
+    """At order 3 and operator precision 1e-6 the scaling blocks of the widest term reach 1014 offsets at depth 10, its bounds
+    far fewer: the matrices are held, the lists fit.  The self-energy of six Gaussians of unit charge about one point,
+    each finding the next on the grid, against 2 / sqrt(pi) sum (a b / (a + b))^(1/2); the bar is the apply's precision
+    carried through <f|V>, 1e-4 ||f|| ||V||, 18 of 2189."""
+    G = gpu_mod
+    m = G.MultiResolutionAnalysis(-2, (0, 0, 0), (1, 1, 1), 3, 14)
+    alpha = [16.0 * 8.0 ** j for j in range(6)]
+    f, out = G.FunctionTree(m), G.FunctionTree(m)
+    G.project(1e-4, f, G.gauss_params([(a / math.pi) ** 1.5 for a in alpha], alpha, [(2.1, 1.9, 2.05)] * 6))
+    G.apply(1e-4, out, G.PoissonOperator(m, 1e-6), f)
+    assert out.export(False)["depth"].max() >= 10
+    energy = sum(2.0 / math.sqrt(math.pi) * math.sqrt(a * b / (a + b)) for a in alpha for b in alpha)
+    assert abs(G.dot(f, out) - energy) < 1e-4 * math.sqrt(f.square_norm() * out.square_norm())

@@ -13,13 +13,13 @@ def plan(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("plan") / "op_plan")
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-I" + os.path.join(ROOT, "mrchem_b200", "csrc"),
                            os.path.join(ROOT, "tests", "cpp", "op_plan.cpp"), "-o", exe])
-    return lambda nop, rows, records: subprocess.check_output([exe, str(nop), str(rows), str(records)], text=True).strip()
+    return lambda nop, rows, scan, records: subprocess.check_output([exe] + [str(v) for v in (nop, rows, scan, records)], text=True).strip()
 
 
 def sizes(nop, nterm, boxes):
-    """rows and records at the root, where every offset of a term whose band is the world's width is listed"""
+    """rows, scanned offsets and records at the root, where every offset of a term whose band is the world's width is listed"""
     w = 2 * (boxes - 1) + 1
-    return nop, nop * nterm * w ** 2, nop * nterm * w ** 3
+    return nop, nop * nterm * w ** 2, nop * nterm * w ** 3, nop * nterm * w ** 3
 
 
 @pytest.mark.parametrize("nop,nterm,boxes,want", [
@@ -35,7 +35,9 @@ def test_plan_of_wide_roots(plan, nop, nterm, boxes, want):
 
 
 def test_plan_edges(plan):
-    assert plan(8, 1000, 2 ** 24) == "together" and plan(8, 1000, 2 ** 24 + 1) == "singly"
-    assert plan(1, 1000, 2 ** 31 - 1024) == "together" and plan(1, 1000, 2 ** 31 - 1023) == "refuse"
-    assert plan(1, 2 ** 30, 5) == "together" and plan(1, 2 ** 30 + 1, 5) == "refuse"
-    assert plan(2, 2 ** 24 + 1, 5) == "singly"
+    assert plan(8, 1000, 1e9, 2 ** 24) == "together" and plan(8, 1000, 1e9, 2 ** 24 + 1) == "singly"
+    assert plan(1, 1000, 1e9, 2 ** 31 - 1024) == "together" and plan(1, 1000, 1e9, 2 ** 31 - 1023) == "refuse"
+    assert plan(1, 2 ** 30, 1e9, 5) == "together" and plan(1, 2 ** 30 + 1, 1e9, 5) == "refuse"
+    assert plan(2, 2 ** 24 + 1, 1e9, 5) == "singly"
+    assert plan(1, 2 ** 24, 1e11, 5) == "together" and plan(1, 2 ** 24, 1.01e11, 5) == "refuse"
+    assert plan(2, 2 ** 24, 1.01e11, 5) == "singly"
