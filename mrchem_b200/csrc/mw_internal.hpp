@@ -23,12 +23,15 @@ struct Error : std::runtime_error {
     Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
 };
 
+// the runtime keeps a failed call's error for the next check of a launch: it is taken from there with the throw
 #define MWB_CUDA(call)                                                                           \
     do {                                                                                         \
         cudaError_t e_ = (call);                                                                 \
-        if (e_ != cudaSuccess)                                                                   \
+        if (e_ != cudaSuccess) {                                                                 \
+            cudaGetLastError();                                                                  \
             throw ::mwb::Error(-2, std::string(#call) + ": " + cudaGetErrorString(e_) + " (" +    \
                                        __FILE__ + ":" + std::to_string(__LINE__) + ")");          \
+        }                                                                                        \
     } while (0)
 
 constexpr int kKeyBits = 19;          // translation bits per dimension in a node key
