@@ -137,16 +137,14 @@ __device__ __forceinline__ void bx_z(const double* X, int q0, int dq, const doub
     }
 }
 
-// every column tile of this warp, two at a time; f(c', n, v0, v1) takes the outputs (n even, and n + 1) of each lane.
-// INPLACE: f puts them in the columns' place
-template <int K, int RO, bool INPLACE = false, typename F>
+// every column tile of this warp, two at a time; f(c', n, v0, v1) takes the outputs (n even, and n + 1) of each lane
+template <int K, int RO, typename F>
 __device__ __forceinline__ void bx_columns(const double* X, const double* fz, F&& f) {
     using C = BX<K, RO>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int q = warp; q < C::NZT; q += 2 * C::NWARP) {
         double v[2][C::RT][2];
         bx_z<K, RO, 2>(X, q, C::NWARP, fz, v);
-        if constexpr (INPLACE) __syncwarp();  // the columns are read
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll

@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(BX<K, K>::NTHR, 1)
         __syncthreads();
         bx_slices<K, K>(X, f, f + B::FRAG);
         __syncthreads();
-        bx_columns<K, K, true>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {
+        bx_columns<K, K>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {  // in the columns' own place
             double* p = X + c * B::LDP + B::physo(n);
             p[0] = v0;
             if (n + 1 < K * K) X[c * B::LDP + B::physo(n + 1)] = v1;
