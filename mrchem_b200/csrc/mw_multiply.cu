@@ -19,6 +19,7 @@
 // number of levels of generation, 2 blocks read and 1 written: bound by the FP64 pipe.
 #include <algorithm>
 #include <cmath>
+#include <numeric>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -269,7 +270,8 @@ __global__ void __launch_bounds__(BX<K, K>::NTHR, 1)
         __syncthreads();
         bx_slices<K, K>(X, f, f + B::FRAG);
         __syncthreads();
-        bx_columns<K, K>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {  // in the columns' own place
+        bx_columns<K, K>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {
+            // in the columns' own place: every lane's reads have fed the matrix instruction, which the warp executes together
             double* p = X + c * B::LDP + B::physo(n);
             p[0] = v0;
             if (n + 1 < K * K) X[c * B::LDP + B::physo(n + 1)] = v1;
@@ -546,6 +548,9 @@ void refine_passes(double prec, int n, Tree** out, int max_iter, LaunchF&& launc
     }
     for (int iter = 0;; ++iter) {
         std::vector<MulItem> items;
+        size_t nwork = 0;
+        for (int i = 0; i < n; ++i) nwork += work[i].size();
+        items.reserve(nwork);  // (lists of 10^4 to 10^5 nodes: their growth showed in a pass)
         for (int i = 0; i < n; ++i)
             for (int q : work[i]) items.push_back({i, q});
         if (items.empty()) break;
@@ -572,6 +577,7 @@ void refine_passes(double prec, int n, Tree** out, int max_iter, LaunchF&& launc
         }
         if (!full.empty()) {
             std::vector<int2> its;
+            its.reserve(nwork);
             std::vector<SplitTree> st(n, SplitTree{nullptr, nullptr, 0.0});
             for (int i : full) {
                 Tree& o = *out[i];
@@ -613,7 +619,8 @@ void refine_passes(double prec, int n, Tree** out, int max_iter, LaunchF&& launc
             for (size_t g = 0; g < gi.size(); ++g) {
                 const int i = gi[g];
                 any = true;
-                for (int v = before[g]; v < out[i]->n; ++v) work[i].push_back(v);
+                work[i].resize(out[i]->n - before[g]);
+                std::iota(work[i].begin(), work[i].end(), before[g]);
                 keys[i].clear();  // host keys are refreshed when the general path needs them
             }
         }
