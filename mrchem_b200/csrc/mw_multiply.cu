@@ -457,7 +457,9 @@ void build_grid(Tree& out, Tree& inp) {
     if (na > 0) {
         const int n0 = out.n, n = n0 + na;
         // the merged arrays, with room to grow; they and a larger index are all there before the tree takes them
-        const int cap = n > out.cap ? std::max(n, 2 * out.cap) : out.cap;
+        // (of a tree that once was larger at most 1 GiB: the old arrays are still there while these are filled)
+        const int spare = (int)((size_t)(1 << 30) / (sizeof(double) * BS));
+        const int cap = n > out.cap ? std::max(n, 2 * out.cap) : std::min(out.cap, n + spare);
         uint32_t hcap = std::max(out.hcap, 1024u);  // hash index at most half full
         while (hcap < 2u * (uint32_t)n) hcap <<= 1;
         Scratch neu(ctx);

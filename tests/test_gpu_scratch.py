@@ -57,3 +57,31 @@ def test_pass_holds_sorted_triples_only(gpu_mod, order, flags):
     held = ctas * (block + 48) + 16 * trip + 33 * ncand + 1000 * 4 * block
     sort = 32 * trip + 20 * trip + 33 * ncand  # the sort itself: both sides and its scratch
     assert high <= max(held, sort) + (32 << 20), (high, held, sort)
+
+
+def test_union_grid_keeps_little_spare_room(gpu_mod):
+    """A grid made in a tree that once held many more nodes: the merged arrays keep room to grow, but no more than 1 GiB of
+    it beside the tree's own (the old ones are still there while they are filled)."""
+    import numpy as np
+
+    G = gpu_mod
+    ctx = G.Context.default()
+    m = G.MultiResolutionAnalysis(*WORLD, 9, 14)
+    rng = np.random.default_rng(1)
+    a = np.exp(rng.uniform(np.log(0.5), np.log(3e3), 120))
+    big, small, pool = G.FunctionTree(m), G.FunctionTree(m), Pool()
+    G.project(1e-8, big, G.gauss_params(list((a / np.pi) ** 0.75), list(a), [tuple(x) for x in rng.uniform(-9, 9, (120, 3))]))
+    G.project(1e-5, small, two_gaussians(G))
+    block, n = 8 * 20 ** 3, small.nnodes()
+    assert big.nnodes() * block > 2 << 30
+    G.clear(big)
+    ctx.synchronize()
+    base = pool.get(USED_CURRENT)
+    pool.reset_high()
+    G.build_grid(big, small)
+    ctx.synchronize()
+    assert big.nnodes() == n
+    assert pool.get(USED_HIGH) - base <= n * block + (1 << 30) + (32 << 20)
+    assert pool.get(USED_CURRENT) < base
+    G.multiply(1e-5, big, 1.0, small, small)  # and it grows again
+    assert big.square_norm() > 0.0
