@@ -846,9 +846,7 @@ static void mra_free(mwb::Mra* m) {
     mwb::Ctx* c = m->ctx;
     cudaSetDevice(c->device);
     mwb::dfree(c, m->d_F);
-    mwb::dfree(c, m->d_FT);
     mwb::dfree(c, m->d_frF);
-    mwb::dfree(c, m->d_MV);
     mwb::dfree(c, m->d_cc);
     mwb::dfree(c, m->d_px);
     mwb::dfree(c, m->d_pw);
@@ -1149,12 +1147,8 @@ int mw_mra_create(mw_ctx ctx, int min_scale, const int* corner, const int* boxes
                     MV[(c * k + q) * K2 + b] = v;
                 }
         cudaStream_t s = ctx->stream;
-        m->d_MV = (double*)dalloc(ctx, sizeof(double) * K2 * K2);
-        MWB_CUDA(cudaMemcpyAsync(m->d_MV, MV.data(), sizeof(double) * K2 * K2, cudaMemcpyHostToDevice, s));
         m->d_F = (double*)dalloc(ctx, sizeof(double) * K2 * K2);
-        m->d_FT = (double*)dalloc(ctx, sizeof(double) * K2 * K2);
         MWB_CUDA(cudaMemcpyAsync(m->d_F, m->F.data(), sizeof(double) * K2 * K2, cudaMemcpyHostToDevice, s));
-        MWB_CUDA(cudaMemcpyAsync(m->d_FT, FT.data(), sizeof(double) * K2 * K2, cudaMemcpyHostToDevice, s));
         world_fragments(*m, PF, MV, FT);
         MWB_CUDA(cudaStreamSynchronize(s));
         ctx->refs++;

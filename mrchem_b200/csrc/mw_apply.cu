@@ -210,45 +210,40 @@ __global__ void k_bresolve_gen(int* csrc, int ncand, const uint64_t* __restrict_
 // 2. generated input nodes: reconstruct the leaf ancestor, take the child on the path, descend
 //    with zero wavelets (s_c = H_c^T s per dimension)
 // ---------------------------------------------------------------------------------------------
-// One block per node: the three directions' matrices from the leaf's block straight to the node (bx_path_operators), then
-// one separable transform on the FP64 matrix instruction, whatever the number of levels.
+// One block per node, level by level from the leaf's block on the FP64 matrix instruction (bx_descend).
 template <int K>
 struct GenCfg {
     using B = BX<K, K>;
-    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 3 * B::FRAG);
+    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 4 * B::FRAG);
     static constexpr int MINB = K <= 6 ? 4 : K <= 10 ? 2 : 1;
 };
 template <int K>
 __global__ void __launch_bounds__(BX<K, K>::NTHR, GenCfg<K>::MINB)
     k_bgenerate(const uint64_t* __restrict__ ukey, const int* __restrict__ uleaf, const BTree* __restrict__ trees,
-                const double* __restrict__ FT, double* gblk, double* gnorm2) {
+                const double* __restrict__ frH, double* gblk, double* gnorm2) {
     using B = BX<K, K>;
     extern __shared__ __align__(16) double sm[];
     __shared__ double red[64];
     double* X = sm;
-    double* f = X + B::VOL;
+    double* h = X + B::VOL;
     const int g = blockIdx.x;
     const uint64_t gkey = ukey[g];
     const BTree& T = trees[(int)(gkey >> 57)];
     const int leaf = uleaf[g];
     long long t[3];
     key_trans(gkey & ((1ull << 57) - 1), t);
-    bx_path_operators<K, false>(FT, nullptr, t, T.depth - key_depth(T.inkey[leaf]), X, f);
-    bx_load<K, K>(X, T.in.coef + (size_t)leaf * Geo<K>::BS);
+    bx_operator(h, frH, 4 * B::FRAG, B::NTHR);
+    bx_load<K, B::NWARP>(X, T.in.coef + (size_t)leaf * Geo<K>::BS);
     cp_async_wait_all();
     __syncthreads();
-    bx_slices<K, K>(X, f, f + B::FRAG);
-    __syncthreads();
+    bx_descend<K, B::NWARP>(X, h, t, T.depth - key_depth(T.inkey[leaf]));
     double n2 = 0.0, dmy = 0.0;
     double* out = gblk + (size_t)g * K * K * K;
-    bx_columns<K, K>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {
-        out[n + K * K * c] = v0;
-        n2 += v0 * v0;
-        if (n + 1 < K * K) {
-            out[n + 1 + K * K * c] = v1;
-            n2 += v1 * v1;
-        }
-    });
+    for (int e = threadIdx.x; e < K * K * K; e += B::NTHR) {
+        const double v = X[e % (K * K) + B::LDP * (e / (K * K))];
+        out[e] = v;
+        n2 += v * v;
+    }
     block_sum2(n2, dmy, red);
     if (threadIdx.x == 0) gnorm2[g] = n2;
 }
@@ -1494,7 +1489,7 @@ void run_batch_pass(BatchPass& bp, cudaStream_t s) {
 #define L_GEN(KK)                                                                                                        \
     {                                                                                                                    \
         MWB_CUDA(cudaFuncSetAttribute(k_bgenerate<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GenCfg<KK>::SMEM)); \
-        k_bgenerate<KK><<<nu, BX<KK, KK>::NTHR, GenCfg<KK>::SMEM, s>>>(d_ukey, d_uleaf, d_trees, m.d_FT, d_gblk, d_gnorm2); \
+        k_bgenerate<KK><<<nu, BX<KK, KK>::NTHR, GenCfg<KK>::SMEM, s>>>(d_ukey, d_uleaf, d_trees, m.d_frH, d_gblk, d_gnorm2); \
     }
         MWB_DISPATCH_K(K, L_GEN)
 #undef L_GEN

@@ -61,11 +61,12 @@ __host__ __device__ inline double bx_frag_b(int e, F&& entry) {
     return o < RO && b < C::K2 ? entry(o, b) : 0.0;
 }
 
-// x and y products of slice c (one warp, in place): X[c][b][a] -> X[c][b'][a'], rows LDA -> LDO
-template <int K, int RO>
+// x and y products of slice c (one warp, in place): X[c][b][a] -> X[c][b'][a'], rows LDI -> LDO.  NI: the input's extent, 2k,
+// or k for a scaling block alone (its wavelets zero)
+template <int K, int RO, int NI = 2 * K, int LDI = BX<K, RO>::LDA>
 __device__ __forceinline__ void bx_slice(double* X, int c, const double* fx, const double* fy) {
     using C = BX<K, RO>;
-    constexpr int K2 = C::K2, RT = C::RT, CT = C::CT, S = C::S;
+    constexpr int RT = C::RT, S = C::S, SI = (NI + 3) / 4, CT = (NI + 7) / 8, SY = NI == C::K2 ? S : 2 * CT;
     const int lane = threadIdx.x & 31, fi = lane & 3, fn = lane >> 2;
     double* P = X + c * C::LDP;
     double D[RT][CT][2];
@@ -74,7 +75,7 @@ __device__ __forceinline__ void bx_slice(double* X, int c, const double* fx, con
 #pragma unroll
         for (int t = 0; t < CT; ++t) D[r][t][0] = D[r][t][1] = 0.0;
 #pragma unroll
-    for (int s = 0; s < S; ++s) {
+    for (int s = 0; s < SI; ++s) {
         double a[RT];
 #pragma unroll
         for (int r = 0; r < RT; ++r) a[r] = fx[(s * RT + r) * 32 + lane];
@@ -82,8 +83,8 @@ __device__ __forceinline__ void bx_slice(double* X, int c, const double* fx, con
 #pragma unroll
         for (int t = 0; t < CT; ++t) {
             const int b = bx_col<K, RO>(t, fn);
-            const bool in = (4 * s + 3 < K2 || ai < K2) && (8 * t + 7 < K2 || b < K2);
-            const double v = in ? P[ai + C::LDA * b] : 0.0;
+            const bool in = (4 * s + 3 < NI || ai < NI) && (8 * t + 7 < NI || b < NI);
+            const double v = in ? P[ai + LDI * b] : 0.0;
 #pragma unroll
             for (int r = 0; r < RT; ++r) dmma(D[r][t], a[r], v);
         }
@@ -95,7 +96,7 @@ __device__ __forceinline__ void bx_slice(double* X, int c, const double* fx, con
 #pragma unroll
         for (int r = 0; r < RT; ++r) Y[r][0] = Y[r][1] = 0.0;
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
+        for (int s = 0; s < SY; ++s) {
             const double m = fy[(j * S + s) * 32 + lane];
 #pragma unroll
             for (int r = 0; r < RT; ++r) dmma(Y[r], D[r][s / 2][s % 2], m);
@@ -112,17 +113,17 @@ __device__ __forceinline__ void bx_slice(double* X, int c, const double* fx, con
 
 // z product of column tile q (one warp): v[r][h] = out at c' = 8 r + lane / 4, column 8 q + 2 (lane mod 4) + h of
 // (a', b')
-template <int K, int RO, int NQ>
+template <int K, int RO, int NQ, int NI = 2 * K>
 __device__ __forceinline__ void bx_z(const double* X, int q0, int dq, const double* fz, double (&v)[NQ][BX<K, RO>::RT][2]) {
     using C = BX<K, RO>;
-    constexpr int K2 = C::K2, RT = C::RT, S = C::S;
+    constexpr int RT = C::RT, SI = (NI + 3) / 4;
     const int lane = threadIdx.x & 31, fi = lane & 3, fn = lane >> 2;
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
 #pragma unroll
         for (int r = 0; r < RT; ++r) v[q][r][0] = v[q][r][1] = 0.0;
 #pragma unroll
-    for (int s = 0; s < S; ++s) {
+    for (int s = 0; s < SI; ++s) {
         double a[RT];
 #pragma unroll
         for (int r = 0; r < RT; ++r) a[r] = fz[(s * RT + r) * 32 + lane];
@@ -130,7 +131,7 @@ __device__ __forceinline__ void bx_z(const double* X, int q0, int dq, const doub
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {
             const int tile = q0 + q * dq;
-            const double b = (4 * s + 3 < K2 || c < K2) && tile < C::NZT ? X[c * C::LDP + C::physo(8 * tile) + fn] : 0.0;
+            const double b = (4 * s + 3 < NI || c < NI) && tile < C::NZT ? X[c * C::LDP + C::physo(8 * tile) + fn] : 0.0;
 #pragma unroll
             for (int r = 0; r < RT; ++r) dmma(v[q][r], a[r], b);
         }
@@ -138,30 +139,31 @@ __device__ __forceinline__ void bx_z(const double* X, int q0, int dq, const doub
 }
 
 // every column tile of this warp, two at a time; f(c', n, v0, v1) takes the outputs (n even, and n + 1) of each lane
-template <int K, int RO, typename F>
+// (NW: the kernel's warps)
+template <int K, int RO, int NI = 2 * K, int NW = BX<K, RO>::NWARP, typename F>
 __device__ __forceinline__ void bx_columns(const double* X, const double* fz, F&& f) {
     using C = BX<K, RO>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int q = warp; q < C::NZT; q += 2 * C::NWARP) {
+    for (int q = warp; q < C::NZT; q += 2 * NW) {
         double v[2][C::RT][2];
-        bx_z<K, RO, 2>(X, q, C::NWARP, fz, v);
+        bx_z<K, RO, 2, NI>(X, q, NW, fz, v);
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int r = 0; r < C::RT; ++r) {
-                const int cz = 8 * r + (lane >> 2), n = 8 * (q + h * C::NWARP) + 2 * (lane & 3);
+                const int cz = 8 * r + (lane >> 2), n = 8 * (q + h * NW) + 2 * (lane & 3);
                 if (cz < RO && n < RO * RO) f(cz, n, v[h][r][0], v[h][r][1]);
             }
     }
 }
 
-// a block from global memory (x fastest) into the shared layout, asynchronously, by the threads of a kernel whose products
-// are those of BX<K, RO> (which differ in number: at k = 9 to 11 eight warps against k)
-template <int K, int RO>
+// a block from global memory (x fastest) into the shared layout, asynchronously, by the NW warps of the kernel (which the kinds
+// of products differ in: at k = 9 to 11 eight against k)
+template <int K, int NW>
 __device__ __forceinline__ void bx_load(double* X, const double* __restrict__ blk) {
-    using C = BX<K, RO>;
+    using C = BX<K, 2 * K>;
     constexpr int H = K, N = C::K2 * C::K2 * H;  // 16-byte pairs
-    for (int e = threadIdx.x; e < N; e += C::NTHR) {
+    for (int e = threadIdx.x; e < N; e += 32 * NW) {
         const int r = e / H, i = e - r * H, b = r % C::K2, c = r / C::K2;
         cp_async16(X + 2 * i + C::LDA * b + C::LDP * c, blk + 2 * (size_t)e);
     }
@@ -189,57 +191,40 @@ __device__ __forceinline__ void bx_lookup(const uint64_t* hk, const int* hv, uin
     idx = m ? __shfl_sync(0xffffffffu, i, depth) : -1;
 }
 
-// The three directions' operators from an ancestor's block to what lies L >= 1 levels below it along the
-// translations t (of the descendant): first the rows of the reconstruction that belong to the child on the path
-// (k x 2k), then zero-wavelet descents (k x k blocks), then, with POST, the first k columns of a 2k x 2k matrix
-// (point values, for instance).  The products replace L transforms of the block by three small matrix products.
-// Fragments (A, B, A order) land in f; w is scratch of 6 k 2k + 3 (2k)^2 doubles; the whole block takes part
-template <int K, bool POST>
-__device__ void bx_path_operators(const double* __restrict__ FT, const double* __restrict__ P, const long long (&t)[3], int L,
-                                  double* w, double* f) {
-    constexpr int K2 = 2 * K, N = K * K2, RO = POST ? K2 : K;
-    using C = BX<K, RO>;
-    double *m0 = w, *m1 = w + 3 * N, *v = w + 6 * N;
-    auto bit = [&](int d, int lev) { return (int)((t[d] >> lev) & 1); };
-    for (int e = threadIdx.x; e < 3 * N; e += blockDim.x) m0[e] = FT[bit(e / N, L - 1) * N + e % N];
-    __syncthreads();
-    for (int lev = L - 2; lev >= 0; --lev) {
-        for (int e = threadIdx.x; e < 3 * N; e += blockDim.x) {
-            const int d = e / N, o = (e % N) / K2, i = e % K2;
-            const double* row = FT + (bit(d, lev) * K + o) * K2;
-            double s = 0.0;
-#pragma unroll
-            for (int q = 0; q < K; ++q) s = fma(row[q], m0[d * N + q * K2 + i], s);
-            m1[e] = s;
-        }
-        __syncthreads();
-        double* x = m0;
-        m0 = m1;
-        m1 = x;
-    }
-    if constexpr (POST) {
-        for (int e = threadIdx.x; e < 3 * K2 * K2; e += blockDim.x) {
-            const int d = e / (K2 * K2), o = (e / K2) % K2, i = e % K2;
-            double s = 0.0;
-#pragma unroll
-            for (int q = 0; q < K; ++q) s = fma(P[o * K2 + q], m0[d * N + q * K2 + i], s);
-            v[e] = s;
-        }
-        __syncthreads();
-        m0 = v;
-    }
-    for (int e = threadIdx.x; e < 3 * C::FRAG; e += blockDim.x) {
-        const int d = e / C::FRAG, q = e - d * C::FRAG;
-        auto entry = [&](int o, int i) { return m0[(d * RO + o) * K2 + i]; };
-        f[e] = d == 1 ? bx_frag_b<K, RO>(q, entry) : bx_frag_a<K, RO>(q, entry);
-    }
-    __syncthreads();
+// x and y products of every slice, distributed over the kernel's NW warps; fx, fy: operators
+template <int K, int RO, int NI = 2 * K, int LDI = BX<K, RO>::LDA, int NW = BX<K, RO>::NWARP>
+__device__ __forceinline__ void bx_slices(double* X, const double* fx, const double* fy) {
+    for (int c = threadIdx.x >> 5; c < NI; c += NW) bx_slice<K, RO, NI, LDI>(X, c, fx, fy);
 }
 
-// x and y products of every slice, distributed over the warps; fx, fy: operators
-template <int K, int RO>
-__device__ __forceinline__ void bx_slices(double* X, const double* fx, const double* fy) {
-    for (int c = threadIdx.x >> 5; c < 2 * K; c += BX<K, RO>::NWARP) bx_slice<K, RO>(X, c, fx, fy);
+// From an ancestor's block in X to the scaling block of the node L >= 1 levels below it along the translations t (of the
+// descendant), in place with rows of k (element (a, b, c) at a + k b + LDP c): first the reconstruction's rows of the child on
+// the path (k x 2k), then zero-wavelet descents (k x k).  h: their images [child bit][A, B order], in shared memory.
+// Level by level: every level's rounding is relative to that level's block.  One product of the levels' matrices on the
+// ancestor's block would do with fewer steps, but leaves in each descendant rounding of the size of the ancestor's largest
+// values; where the function falls off inside the ancestor, a product of two such factors was noise, and refinement
+// followed it down (404 nodes and growing fourfold per level against 236).
+// The caller has X and h complete for every warp (a barrier), and so has it the result
+template <int K, int NW>
+__device__ __forceinline__ void bx_descend(double* X, const double* h, const long long (&t)[3], int L) {
+    using C = BX<K, K>;
+    auto img = [&](int d, int lev, int form) { return h + (2 * (int)((t[d] >> lev) & 1) + form) * C::FRAG; };
+    auto put = [&](int c, int n, double v0, double v1) {
+        // in the columns' own place: every lane's reads have fed the matrix instruction, which the warp executes together
+        double* p = X + c * C::LDP + C::physo(n);
+        p[0] = v0;
+        if (n + 1 < K * K) X[c * C::LDP + C::physo(n + 1)] = v1;
+    };
+    bx_slices<K, K, 2 * K, C::LDA, NW>(X, img(0, L - 1, 0), img(1, L - 1, 1));
+    __syncthreads();
+    bx_columns<K, K, 2 * K, NW>(X, img(2, L - 1, 0), put);
+    __syncthreads();
+    for (int lev = L - 2; lev >= 0; --lev) {
+        bx_slices<K, K, K, C::LDO, NW>(X, img(0, lev, 0), img(1, lev, 1));
+        __syncthreads();
+        bx_columns<K, K, K, NW>(X, img(2, lev, 0), put);
+        __syncthreads();
+    }
 }
 
 }  // namespace mwb

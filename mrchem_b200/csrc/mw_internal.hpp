@@ -84,10 +84,10 @@ struct Mra {
     std::vector<double> F;  // (2k)^2 two-scale filter
     std::vector<double> W;  // k x k projection quadrature matrix
     double* d_F = nullptr;   // two-scale filter
-    double* d_FT = nullptr;  // F^T
     // F, F^T, PF and MV as fragments of the block transform (mw_block.cuh), A then B order, each 2 x fr_n doubles
     double *d_frF = nullptr, *d_frFT = nullptr, *d_frPF = nullptr, *d_frMV = nullptr;
     int fr_n = 0;
+    double* d_frH = nullptr;  // the rows of F^T of either child, k x 2k (bx_descend): [child bit][A, B order]
     // operator construction (GaussianOperatorBuilder): cross-correlation coefficients [c+ | c-][p][i k + j], and
     // the Gauss-Legendre rule of the moments
     std::unique_ptr<GaussianOperatorBuilder> builder;
@@ -95,7 +95,6 @@ struct Mra {
     double* d_px = nullptr;
     double* d_pw = nullptr;
     std::mutex op_mtx;  // the tables above and those of the world's operators: held from the look for one to its insertion
-    double* d_MV = nullptr;  // evaluation matrix blkdiag(E, E) * F^T (pointwise product)
     // trees and operators that point here; a destroyed world is freed with the last of them
     int refs = 0;
     bool closed = false;

@@ -196,7 +196,7 @@ __device__ __forceinline__ void transform_node(int mode, int node, const TView& 
             else X[at(a, b, c)] = *src;
         }
     } else {
-        bx_load<K, K2>(X, t.coef + (size_t)node * BS);
+        bx_load<K, B::NWARP>(X, t.coef + (size_t)node * BS);
     }
     cp_async_wait_all();
     __syncthreads();
@@ -575,13 +575,23 @@ void world_fragments(Mra& m, const std::vector<double>& PF, const std::vector<do
                 f[(2 * q + 1) * N + e] = bx_frag_b<KK, 2 * KK>(e, entry);                    \
             }                                                                                \
         }                                                                                    \
+        constexpr int NH = BX<KK, KK>::FRAG;                                                 \
+        f.resize(8 * N + 4 * NH);                                                            \
+        for (int bit = 0; bit < 2; ++bit) {                                                  \
+            auto entry = [&](int o, int i) { return FT[(size_t)(bit * KK + o) * W + i]; };   \
+            for (int e = 0; e < NH; ++e) {                                                   \
+                f[8 * N + 2 * bit * NH + e] = bx_frag_a<KK, KK>(e, entry);                   \
+                f[8 * N + (2 * bit + 1) * NH + e] = bx_frag_b<KK, KK>(e, entry);             \
+            }                                                                                \
+        }                                                                                    \
     }
     MWB_DISPATCH_K(m.k, L_FR)
 #undef L_FR
-    m.d_frF = (double*)dalloc(m.ctx, sizeof(double) * f.size());  // one allocation for the four
+    m.d_frF = (double*)dalloc(m.ctx, sizeof(double) * f.size());  // one allocation for all
     m.d_frFT = m.d_frF + 2 * m.fr_n;
     m.d_frPF = m.d_frF + 4 * m.fr_n;
     m.d_frMV = m.d_frF + 6 * m.fr_n;
+    m.d_frH = m.d_frF + 8 * m.fr_n;
     upload_bytes(m.ctx, m.d_frF, f.data(), sizeof(double) * f.size());
 }
 

@@ -59,7 +59,7 @@ struct MulItem {
 template <int K>
 struct MulCfg {
     using B = BX<K, 2 * K>;
-    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 5 * B::FRAG);
+    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 4 * B::FRAG + 4 * BX<K, K>::FRAG);
     static constexpr int MINB = K <= 6 ? 4 : K <= 10 ? 2 : 1;
     // the first factor's point values wait in tensor memory: 4 RT doubles per lane and couple of column tiles
     static constexpr int NIT = (B::NZT + 2 * B::NWARP - 1) / (2 * B::NWARP), WORDS = 8 * B::RT;
@@ -68,15 +68,15 @@ struct MulCfg {
     static_assert(TNEED <= 256 && MINB * TCOLS <= 512, "tensor memory");
 };
 
-// One output node per block.  Per factor: its block (own, or the deepest ancestor's with the path's operators) to the
-// point values in one separable transform; the product goes back through PF.  FP64-bound: 9 mode products per node on
+// One output node per block.  Per factor: its block, own or generated below the deepest ancestor (bx_descend: a scaling block
+// alone), to the point values in a separable transform; the product goes back through PF.  FP64-bound: 9 mode products per node on
 // the matrix instruction (16 us per node and SM at k = 10), two blocks per SM so that one's loads and barriers hide behind
 // the other's products.  28 pairs at k = 10: 15.5 ms with a thread per pencil and a reconstruction per level of a
 // missing node.
 template <int K>
 __global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, MulCfg<K>::MINB)
-    k_mul(const MulItem* __restrict__ items, const MulTree* __restrict__ trees, const double* __restrict__ MVg,
-          const double* __restrict__ frMV, const double* __restrict__ frPF, const double* __restrict__ FTg, int n0) {
+    k_mul(const MulItem* __restrict__ items, const MulTree* __restrict__ trees, const double* __restrict__ frMV,
+          const double* __restrict__ frPF, const double* __restrict__ frH, int n0) {
     using B = BX<K, 2 * K>;
     using C = MulCfg<K>;
     constexpr int K2 = 2 * K, BS = Geo<K>::BS, RT = B::RT;
@@ -85,14 +85,16 @@ __global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, MulCfg<K>::MINB)
     __shared__ int found[2][2];
     __shared__ uint32_t tmem_slot;
     double* X = msm;
-    double* fq = X + B::VOL;         // the factor's operators (A, B, A order)
-    double* fp = fq + 3 * B::FRAG;   // PF (A, B order)
+    double* fq = X + B::VOL;        // MV (A, B order)
+    double* fp = fq + 2 * B::FRAG;  // PF (A, B order)
+    double* fh = fp + 2 * B::FRAG;  // the half filters' images, for a generated factor
     const MulItem it = items[blockIdx.x];
     const MulTree& T = trees[it.tree];
     const uint64_t key = T.okey[it.node];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, depth = key_depth(key);
     long long tr[3];
     key_trans(key, tr);
+    bx_operator(fq, frMV, 2 * B::FRAG, B::NTHR);
     bx_operator(fp, frPF, 2 * B::FRAG, B::NTHR);
     if (warp < 2) {
         int idx, da;
@@ -116,27 +118,28 @@ __global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, MulCfg<K>::MINB)
     for (int q = sq ? 1 : 0; q < 2; ++q) {
         const int idx = found[q][0], da = found[q][1];
         const double* coef = q ? T.bcoef : T.acoef;
+        const bool gen = idx >= 0 && da < depth;
         if (idx >= 0) {
-            if (da == depth) {
-                bx_operator(fq, frMV, 2 * B::FRAG, B::NTHR);
-                bx_operator(fq + 2 * B::FRAG, frMV, B::FRAG, B::NTHR);
-            } else {
-                bx_path_operators<K, true>(FTg, MVg, tr, depth - da, X, fq);
-            }
-            bx_load<K, K2>(X, coef + (size_t)idx * BS);
+            if (gen) bx_operator(fh, frH, 4 * BX<K, K>::FRAG, B::NTHR);
+            bx_load<K, B::NWARP>(X, coef + (size_t)idx * BS);
         } else {  // outside the factor's roots (cannot happen on one world): zero
             for (int e = tid; e < B::VOL; e += B::NTHR) X[e] = 0.0;
-            for (int e = tid; e < 3 * B::FRAG; e += B::NTHR) fq[e] = 0.0;
         }
         cp_async_wait_all();
         __syncthreads();
-        bx_slices<K, K2>(X, fq, fq + B::FRAG);
+        if (gen) {
+            bx_descend<K, B::NWARP>(X, fh, tr, depth - da);
+            bx_slices<K, K2, K, BX<K, K>::LDO>(X, fq, fq + B::FRAG);
+        } else {
+            bx_slices<K, K2>(X, fq, fq + B::FRAG);
+        }
         __syncthreads();
 #pragma unroll 1
         for (int i = 0; i < C::NIT; ++i) {
             const int t0 = warp + 2 * B::NWARP * i;
             double v[2][RT][2];
-            bx_z<K, K2, 2>(X, t0, B::NWARP, fq + 2 * B::FRAG, v);
+            if (gen) bx_z<K, K2, 2, K>(X, t0, B::NWARP, fq, v);
+            else bx_z<K, K2, 2>(X, t0, B::NWARP, fq, v);
             uint32_t w[C::WORDS];
             if (q == 0) {
 #pragma unroll
@@ -210,17 +213,17 @@ constexpr int kAddMaxTerms = 256;
 // Block of sum_i c_i f_i at one output node: compressed blocks are linear in the function, so the
 // inputs' blocks (own, or generated below the deepest ancestor) are combined as they are.  A lane keeps its
 // elements' sums in registers (element pairs in the order of the z product's outputs) and adds an own block
-// straight from global memory; a generated one comes from one separable transform.  HBM-bound when the inputs have the
+// straight from global memory; a generated one comes from bx_descend.  HBM-bound when the inputs have the
 // nodes.
 template <int K>
 struct AddCfg {
     using B = BX<K, K>;
-    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 3 * B::FRAG);
+    static constexpr size_t SMEM = sizeof(double) * (B::VOL + 4 * B::FRAG);
     static constexpr int PAIRS = 4 * K * K * K, PER = (PAIRS + B::NTHR - 1) / B::NTHR;  // element pairs per thread
 };
 template <int K>
 __global__ void __launch_bounds__(BX<K, K>::NTHR, 1)
-    k_add(const MulItem* __restrict__ items, AddOut out, const AddIn* __restrict__ in, int nin, const double* __restrict__ FTg) {
+    k_add(const MulItem* __restrict__ items, AddOut out, const AddIn* __restrict__ in, int nin, const double* __restrict__ frH) {
     using B = BX<K, K>;
     using C = AddCfg<K>;
     constexpr int K2 = 2 * K, BS = Geo<K>::BS;
@@ -228,7 +231,8 @@ __global__ void __launch_bounds__(BX<K, K>::NTHR, 1)
     __shared__ double red[64];
     __shared__ int found[kAddMaxTerms][2];
     double* X = asm_;
-    double* f = X + B::VOL;
+    double* h = X + B::VOL;
+    bool filters = false;  // h is loaded
     const int node = items[blockIdx.x].node, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t key = out.key[node];
     const int depth = key_depth(key);
@@ -264,19 +268,12 @@ __global__ void __launch_bounds__(BX<K, K>::NTHR, 1)
             continue;
         }
         __syncthreads();  // X is free
-        bx_path_operators<K, false>(FTg, nullptr, tr, depth - da, X, f);
-        bx_load<K, K>(X, blk);
+        if (!filters) bx_operator(h, frH, 4 * B::FRAG, B::NTHR);
+        filters = true;
+        bx_load<K, B::NWARP>(X, blk);
         cp_async_wait_all();
         __syncthreads();
-        bx_slices<K, K>(X, f, f + B::FRAG);
-        __syncthreads();
-        bx_columns<K, K>(X, f + 2 * B::FRAG, [&](int c, int n, double v0, double v1) {
-            // in the columns' own place: every lane's reads have fed the matrix instruction, which the warp executes together
-            double* p = X + c * B::LDP + B::physo(n);
-            p[0] = v0;
-            if (n + 1 < K * K) X[c * B::LDP + B::physo(n + 1)] = v1;
-        });
-        __syncthreads();
+        bx_descend<K, B::NWARP>(X, h, tr, depth - da);
 #pragma unroll
         for (int i = 0; i < C::PER; ++i) {
             const int e = tid + i * B::NTHR, a = 2 * (e % K), b = (e / K) % K2, c = e / (K * K2);
@@ -683,8 +680,8 @@ void multiply_batched(double prec, int n, Tree** out, const double* c, Tree** a,
     {                                                                                                             \
         const size_t smem = MulCfg<KK>::SMEM;                                                                     \
         MWB_CUDA(cudaFuncSetAttribute(k_mul<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));        \
-        k_mul<KK><<<(unsigned)items.size(), BX<KK, 2 * KK>::NTHR, smem, s>>>(d_items, d_trees, m->d_MV, m->d_frMV,  \
-                                                                             m->d_frPF, m->d_FT, m->n0);          \
+        k_mul<KK><<<(unsigned)items.size(), BX<KK, 2 * KK>::NTHR, smem, s>>>(d_items, d_trees, m->d_frMV, m->d_frPF, \
+                                                                             m->d_frH, m->n0);                    \
     }
         MWB_MUL_DISPATCH_K(K, L_MUL)
 #undef L_MUL
@@ -718,7 +715,7 @@ void add_trees(double prec, Tree* out, int n, const double* c, Tree** f, int max
     {                                                                                                               \
         const size_t smem = AddCfg<KK>::SMEM;                                                                       \
         MWB_CUDA(cudaFuncSetAttribute(k_add<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
-        k_add<KK><<<(unsigned)items.size(), BX<KK, KK>::NTHR, smem, s>>>(d_items, ao, d_in, n, m->d_FT);           \
+        k_add<KK><<<(unsigned)items.size(), BX<KK, KK>::NTHR, smem, s>>>(d_items, ao, d_in, n, m->d_frH);           \
     }
         MWB_MUL_DISPATCH_K(K, L_ADD)
 #undef L_ADD
