@@ -1,6 +1,7 @@
 // mw_block.cuh -- separable transform of one (2k)^3 FP64 node block on the FP64 matrix instruction, in place in
 // shared memory:  out = (Mz (x) My (x) Mx) in  with RO x 2k matrices (RO = 2k: projection, compression,
-// reconstruction, point values; RO = k: the scaling part of a node generated below its ancestor).
+// reconstruction, point values; RO = k: one level of the descent to a node generated below its ancestor).  The input's
+// wavelet half may be absent (NI = k).
 //
 // Bound by the FP64 pipe.  The pencil form (a thread per pencil, one operator element read from shared memory per
 // FMA) ran at the shared-memory rate, a quarter of it.  Here a warp takes whole z slices: the x product's C
@@ -34,7 +35,7 @@ struct BX {
     static constexpr int FRAG = S * RT * 32;  // one operator
     // A warp belongs to one SM sub-partition: with k warps of two slices each, k = 9, 10 loads two of the four half as much
     // again as the others, eight warps with slices dealt in turn load them evenly (28 pair products: k = 9 8.80 -> 8.07 ms,
-    // k = 10 8.18 -> 7.92, k = 11 10.95 -> 10.77; k = 5, 6, 7 do not gain).  The sums' kernel (RO = k) holds a block in
+    // k = 10 8.08 -> 7.82, k = 11 10.95 -> 10.77; k = 5, 6, 7 do not gain).  The sums' kernel (RO = k) holds a block in
     // registers and needs the threads (k = 11: 4 % slower with eight warps).
     static constexpr int NWARP = RO == K2 && K >= 9 && K <= 11 ? 8 : K, NTHR = 32 * NWARP;
 };

@@ -11,7 +11,7 @@
 // register-tiled scalar GEMM reads 10 shared words per 25 FMAs and ran at the shared-memory rate.  Contraction
 // time of whole applies, scalar kernel -> this one: 16 Helmholtz orbitals at k = 10 46.2 -> 25.4 ms (the
 // instructions alone, padded rows included: 17.8), 20-atom Poisson at k = 12 302 -> 41.2 ms (37.3), three-charge
-// Poisson at k = 8 5.2 -> 2.2 ms and at k = 6 1.42 -> 0.63 ms.
+// Poisson at k = 8, prec 1e-5 5.1 -> 2.1 ms, at k = 6 3.11 -> 1.19 ms (prec 1e-5) and 1.44 -> 0.58 (prec 1e-3).
 //
 // Work split (k = 6 and k > 8 share the last pairs out as extra units, see DCfg).  Warp p owns the z-index pair
 // (c = p, p + k): one slice of the scaling half and one of the wavelet half, so that generated (scaling-only) inputs and the s->s correction load every warp alike.
@@ -51,7 +51,7 @@ struct DCfg {
     // one pair per warp; at k = 6 and from k = 9 up fewer: eight warps (two per SM sub-partition, 255 registers each) take a pair
     // each and share the last K - 8 pairs by slices: an extra unit = one slice c, at most one per warp.  (One warp
     // per pair puts three warps on one or two sub-partitions and two on the others at k = 9, 10.)  k = 6 likewise
-    // with four warps of a pair and an extra unit each: 1.33 -> 1.23 ms in the three-charge Poisson; at k = 5 the two extra
+    // with four warps of a pair and an extra unit each: 1.33 -> 1.23 ms in a three-charge Poisson apply at prec 1e-5; at k = 5 the two extra
     // units leave two warps idle for a third of the time (1.13 -> 1.16, not used).
     static constexpr int NWARP = K > 8 ? 8 : K == 6 ? 4 : K, NTHR = 32 * NWARP;
     static constexpr int NXU = 2 * (K - NWARP);  // extra units: pair 8 + u / 2, slice u mod 2

@@ -15,8 +15,9 @@
 // Refinement follows the adaptive projection: after every pass the leaves whose wavelet norm exceeds
 // prec ||out|| 2^{-depth/2} are split and their children computed.
 //
-// Work per node: 9 mode products of a (2k)^3 FP64 tensor on the FP64 matrix instruction (mw_block.cuh), whatever the
-// number of levels of generation, 2 blocks read and 1 written: bound by the FP64 pipe.
+// Work per node: 9 mode products of a (2k)^3 FP64 tensor on the FP64 matrix instruction (mw_block.cuh); a generated factor
+// takes a third of its three instead, after a descent of about as much for the first level and a fifth of that for each
+// further one; 2 blocks read and 1 written: bound by the FP64 pipe.
 #include <algorithm>
 #include <cmath>
 #include <numeric>
@@ -71,8 +72,8 @@ struct MulCfg {
 // One output node per block.  Per factor: its block, own or generated below the deepest ancestor (bx_descend: a scaling block
 // alone), to the point values in a separable transform; the product goes back through PF.  FP64-bound: 9 mode products per node on
 // the matrix instruction (16 us per node and SM at k = 10), two blocks per SM so that one's loads and barriers hide behind
-// the other's products.  28 pairs at k = 10: 15.5 ms with a thread per pencil and a reconstruction per level of a
-// missing node.
+// the other's products.  28 pairs at k = 10: 15.5 ms with a thread per pencil and a whole reconstruction per level of a
+// missing node, 5.2 ms now.
 template <int K>
 __global__ void __launch_bounds__(BX<K, 2 * K>::NTHR, MulCfg<K>::MINB)
     k_mul(const MulItem* __restrict__ items, const MulTree* __restrict__ trees, const double* __restrict__ frMV,
