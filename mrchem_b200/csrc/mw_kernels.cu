@@ -452,33 +452,31 @@ __global__ void __launch_bounds__(kDotThreads) k_dot(TView a, int na, const doub
     __shared__ double red[64];
     __shared__ unsigned done;
     __shared__ double ws[kDotThreads / 32];
-    const int group = blockIdx.x * kDotGroups + threadIdx.x / 128, ngroup = gridDim.x * kDotGroups, t = threadIdx.x & 127;
+    const int group = blockIdx.x * kDotGroups + threadIdx.x / 128, t = threadIdx.x & 127;
+    const int nparts = dot_in_turn(K) ? min(na, (int)gridDim.x * kDotGroups) : na;
     double s = 0.0;
-    auto add = [&](int node) {
+    for (int node = group; node < na; node += gridDim.x * kDotGroups) {
         const uint64_t key = a.key[node];
         const int j = hlookup(hk, hv, hcap, key);
-        if (j < 0) return;
-        const bool root = key_depth(key) == 0;
-        const double2* x = reinterpret_cast<const double2*>(a.coef + (size_t)node * G::BS);
-        const double2* y = reinterpret_cast<const double2*>(bcoef + (size_t)j * G::BS);
+        if (j >= 0) {
+            const bool root = key_depth(key) == 0;
+            const double2* x = reinterpret_cast<const double2*>(a.coef + (size_t)node * G::BS);
+            const double2* y = reinterpret_cast<const double2*>(bcoef + (size_t)j * G::BS);
 #pragma unroll 8
-        for (int e = t; e < G::BS / 2; e += 128) {
-            const double2 u = x[e], v = y[e];
-            const int aa = 2 * (e % K), bb = (e / K) % G::K2, cc = e / (K * G::K2);
-            const bool sc = !root && bb < K && cc < K;
-            if (!(sc && aa < K)) s = fma(u.x, v.x, s);
-            if (!(sc && aa + 1 < K)) s = fma(u.y, v.y, s);
+            for (int e = t; e < G::BS / 2; e += 128) {
+                const double2 u = x[e], v = y[e];
+                const int aa = 2 * (e % K), bb = (e / K) % G::K2, cc = e / (K * G::K2);
+                const bool sc = !root && bb < K && cc < K;
+                if (!(sc && aa < K)) s = fma(u.x, v.x, s);
+                if (!(sc && aa + 1 < K)) s = fma(u.y, v.y, s);
+            }
         }
-    };
-    if constexpr (dot_in_turn(K)) {
-        for (int node = group; node < na; node += ngroup) add(node);
-    } else {
-        if (group < na) add(group);
+        if constexpr (!dot_in_turn(K)) break;
     }
     for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
     __syncthreads();
-    if (t == 0) {
+    if (t == 0 && group < nparts) {
         const double* w = ws + (threadIdx.x >> 5);
         part[group] = (w[0] + w[1]) + (w[2] + w[3]);
     }
@@ -490,7 +488,7 @@ __global__ void __launch_bounds__(kDotThreads) k_dot(TView a, int na, const doub
     __threadfence();
     double d = 0.0;
     s = 0.0;
-    for (int i = threadIdx.x; i < ngroup; i += kDotThreads) s += __ldcg(part + i);
+    for (int i = threadIdx.x; i < nparts; i += kDotThreads) s += __ldcg(part + i);
     block_sum2(s, d, red);
     if (threadIdx.x == 0) {
         *ticket = 0u;  // for the next call on this stream
